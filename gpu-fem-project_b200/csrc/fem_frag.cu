@@ -75,12 +75,12 @@ namespace dev {
 template <int P>
 struct FragDims {
   static constexpr int P1 = P + 1, NN = P1 * P1, NQ = NN;
-  static constexpr int K4 = (NN + 3) / 4;   // node k-steps = quadrature k-steps = J column tiles
+  static constexpr int K4 = (NN + 3) / 4;   // node k-steps = quadrature k-steps
   static constexpr int NQP = 4 * K4;        // padded quadrature points
+  static constexpr int QT = 2 * ((NQ + 15) / 16);  // J-stage row tiles (8 quadrature points each), in pairs
   static constexpr int NTN = (NN + 7) / 8;  // node tiles of the component-major stiffness product
   static constexpr int CS = Dims<P>::CS;    // plan code record bytes per element
   static constexpr int WARPS = 4;           // warps per CTA
-  static constexpr int TG = (K4 + 3) / 4;   // transpose groups: quadrature points per lane
   // Stiffness layout: component-major node tiles at p = 2, 3 (two tiles of 8 nodes),
   // interleaved rows r = 2a + i at p = 4 (50 rows in seven tiles, where node tiles
   // would pad 25 nodes to 32 and need 280 instead of 196 MMAs per element).
@@ -102,19 +102,26 @@ struct FragLayout {
   using F = FragDims<P>;
   static constexpr int K4 = F::K4, NTN = F::NTN, NQP = F::NQP, NN = F::NN;
   static constexpr int CS = DROP ? 4 * NN * NN : F::CS;  // staged bytes per element
-  static constexpr size_t tabJ = 0;                          // double [K4][K4][32]
-  static constexpr size_t tabF = tabJ + 8 * K4 * K4 * 32;    // double2 [K4][NTAB][TABW]
+  // Slot of quadrature point q of an element's arrays, and the slots between the two
+  // elements: a quarter-warp of the quadrature stage stores points q, q + 1 of two
+  // tiles of both elements (slots g, g + 10, g + PS, g + PS + 10 with PS = 4 mod 8:
+  // eight distinct 16-byte bank groups); the fragment loads read four consecutive slots.
+  static constexpr int PS = (NQP + 2 * ((NQP - 1) / 8) + 11) / 8 * 8 - 4;
+  __host__ __device__ static constexpr int slot(int q) { return q + 2 * (q >> 3); }
+  static constexpr size_t tabJ = 0;                          // double2 [K4][QT][32]
+  static constexpr size_t tabF = tabJ + 16 * K4 * F::QT * 32;  // double2 [K4][NTAB][TABW]
   static constexpr size_t wq = tabF + 16 * K4 * F::NTAB * F::TABW;  // double [NQP]
   static constexpr size_t csum = align16(wq + 8 * NQP);       // double2 [NQP]: sum_a dN(a, q)
   static constexpr size_t tabB = align16(csum + 16 * NQP);    // double2 [8][32]: BF16x6 stiffness operands
   static constexpr size_t warps = align16(tabB + (B16 ? 16 * 8 * 32 : 0));
-  // warp-relative; [2] = the two elements of the step
-  static constexpr size_t WI0 = 0;                 // double2 [2][NQP]: sqrt|s| (J^-1_0x, J^-1_1x)
-  static constexpr size_t WI1 = WI0 + 16 * 2 * NQP;  // double2 [2][NQP]: sqrt|s| (J^-1_0y, J^-1_1y)
-  static constexpr size_t WS0 = WI1 + 16 * 2 * NQP;  // double2 [2][NQP]: (S-hat_xx, S-hat_xy)
-  static constexpr size_t WS1 = WS0 + 16 * 2 * NQP;  // double2 [2][NQP]: (S-hat_xy, S-hat_yy)
-  static constexpr size_t SG = WS1 + 16 * 2 * NQP;   // double [2][NQP]: sign of s (0 on padding)
-  static constexpr size_t NID = SG + 8 * 2 * NQP;    // int [2][NN]: node ids
+  // warp-relative; [2] = the two elements of the step, point q at slot(q) of PS
+  static constexpr size_t WI0 = 0;                  // double2 [2][PS]: sqrt|s| (J^-1_0x, J^-1_1x)
+  static constexpr size_t WI1 = WI0 + 16 * 2 * PS;  // double2 [2][PS]: sqrt|s| (J^-1_0y, J^-1_1y)
+  static constexpr size_t WS0 = WI1 + 16 * 2 * PS;  // double2 [2][PS]: (S-hat_xx, S-hat_xy)
+  static constexpr size_t WS1 = WS0 + 16 * 2 * PS;  // double2 [2][PS]: (S-hat_xy, S-hat_yy)
+  static constexpr size_t SG = WS1 + 16 * 2 * PS;   // double [2][NQP]: sign of s (0 on padding)
+  static constexpr size_t MC = align16(SG + 8 * 2 * NQP);  // double2: the mesh's (+-sqrt|t| or |t mu|, lam / mu)
+  static constexpr size_t NID = MC + 16;            // int [2][NN]: node ids
   static constexpr size_t RB = align16(NID + 4 * 2 * NN);  // int [2][NN]: rowp[node]
   static constexpr size_t STAGE = align16(RB + 4 * 2 * NN);  // [2 buffers][2 elements][CS] code records
   // staging slots: p = 3, 3 node-tile pairs x 2 halves, direct and transposed; p = 2,
@@ -126,6 +133,13 @@ struct FragLayout {
   static constexpr size_t warp_bytes = align16(AT + (NL ? 8 * 2 * NQP * 16 : 0));
   static constexpr size_t total = warps + F::WARPS * warp_bytes;
 };
+
+// D = A B, the first product of an accumulator (no zeroed registers needed).
+__device__ __forceinline__ void dmma_first(double &c0, double &c1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%4,%4};"
+               : "=d"(c0), "=d"(c1)
+               : "d"(a), "d"(b), "d"(0.0));
+}
 
 // D += A B, m16n8k16, BF16 operands, FP32 accumulate.
 __device__ __forceinline__ void bmma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -147,16 +161,12 @@ __device__ __forceinline__ void split3(double v, uint32_t &hi, uint32_t &mid, ui
   lo = __bfloat16_as_ushort(l);
 }
 
-__device__ __forceinline__ double sel4(double x0, double x1, double x2, double x3, int i) {
-  return i == 0 ? x0 : (i == 1 ? x1 : (i == 2 ? x2 : x3));
-}
-
-template <int P, bool B16 = false>
+template <int P, bool B16 = false, bool NL = false>
 __device__ __forceinline__ void frag_prologue(unsigned char *smem) {
   using F = FragDims<P>;
   using L = FragLayout<P, false, false, B16>;
-  constexpr int P1 = F::P1, NN = F::NN, NQ = F::NQ, K4 = F::K4, NTAB = F::NTAB, TABW = F::TABW;
-  double *tabJ = reinterpret_cast<double *>(smem + L::tabJ);
+  constexpr int P1 = F::P1, NN = F::NN, NQ = F::NQ, K4 = F::K4, QT = F::QT, NTAB = F::NTAB, TABW = F::TABW;
+  double2 *tabJ = reinterpret_cast<double2 *>(smem + L::tabJ);
   double2 *tabF = reinterpret_cast<double2 *>(smem + L::tabF);
   double *wq = reinterpret_cast<double *>(smem + L::wq);
   // dN(a, q) = (N_y dN_x, N_x dN_y) with the rounding of the element kernel's table
@@ -166,17 +176,11 @@ __device__ __forceinline__ void frag_prologue(unsigned char *smem) {
     lag1d(P, kGX[P][q / P1], a / P1, Ny, dNy);
     return make_double2(__dmul_rn(Ny, dNx), __dmul_rn(Nx, dNy));
   };
-  // J-stage B fragments: lane (g, t) of (ks, tn) holds dN_{g%2}(a = 4ks + t, q = 4tn + g/2)
-  for (int i = threadIdx.x; i < K4 * K4 * 32; i += blockDim.x) {
-    const int lane = i & 31, blk = i >> 5, ks = blk / K4, tn = blk - ks * K4;
-    const int g = lane >> 2, t = lane & 3;
-    const int a = 4 * ks + t, q = 4 * tn + (g >> 1);
-    double v = 0.0;
-    if (a < NN && q < NQ) {
-      const double2 d = dN(a, q);
-      v = (g & 1) ? d.y : d.x;
-    }
-    tabJ[i] = v;
+  // J-stage A fragments: lane (g, t) of (ks, tm) holds dN(a = 4ks + t, q = 8tm + g)
+  for (int i = threadIdx.x; i < K4 * QT * 32; i += blockDim.x) {
+    const int lane = i & 31, blk = i >> 5, ks = blk / QT, tm = blk - ks * QT;
+    const int a = 4 * ks + (lane & 3), q = 8 * tm + (lane >> 2);
+    tabJ[i] = (a < NN && q < NQ) ? dN(a, q) : make_double2(0.0, 0.0);
   }
   // stiffness fragments at (ks, T), q = 4ks + t: component-major, lane (g, t) holds
   // dN(a = 8T + pi(g), q); interleaved, entry 4(g/2) + t holds dN(a = 4T + g/2, q)
@@ -193,8 +197,11 @@ __device__ __forceinline__ void frag_prologue(unsigned char *smem) {
     }
     tabF[i] = (a < NN && q < NQ) ? dN(a, q) : make_double2(0.0, 0.0);
   }
-  for (int q = threadIdx.x; q < F::NQP; q += blockDim.x)
-    wq[q] = q < NQ ? __dmul_rn(kGW[P][q % P1], kGW[P][q / P1]) : 0.0;
+  // Gauss weights (NONLINEAR), their square roots (LINEAR)
+  for (int q = threadIdx.x; q < F::NQP; q += blockDim.x) {
+    const double w = q < NQ ? __dmul_rn(kGW[P][q % P1], kGW[P][q / P1]) : 0.0;
+    wq[q] = NL ? w : sqrt(w);
+  }
   // BF16x6 stiffness (order 3): entry (2k + h, lane (g, t)) holds dN(a, q) for the
   // node a = 8h + pi(g) and quadrature point q = 2t + (k & 1) + 8 (k >> 1) that lane
   // (g, t) places in its m16n8k16 fragments
@@ -208,16 +215,14 @@ __device__ __forceinline__ void frag_prologue(unsigned char *smem) {
   }
   // sum_a dN(a, q): zero in exact arithmetic, a few ulp of the table entries in
   // FP64; summed with Neumaier compensation (error ~1e-30 absolute) over the J-stage
-  // table entries written above (lane (g, t) of block (ks, tn) holds component g%2 of
-  // dN(4ks + t, 4tn + g/2)) instead of evaluating the basis again
+  // table entries written above instead of evaluating the basis again
   __syncthreads();
   double2 *csum = reinterpret_cast<double2 *>(smem + L::csum);
   for (int q = threadIdx.x; q < F::NQP; q += blockDim.x) {
     double s0 = 0.0, c0 = 0.0, s1 = 0.0, c1 = 0.0;
     if (q < NQ) {
       for (int a = 0; a < NN; a++) {
-        const int e = (((a >> 2) * K4 + (q >> 2)) * 32) + ((2 * (q & 3)) << 2) + (a & 3);
-        const double2 d = make_double2(tabJ[e], tabJ[e + 4]);
+        const double2 d = tabJ[((a >> 2) * QT + (q >> 3)) * 32 + 4 * (q & 7) + (a & 3)];
         const double t0 = s0 + d.x, t1 = s1 + d.y;
         c0 += fabs(s0) >= fabs(d.x) ? (s0 - t0) + d.x : (d.x - t0) + s0;
         c1 += fabs(s1) >= fabs(d.y) ? (s1 - t1) + d.y : (d.y - t1) + s1;
@@ -614,18 +619,22 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
   constexpr bool B16 = (MODE & kB16) != 0;  // BF16x6 element stiffness
   using F = FragDims<P>;
   using L = FragLayout<P, !PLAN, NL, B16, (MODE & kJac) != 0>;
-  constexpr int NN = F::NN, NQ = F::NQ, K4 = F::K4, NTN = F::NTN, NQP = F::NQP, CS = F::CS;
+  constexpr int NN = F::NN, NQ = F::NQ, K4 = F::K4, QT = F::QT, NTN = F::NTN, NQP = F::NQP, PS = L::PS, CS = F::CS;
   constexpr int STG = L::CS;  // staged bytes per element: plan code record or map rows
   constexpr bool RES = (MODE & kRes) != 0, JAC = (MODE & kJac) != 0;
   constexpr bool RUNS = (P == 3);  // order 3: staged row runs, one bulk reduction per adjacent run
   static_assert(!NL || !F::IL, "NONLINEAR strain: orders 2 and 3");
   static_assert(PLAN || !Gen::kBatched, "drop-in mode assembles one mesh");
   static_assert(!B16 || (!NL && P == 3), "BF16x6 stiffness: LINEAR, order 3");
+  // LINEAR FP64: mu is folded into the gradients (G-hat carries sqrt|s mu|), so a block
+  // is four FMAs of M with the one constant lam / mu.  (B16 keeps sqrt|s|: the BF16
+  // split rounds the operands.)
+  constexpr bool SCALED = !NL && !B16;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   const int e_ld = g >> 2, c_ld = g & 3;  // element / component this lane gathers
-  const double *tabJ = reinterpret_cast<const double *>(smem + L::tabJ);
+  const double2 *tabJ = reinterpret_cast<const double2 *>(smem + L::tabJ);
   const double2 *tabF = reinterpret_cast<const double2 *>(smem + L::tabF);
   const double *wqs = reinterpret_cast<const double *>(smem + L::wq);
   const double2 *csum = reinterpret_cast<const double2 *>(smem + L::csum);
@@ -636,6 +645,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
   double2 *WS0 = reinterpret_cast<double2 *>(ws + L::WS0);
   double2 *WS1 = reinterpret_cast<double2 *>(ws + L::WS1);
   double *SGs = reinterpret_cast<double *>(ws + L::SG);
+  volatile double2 *MC = reinterpret_cast<volatile double2 *>(ws + L::MC);
   int *nid = reinterpret_cast<int *>(ws + L::NID);
   int *rb = reinterpret_cast<int *>(ws + L::RB);
   unsigned char *stage = ws + L::STAGE;
@@ -702,6 +712,18 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
     cp_async_commit();
   };
 
+  // the mesh's constants of the quadrature stage and of the blocks (LINEAR)
+  auto mesh_constants = [&](const AsmArgs &M) {
+    if constexpr (!NL) {
+      const double ts = SCALED ? M.t * M.mu : M.t;
+      if (lane == 0) {
+        MC->x = ts < 0.0 ? -sqrt(-ts) : sqrt(ts);
+        MC->y = M.mu != 0.0 ? M.lam / M.mu : 0.0;
+      }
+      __syncwarp();
+    }
+  };
+  int meshC = -1;
   // a grid launched after this one with programmatic serialization may start its CTAs
   // as this one's retire; it waits (griddepcontrol.wait) before it writes
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -718,7 +740,11 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
     if constexpr (P == 4) asm volatile("" : "+l"(mtab));
     const int ne = cur.ne;
     const AsmArgs &M = args(cur);
-    const double mu = M.mu, lam = M.lam, thick = M.t, c11 = lam + 2.0 * mu;
+    const double mu = M.mu, lam = M.lam, c11 = lam + 2.0 * mu;
+    if (cur.mesh != meshC) {
+      mesh_constants(M);
+      meshC = cur.mesh;
+    }
     // 0. commit this pair's gathered data
     double val[K4];
 #pragma unroll
@@ -740,71 +766,73 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
     load_values(nxt, nodeB, valB, rbB);
     load_nodes(nn2, nodeA);
 
-    // 1. J stage: cj[tn] = (d/dxi, d/deta) of component c_ld of element e_ld at q = 4tn + t.
+    // 1. J stage: rows = quadrature points (8 per tile), columns = (element, component):
+    //    lane (g, t) ends with component pair (x, y) (t even) or (u, v) (t odd) of element
+    //    t/2 at points q = 8tm + g, derivative d of each.
     //    J = sum_a x_a dN_a cancels by ~h/|x| (1e-4 on a 10x10 square of 1024^2
     //    elements), so the coordinates enter relative to the element's node 0 (an
     //    exact subtraction for nearby values) and x_0 sum_a dN_a is added back: the
     //    same sum, evaluated without the cancellation.
+    const int e_q = t >> 1, odd = t & 1;
+    const double xq = __shfl_sync(0xffffffffu, val[0], 16 * e_q), yq = __shfl_sync(0xffffffffu, val[0], 16 * e_q + 4);
     const double xn0 = __shfl_sync(0xffffffffu, val[0], lane & ~3);
     const double x0 = c_ld < 2 ? xn0 : 0.0;
 #pragma unroll
     for (int ks = 0; ks < K4; ks++) val[ks] -= x0;
-    constexpr int TG = F::TG;
-    double cj[4 * TG][2];
-#pragma unroll
-    for (int tn = 0; tn < 4 * TG; tn++) cj[tn][0] = cj[tn][1] = 0.0;
+    double cj[QT][2][2];  // [tile][d][component of the pair]
 #pragma unroll
     for (int ks = 0; ks < K4; ks++)
 #pragma unroll
-      for (int tn = 0; tn < K4; tn++) dmma(cj[tn][0], cj[tn][1], val[ks], tabJ[(ks * K4 + tn) * 32 + lane]);
-#pragma unroll
-    for (int tn = 0; tn < K4; tn++) {
-      const double2 cs = csum[4 * tn + t];
-      cj[tn][0] = fma(x0, cs.x, cj[tn][0]);
-      cj[tn][1] = fma(x0, cs.y, cj[tn][1]);
-    }
-
-    // 2. transpose, per group m of four column tiles: this lane takes quadrature
-    //    point q = 4(4m + c_ld) + t of element e_ld
-#pragma unroll
-    for (int m = 0; m < TG; m++) {
-      double rv[4][2];
-      rv[0][0] = sel4(cj[4 * m][0], cj[4 * m + 1][0], cj[4 * m + 2][0], cj[4 * m + 3][0], c_ld);
-      rv[0][1] = sel4(cj[4 * m][1], cj[4 * m + 1][1], cj[4 * m + 2][1], cj[4 * m + 3][1], c_ld);
-#pragma unroll
-      for (int r = 1; r < 4; r++) {
-        const int src = c_ld ^ r;
-        const double s0 = sel4(cj[4 * m][0], cj[4 * m + 1][0], cj[4 * m + 2][0], cj[4 * m + 3][0], src);
-        const double s1 = sel4(cj[4 * m][1], cj[4 * m + 1][1], cj[4 * m + 2][1], cj[4 * m + 3][1], src);
-        rv[r][0] = __shfl_xor_sync(0xffffffffu, s0, r << 2);
-        rv[r][1] = __shfl_xor_sync(0xffffffffu, s1, r << 2);
+      for (int tm = 0; tm < QT; tm++) {
+        const double2 d = tabJ[(ks * QT + tm) * 32 + lane];
+        if (ks == 0) {
+          dmma_first(cj[tm][0][0], cj[tm][0][1], d.x, val[ks]);
+          dmma_first(cj[tm][1][0], cj[tm][1][1], d.y, val[ks]);
+        } else {
+          dmma(cj[tm][0][0], cj[tm][0][1], d.x, val[ks]);
+          dmma(cj[tm][1][0], cj[tm][1][1], d.y, val[ks]);
+        }
       }
-      // component k of this quadrature point came from round k ^ c_ld
-      auto comp = [&](int k, int d) {
-        const int r = k ^ c_ld;
-        return d == 0 ? sel4(rv[0][0], rv[1][0], rv[2][0], rv[3][0], r)
-                      : sel4(rv[0][1], rv[1][1], rv[2][1], rv[3][1], r);
-      };
-      const int tq = 4 * m + c_ld;  // column tile of this lane's quadrature point
-      const int q = 4 * tq + t;
-      const bool valid = e_ld < ne && tq < K4 && q < NQ;
+
+    // 2. per pair m of tiles: lanes t, t^1 exchange halves, so that each takes one
+    //    quadrature point, q = 16m + 8 (t%2) + g of element t/2, with J and the
+    //    reference gradient of the state
+    unsigned negm = 0;  // lanes whose point has s (mu) < 0
+#pragma unroll
+    for (int m = 0; m < QT / 2; m++) {
+      double jm[2][2], um[2][2];  // [d][component]
+#pragma unroll
+      for (int d = 0; d < 2; d++)
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+          const double lo = cj[2 * m][d][c], hi = cj[2 * m + 1][d][c];
+          const double r = __shfl_xor_sync(0xffffffffu, odd ? lo : hi, 1);
+          jm[d][c] = odd ? r : lo;
+          um[d][c] = odd ? hi : r;
+        }
+      const int q = 16 * m + 8 * odd + g;
+      const bool valid = e_q < ne && q < NQ;
+      const int o = e_q * PS + L::slot(q);
       double2 wi0 = make_double2(0, 0), wi1 = make_double2(0, 0), ws0 = make_double2(0, 0), ws1 = make_double2(0, 0);
       double sg = 0.0;
+      bool ng = false;
       if (valid) {
-        const double j00 = comp(0, 0), j01 = comp(0, 1), j10 = comp(1, 0), j11 = comp(1, 1);
-        const double g00 = comp(2, 0), g01 = comp(2, 1), g10 = comp(3, 0), g11 = comp(3, 1);
+        const double2 cs = csum[q];
+        const double j00 = fma(xq, cs.x, jm[0][0]), j01 = fma(xq, cs.y, jm[1][0]);
+        const double j10 = fma(yq, cs.x, jm[0][1]), j11 = fma(yq, cs.y, jm[1][1]);
+        const double g00 = um[0][0], g01 = um[1][0], g10 = um[0][1], g11 = um[1][1];
         const double det = j00 * j11 - j01 * j10;
-        const double inv = 1.0 / det;
-        const double i00 = j11 * inv, i01 = -j01 * inv, i10 = -j10 * inv, i11 = j00 * inv;
-        const double st = wqs[q] * det * thick;
-        const double rs = sqrt(fabs(st));
-        sg = st < 0.0 ? -1.0 : 1.0;
-        const double sw = sg * rs;
-        const double uxx = g00 * i00 + g01 * i10, uxy = g00 * i01 + g01 * i11;
-        const double uyx = g10 * i00 + g11 * i10, uyy = g10 * i01 + g11 * i11;
-        wi0 = make_double2(rs * i00, rs * i10);
-        wi1 = make_double2(rs * i01, rs * i11);
         if constexpr (NL) {
+          const double inv = 1.0 / det;
+          const double i00 = j11 * inv, i01 = -j01 * inv, i10 = -j10 * inv, i11 = j00 * inv;
+          const double st = wqs[q] * det * M.t;
+          const double rs = sqrt(fabs(st));
+          sg = st < 0.0 ? -1.0 : 1.0;
+          const double sw = sg * rs;
+          const double uxx = g00 * i00 + g01 * i10, uxy = g00 * i01 + g01 * i11;
+          const double uyx = g10 * i00 + g11 * i10, uyy = g10 * i01 + g11 * i11;
+          wi0 = make_double2(rs * i00, rs * i10);
+          wi1 = make_double2(rs * i01, rs * i11);
           // Green strain E = 1/2 (g + g^T + g^T g), S = 2 mu E + lam tr(E) I, first Piola
           // P = F S (F = I + g); tangent A_{il,kn} = delta_ik S_ln + mu F_in F_kl
           // + mu (F F^T)_ik delta_ln + lam F_il F_kn (element/FEKernels.h:286-315,
@@ -819,8 +847,8 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
           const double pyx = F[1][0] * Sm[0][0] + F[1][1] * Sm[1][0], pyy = F[1][0] * Sm[0][1] + F[1][1] * Sm[1][1];
           ws0 = make_double2(sw * pxx, sw * pyx);  // (P-hat_x0, P-hat_y0)
           ws1 = make_double2(sw * pxy, sw * pyy);  // (P-hat_x1, P-hat_y1)
-          if (JAC && tq < K4) {
-            double *at = ATs + (e_ld * NQP + q) * 16;
+          if constexpr (JAC) {
+            double *at = ATs + (e_q * NQP + q) * 16;
 #pragma unroll
             for (int ll = 0; ll < 2; ll++)
 #pragma unroll
@@ -840,26 +868,39 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
                 }
           }
         } else {
-          const double tr = uxx + uyy;
-          const double sxx = sw * (2.0 * mu * uxx + lam * tr);
-          const double sxy = sw * (mu * (uxy + uyx));
-          const double syy = sw * (2.0 * mu * uyy + lam * tr);
-          ws0 = make_double2(sxx, sxy);
-          ws1 = make_double2(sxy, syy);
+          // s = w det t, J^-1 = adj(J) / det: sqrt|s| J^-1 = +-c adj(J) with
+          // c = sqrt|w t| / sqrt|det| (the sign leaves every product of two gradients
+          // alone), grad u = g adj(J) / det, and s sigma G = (+-c sigma(g adj(J))) (c adj(J) dN):
+          // one reciprocal square root instead of a division and a square root.
+          // A singular point (det = 0) gives NaN.
+          const double2 mc = make_double2(MC->x, MC->y);
+          const double r = det != 0.0 ? rsqrt(fabs(det)) : __longlong_as_double(0x7ff8000000000000LL);
+          const double c = wqs[q] * fabs(mc.x) * r;
+          ng = (det < 0.0) != (mc.x < 0.0);
+          sg = ng ? -1.0 : 1.0;
+          const double cw = sg * c;
+          const double uxx = g00 * j11 - g01 * j10, uxy = g01 * j00 - g00 * j01;
+          const double uyx = g10 * j11 - g11 * j10, uyy = g11 * j00 - g10 * j01;
+          wi0 = make_double2(c * j11, -(c * j10));
+          wi1 = make_double2(-(c * j01), c * j00);
+          const double m1 = SCALED ? 1.0 : mu, lt = (SCALED ? mc.y : lam) * (uxx + uyy);
+          const double sxy = cw * (m1 * (uxy + uyx));
+          ws0 = make_double2(cw * fma(2.0 * m1, uxx, lt), sxy);
+          ws1 = make_double2(sxy, cw * fma(2.0 * m1, uyy, lt));
         }
-      } else if (NL && JAC && tq < K4) {
-        double2 *at = reinterpret_cast<double2 *>(ATs + (e_ld * NQP + q) * 16);
+      } else if (NL && JAC && q < NQP) {
+        double2 *at = reinterpret_cast<double2 *>(ATs + (e_q * NQP + q) * 16);
 #pragma unroll
         for (int j = 0; j < 8; j++) at[j] = make_double2(0.0, 0.0);
       }
-      if (tq < K4) {
-        const int o = e_ld * NQP + q;
+      if (q < NQP) {
         WI0[o] = wi0;
         WI1[o] = wi1;
         WS0[o] = ws0;
         WS1[o] = ws1;
-        SGs[o] = sg;
+        if constexpr (!NL) SGs[e_q * NQP + q] = sg;
       }
+      if constexpr (SCALED) negm |= __ballot_sync(0xffffffffu, ng);
     }
     __syncwarp();
 
@@ -871,6 +912,22 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
     }
     if constexpr (Gen::kSched) gen.acquire(cur, lane);
     const Out O{M.mat, M.residual, stage + buf * 2 * STG, rb, reinterpret_cast<const int *>(stage + buf * 2 * STG)};
+    // the 2x2 block of M (LINEAR: the plane-stress combination, divided by mu where
+    // the gradients carry sqrt mu; NONLINEAR: the product is the block)
+    const double lm = SCALED ? MC->y : 0.0, lm2 = lm + 2.0;
+    auto block = [&](double mxx, double mxy, double myx, double myy, double &kxx, double &kxy, double &kyx, double &kyy) {
+      if constexpr (NL) {
+        kxx = mxx, kxy = mxy, kyx = myx, kyy = myy;
+      } else if constexpr (SCALED) {
+        kxx = fma(lm2, mxx, myy);
+        kxy = fma(lm, mxy, myx);
+        kyx = fma(lm, myx, mxy);
+        kyy = fma(lm2, myy, mxx);
+      } else {
+        kxx = c11 * mxx + mu * myy, kxy = lam * mxy + mu * myx;
+        kyx = lam * myx + mu * mxy, kyy = c11 * myy + mu * mxx;
+      }
+    };
     if constexpr (!F::IL) {
       // node tiles on the tensor cores: both at p = 3; at p = 2 only tile 0 (nodes 0-7),
       // node 8 (alone in tile 1) has its row and column on the FP64 pipe (12 instead of
@@ -895,10 +952,10 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
 #pragma unroll
           for (int k = 0; k < 4; k++) {
             const int q = 2 * t + (k & 1) + 8 * (k >> 1);
-            const int o = el * NQP + q;
+            const int o = el * PS + L::slot(q);
             const bool qv = q < NQ;
             const double2 w0 = qv ? WI0[o] : make_double2(0.0, 0.0), w1 = qv ? WI1[o] : make_double2(0.0, 0.0);
-            sgk[k] = qv ? SGs[o] : 0.0;
+            sgk[k] = qv ? SGs[el * NQP + q] : 0.0;
             double2 s0 = make_double2(0.0, 0.0), s1 = make_double2(0.0, 0.0);
             if (RES && qv) {
               s0 = WS0[o];
@@ -995,8 +1052,8 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
                   if (a < NN && b < NN) {
                     const double mxx = acc[0][0][h][c], mxy = acc[0][1][h][c];
                     const double myx = acc[1][0][h][c], myy = acc[1][1][h][c];
-                    const double kxx = c11 * mxx + mu * myy, kxy = lam * mxy + mu * myx;
-                    const double kyx = lam * myx + mu * mxy, kyy = c11 * myy + mu * mxx;
+                    double kxx, kxy, kyx, kyy;
+                    block(mxx, mxy, myx, myy, kxx, kxy, kyx, kyy);
                     const int sl = (r == 1 && h == 0) ? frag_slot(1, g & 1, 1) : frag_slot(r + h, u, 0);
                     const int pos = (r == 1 && h == 0) ? 8 * (g >> 1) + 4 * u + t : 4 * g + t;
                     frag_put<P, PLAN>(O, el, a, b, 0, kxx, kxy, kyx, kyy, redsW + 128 * sl + 4 * pos);
@@ -1021,17 +1078,21 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
         double acc[NPAIR][4][2];
         double rp[NTN][2];
         double n8[4] = {0.0, 0.0, 0.0, 0.0}, d8[4] = {0.0, 0.0, 0.0, 0.0};  // p = 2: M[8][pi(g)], M[8][8]
+        if constexpr (NL) {
   #pragma unroll
-        for (int k = 0; k < NPAIR; k++)
+          for (int k = 0; k < NPAIR; k++)
   #pragma unroll
-          for (int c = 0; c < 4; c++) acc[k][c][0] = acc[k][c][1] = 0.0;
+            for (int c = 0; c < 4; c++) acc[k][c][0] = acc[k][c][1] = 0.0;
+        }
   #pragma unroll
         for (int T = 0; T < NTN; T++) rp[T][0] = rp[T][1] = 0.0;
+        // whether a point of this element has s (mu) < 0 (inverted element or negative
+        // thickness or modulus): only then do the A fragments take the points' signs
+        const bool neg = SCALED && (negm & (el ? 0xccccccccu : 0x33333333u)) != 0;
   #pragma unroll
         for (int ks = 0; ks < K4; ks++) {
-          const int o = el * NQP + 4 * ks + t;
+          const int o = el * PS + L::slot(4 * ks) + t;
           const double2 w0 = WI0[o], w1 = WI1[o];
-          const double sg = SGs[o];
           double fr[NTN][2];
   #pragma unroll
           for (int T = 0; T < NTN; T++) {
@@ -1040,17 +1101,19 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
             fr[T][1] = fma(w1.x, d.x, w1.y * d.y);
           }
           if constexpr (RES) {
-            const double2 s0 = WS0[o], s1 = WS1[o];
+            // LINEAR: the stress is symmetric, S-hat_yx = S-hat_xy
+            const double2 s0 = WS0[o];
+            const double s1y = WS1[o].y, s1x = NL ? WS1[o].x : s0.y;
   #pragma unroll
             for (int T = 0; T < NTN; T++) {
-              rp[T][0] = fma(fr[T][0], s0.x, fma(fr[T][1], s1.x, rp[T][0]));
-              rp[T][1] = fma(fr[T][0], s0.y, fma(fr[T][1], s1.y, rp[T][1]));
+              rp[T][0] = fma(fr[T][0], s0.x, fma(fr[T][1], s1x, rp[T][0]));
+              rp[T][1] = fma(fr[T][0], s0.y, fma(fr[T][1], s1y, rp[T][1]));
             }
           }
           if constexpr (JAC && NL) {
             // K_ik[a][b] = sum over (q, l) of G-hat_l(q, a) B_ikl(q, b),
             // B_ikl = sign(s) sum_n A_{il,kn} G-hat_n(q, b): 4 (i, k) x 2 (l) MMAs per pair
-            const double *at = ATs + o * 16;
+            const double *at = ATs + (el * NQP + 4 * ks + t) * 16;
             double h0 = 0.0, h1 = 0.0;
             if constexpr (P == 2) {
               h0 = __shfl_sync(0xffffffffu, fr[1][0], t);
@@ -1090,7 +1153,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
           if constexpr (JAC && P == 2 && !NL) {
             // G-hat_i(q, 8) sits in lane (g = 0, t), tile 1
             const double h0 = __shfl_sync(0xffffffffu, fr[1][0], t), h1 = __shfl_sync(0xffffffffu, fr[1][1], t);
-            const double s0 = sg * h0, s1 = sg * h1;
+            const double s0 = neg ? SGs[el * NQP + 4 * ks + t] * h0 : h0, s1 = neg ? SGs[el * NQP + 4 * ks + t] * h1 : h1;
             n8[0] = fma(s0, fr[0][0], n8[0]);
             n8[1] = fma(s0, fr[0][1], n8[1]);
             n8[2] = fma(s1, fr[0][0], n8[2]);
@@ -1104,13 +1167,24 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
             int k = 0;
   #pragma unroll
             for (int TA = 0; TA < NTM; TA++) {
-              const double a0 = sg * fr[TA][0], a1 = sg * fr[TA][1];
+              double a0 = fr[TA][0], a1 = fr[TA][1];
+              if (neg) {
+                a0 *= SGs[el * NQP + 4 * ks + t];
+                a1 *= SGs[el * NQP + 4 * ks + t];
+              }
   #pragma unroll
               for (int TB = TA; TB < NTM; TB++, k++) {
-                dmma(acc[k][0][0], acc[k][0][1], a0, fr[TB][0]);
-                dmma(acc[k][1][0], acc[k][1][1], a0, fr[TB][1]);
-                dmma(acc[k][2][0], acc[k][2][1], a1, fr[TB][0]);
-                dmma(acc[k][3][0], acc[k][3][1], a1, fr[TB][1]);
+                if (ks == 0) {
+                  dmma_first(acc[k][0][0], acc[k][0][1], a0, fr[TB][0]);
+                  dmma_first(acc[k][1][0], acc[k][1][1], a0, fr[TB][1]);
+                  dmma_first(acc[k][2][0], acc[k][2][1], a1, fr[TB][0]);
+                  dmma_first(acc[k][3][0], acc[k][3][1], a1, fr[TB][1]);
+                } else {
+                  dmma(acc[k][0][0], acc[k][0][1], a0, fr[TB][0]);
+                  dmma(acc[k][1][0], acc[k][1][1], a0, fr[TB][1]);
+                  dmma(acc[k][2][0], acc[k][2][1], a1, fr[TB][0]);
+                  dmma(acc[k][3][0], acc[k][3][1], a1, fr[TB][1]);
+                }
               }
             }
           }
@@ -1155,11 +1229,8 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
                 const int b = 8 * TB + 4 * h + t;
                 if (a < NN && b < NN) {
                   const double mxx = acc[k][0][h], mxy = acc[k][1][h], myx = acc[k][2][h], myy = acc[k][3][h];
-                  // LINEAR: plane-stress combination of M; NONLINEAR: the block itself
-                  const double kxx = NL ? mxx : c11 * mxx + mu * myy;
-                  const double kxy = NL ? mxy : lam * mxy + mu * myx;
-                  const double kyx = NL ? myx : lam * myx + mu * mxy;
-                  const double kyy = NL ? myy : c11 * myy + mu * mxx;
+                  double kxx, kxy, kyx, kyy;
+                  block(mxx, mxy, myx, myy, kxx, kxy, kyx, kyy);
                   const int s0 = frag_slot(k, h, 0);
                   if (TA < TB) {
                     const int s1 = frag_slot(k, h, 1);
@@ -1206,8 +1277,8 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
 #pragma unroll
           for (int h = 0; h < 2; h++) {
             const double mxx = acc[0][0][h], mxy = acc[0][1][h], myx = acc[0][2][h], myy = acc[0][3][h];
-            const double kxx = c11 * mxx + mu * myy, kxy = lam * mxy + mu * myx;
-            const double kyx = lam * myx + mu * mxy, kyy = c11 * myy + mu * mxx;
+            double kxx, kxy, kyx, kyy;
+            block(mxx, mxy, myx, myy, kxx, kxy, kyx, kyy);
             dst[h] = frag_stage<P>(O, el, pa, 4 * h + t, 0, kxx, kxy, kyx, kyy, reds + 128 * h);
           }
 #pragma unroll
@@ -1221,8 +1292,8 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
           if (t < 2 || diag) {
             const double mxx = diag ? d8[0] : n8[0], mxy = diag ? d8[1] : n8[1];
             const double myx = diag ? d8[2] : n8[2], myy = diag ? d8[3] : n8[3];
-            const double kxx = c11 * mxx + mu * myy, kxy = lam * mxy + mu * myx;
-            const double kyx = lam * myx + mu * mxy, kyy = c11 * myy + mu * mxx;
+            double kxx, kxy, kyx, kyy;
+            block(mxx, mxy, myx, myy, kxx, kxy, kyx, kyy);
             dst[2] = frag_stage<P>(O, el, 8, diag ? 8 : pa, diag ? 0 : t, kxx, kxy, kyx, kyy, reds + 128 * 2);
           }
           if (dst[0] || dst[1] || dst[2]) {
@@ -1250,11 +1321,8 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
                 const int b = 8 * TB + 4 * h + t;
                 if (a < NN && b < NN) {
                   const double mxx = acc[k][0][h], mxy = acc[k][1][h], myx = acc[k][2][h], myy = acc[k][3][h];
-                  // LINEAR: plane-stress combination of M; NONLINEAR: the block itself
-                  const double kxx = NL ? mxx : c11 * mxx + mu * myy;
-                  const double kxy = NL ? mxy : lam * mxy + mu * myx;
-                  const double kyx = NL ? myx : lam * myx + mu * mxy;
-                  const double kyy = NL ? myy : c11 * myy + mu * mxx;
+                  double kxx, kxy, kyx, kyy;
+                  block(mxx, mxy, myx, myy, kxx, kxy, kyx, kyy);
                   // NONLINEAR diagonal tiles: (a, b) for a <= b and its exact transpose
                   const bool dir = TA < TB || !NL || a <= b;
                   const bool trn = TA < TB || (NL && a < b);
@@ -1283,10 +1351,8 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
             if (t < 2 || diag) {
               const double mxx = diag ? d8[0] : n8[0], mxy = diag ? d8[1] : n8[1];
               const double myx = diag ? d8[2] : n8[2], myy = diag ? d8[3] : n8[3];
-              const double kxx = NL ? mxx : c11 * mxx + mu * myy;
-              const double kxy = NL ? mxy : lam * mxy + mu * myx;
-              const double kyx = NL ? myx : lam * myx + mu * mxy;
-              const double kyy = NL ? myy : c11 * myy + mu * mxx;
+              double kxx, kxy, kyx, kyy;
+              block(mxx, mxy, myx, myy, kxx, kxy, kyx, kyy);
               const int b = diag ? 8 : pa, w = diag ? 0 : t;
               if constexpr (PLAN) {
                 frag_write<P>(O, el, 8, b, w, kxx, kxy, kyx, kyy, reds + 128 * slot);
@@ -1310,6 +1376,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
       int nw = 0;  // writes so far: ring position of the staging slot
       for (int el = 0; el < ne; el++) {
         if (PLAN && el > 0) pair_order_fence();
+        const bool neg = (negm & (el ? 0xccccccccu : 0x33333333u)) != 0;
         // residual R_(a,i'): lane partials rp over its quadrature points (with the
         // Jacobian, accumulated by the first three stiffness groups, which between them
         // form every column tile's fragments; alone, in a pass of its own), then a full
@@ -1352,7 +1419,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
         if constexpr (RES && !JAC) {
 #pragma unroll
           for (int ks = 0; ks < K4; ks++) {
-            const int o = el * NQP + 4 * ks + t;
+            const int o = el * PS + L::slot(4 * ks) + t;
             const double2 w = WIi[o];
             const double2 sj = WSi[o];  // (S-hat_xj, S-hat_yj), j = this lane's component
 #pragma unroll
@@ -1381,9 +1448,8 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
             for (int C = C0; C < C1; C++) acc[R - R0][C - C0][0] = acc[R - R0][C - C0][1] = 0.0;
 #pragma unroll
           for (int ks = 0; ks < K4; ks++) {
-            const int o = el * NQP + 4 * ks + t;
+            const int o = el * PS + L::slot(4 * ks) + t;
             const double2 w = WIi[o];
-            const double sg = SGs[o];
             double fr[K4];
 #pragma unroll
             for (int T = 0; T < K4; T++) {
@@ -1402,7 +1468,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
             }
 #pragma unroll
             for (int R = R0; R < R1; R++) {
-              const double af = sg * fr[R];
+              const double af = neg ? SGs[el * NQP + 4 * ks + t] * fr[R] : fr[R];
 #pragma unroll
               for (int C = (R > C0 ? R : C0); C < C1; C++)
                 dmma(acc[R - R0][C - C0][0], acc[R - R0][C - C0][1], af, fr[C]);
@@ -1421,10 +1487,8 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
               const double myx = ii ? acc[R - R0][C - C0][0] : o0, myy = ii ? acc[R - R0][C - C0][1] : o1;
               const int b = 4 * C + t;
               if (a < NN && b < NN && a <= b && (ii == 0 || a < b)) {
-                const double kxx = c11 * mxx + mu * myy;
-                const double kxy = lam * mxy + mu * myx;
-                const double kyx = lam * myx + mu * mxy;
-                const double kyy = c11 * myy + mu * mxx;
+                double kxx, kxy, kyx, kyy;
+                block(mxx, mxy, myx, myy, kxx, kxy, kyx, kyy);
                 // the ring slot's previous bulk read (NSLOT writes ago) is complete
                 asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(L::NSLOT - 1) : "memory");
                 double *slot = reds + 128 * (nw % L::NSLOT);
@@ -1473,7 +1537,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
 template <int P, int MODE>
 __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB) frag_kernel(const __grid_constant__ AsmArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
-  frag_prologue<P, (MODE & kB16) != 0>(smem);
+  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) != 0>(smem);
   const int warp = threadIdx.x >> 5;
   PairStride gen{A.begin, A.begin + A.count, (int64_t)blockIdx.x * FragDims<P>::WARPS + warp,
                  (int64_t)gridDim.x * FragDims<P>::WARPS};
@@ -1485,7 +1549,7 @@ template <int P, int MODE>
 __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB)
     frag_ranges_kernel(const __grid_constant__ AsmArgs A, const RangeList R) {
   extern __shared__ __align__(16) unsigned char smem[];
-  frag_prologue<P, (MODE & kB16) != 0>(smem);
+  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) != 0>(smem);
   const int warp = threadIdx.x >> 5;
   PairRanges gen{R, (int64_t)blockIdx.x * FragDims<P>::WARPS + warp, (int64_t)gridDim.x * FragDims<P>::WARPS};
   frag_loop<P, MODE>(smem, gen, A, &A);
@@ -1496,7 +1560,7 @@ template <int P, int MODE>
 __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB)
     frag_sched_kernel(const __grid_constant__ AsmArgs A, const __grid_constant__ SchedArgs S) {
   extern __shared__ __align__(16) unsigned char smem[];
-  frag_prologue<P, (MODE & kB16) != 0>(smem);
+  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) != 0>(smem);
   PairSched gen{&S};
   frag_loop<P, MODE>(smem, gen, A, &A);
 }
@@ -1508,7 +1572,7 @@ template <int P, int MODE>
 __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB)
     frag_batched_sched_kernel(const AsmArgs *__restrict__ meshes, const __grid_constant__ SchedArgs S) {
   extern __shared__ __align__(16) unsigned char smem[];
-  frag_prologue<P, (MODE & kB16) != 0>(smem);
+  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) != 0>(smem);
   PairSchedT<true> gen{&S};
   frag_loop<P, MODE>(smem, gen, meshes[0], meshes);
 }
@@ -1518,7 +1582,7 @@ template <int P, int MODE>
 __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB)
     frag_batched_kernel(const AsmArgs *__restrict__ meshes, const Tile *__restrict__ tiles, int ntiles, int *counter) {
   extern __shared__ __align__(16) unsigned char smem[];
-  frag_prologue<P, (MODE & kB16) != 0>(smem);
+  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) != 0>(smem);
   PairQueue gen{tiles, ntiles, counter, 0, 0, 0, false};
   frag_loop<P, MODE>(smem, gen, meshes[0], meshes);
 }
