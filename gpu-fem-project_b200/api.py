@@ -193,7 +193,18 @@ class Plan:
         if self.scheduled(strain, precision):
             return 1
         lay, _, pair_colours = self.layout()
-        return pair_colours if lay == "pairs" and self.fragment(strain, precision) else self.num_colours
+        if lay != "pairs" or not self.fragment(strain, precision):
+            return self.num_colours
+        _, strip_colours = self.strips()
+        if strip_colours:
+            return strip_colours if _strain(strain) == FEM_STRAIN_LINEAR else self.num_colours
+        return pair_colours
+
+    def strips(self):
+        """(strips, strip colours) of an order-3 plan's LINEAR Jacobian; (0, 0): none."""
+        n, c = C.c_int(), C.c_int()
+        check(lib.fem_plan_get_strips(self._h, C.byref(n), C.byref(c)), "fem_plan_get_strips")
+        return n.value, c.value
 
     def fragment(self, strain="linear", precision="fp64") -> bool:
         """Whether assemble() runs the warp-fragment kernel (orders 2-3, order 4 in

@@ -9,6 +9,20 @@
 
 namespace fem {
 
+namespace dev {
+// A strip of a plan's strip layout (HostPlan::strips): listed elements [begin, begin +
+// count), each the right neighbour of the one before; lead: id of the first element
+// that is not the halo.
+struct alignas(16) Strip {
+  int begin, count, flags, lead;
+};
+// Flags of a strip (kHalo, kRight) and of one of its steps: its first element is a halo,
+// assembled for its right edge only; its first element continues the strip and takes
+// the sums of its left edge from the element before it; its last element has a right
+// neighbour, which owns the edge between them.
+enum : int { kHalo = 1, kCarry = 2, kRight = 4 };
+}  // namespace dev
+
 // Records a message for fem_last_error() on this host thread and returns `status`.
 int fail(int status, const char *fmt, ...);
 void clear_error();
@@ -54,8 +68,24 @@ struct HostPlan {
   std::vector<int> pairColourPtr, pairList, pairConnList;
   std::vector<int> pairRegionEnd;  // per colour: the end of its pairs (its unpaired elements follow)
   std::vector<uint8_t> pairCode;
+  // Order kStripOrder: strip layout (LINEAR Jacobians, in the pair layout's place; the
+  // pair tables are then left out).  Chains of right neighbours are coloured so that the
+  // chains of one colour share no node and cut into strips.  The blocks of an edge's nodes among
+  // themselves and their residual rows belong to the element right of the edge; a strip
+  // that does not begin its chain lists the element before it first, as a halo whose
+  // share of the strip's left edge is assembled again, so the strips of a chain share no
+  // output and one launch takes all of a colour.  strips: by colour, ascending lead.
+  // Codes in list order (a halo's are unused); a block left to the right neighbour has
+  // the store flag, so that nothing is added there.
+  int numStripColours = 0;
+  std::vector<dev::Strip> strips;
+  std::vector<int> stripColourPtr, stripConn, stripLo, stripHi;  // Lo, Hi: node span per strip, halo included
+  std::vector<uint8_t> stripCode;
 };
+constexpr int kStripOrder = 3;
+constexpr int kStripWarps = 148 * 12;  // resident warps of the strip kernel
 constexpr int kRowChunkRows = 32, kRowChunkBlocks = 320;
-int build_host_plan(int order, int numNodes, const int *connPtr, const int *conn, int numElements, HostPlan &hp);
+int build_host_plan(int order, int numNodes, const int *connPtr, const int *conn, int numElements, HostPlan &hp,
+                    bool strips = true);
 
 }  // namespace fem

@@ -32,6 +32,7 @@
 #include <cstdint>
 #include <type_traits>
 
+#include "fem_common.h"
 #include "fem_umma.cuh"
 
 namespace fem {

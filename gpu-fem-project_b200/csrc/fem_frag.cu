@@ -113,7 +113,8 @@ struct FragLayout {
   static constexpr size_t wq = tabF + 16 * K4 * F::NTAB * F::TABW;  // double [NQP]
   static constexpr size_t csum = align16(wq + 8 * NQP);       // double2 [NQP]: sum_a dN(a, q)
   static constexpr size_t tabB = align16(csum + 16 * NQP);    // double2 [8][32]: BF16x6 stiffness operands
-  static constexpr size_t warps = align16(tabB + (B16 ? 16 * 8 * 32 : 0));
+  static constexpr size_t tabR = align16(tabB + (B16 ? 16 * 8 * 32 : 0));  // uint32 [64]: runs (order 3)
+  static constexpr size_t warps = align16(tabR + (P == 3 ? 4 * 64 : 0));
   // warp-relative; [2] = the two elements of the step, point q at slot(q) of PS
   static constexpr size_t WI0 = 0;                  // double2 [2][PS]: sqrt|s| (J^-1_0x, J^-1_1x)
   static constexpr size_t WI1 = WI0 + 16 * 2 * PS;  // double2 [2][PS]: sqrt|s| (J^-1_0y, J^-1_1y)
@@ -159,6 +160,28 @@ __device__ __forceinline__ void split3(double v, uint32_t &hi, uint32_t &mid, ui
   hi = __bfloat16_as_ushort(h);
   mid = __bfloat16_as_ushort(m);
   lo = __bfloat16_as_ushort(l);
+}
+
+// Run r of staging slot sl (see frag_slot): four blocks of one matrix row `row` with four
+// consecutive element-local columns from col0, staged from position pos0 of the slot.
+// Packed as row NN + col0 (a code record offset) | first staged double << 16.
+__device__ __forceinline__ uint32_t frag_run(int sl, int r) {
+  const int k = sl < 2 ? 0 : (sl < 6 ? 1 : 2);
+  const int h = sl < 2 ? sl : (sl < 6 ? (sl - 2) >> 1 : sl - 6);
+  const int w = (sl >= 2 && sl < 6) ? ((sl - 2) & 1) : 0;
+  const int TA = k == 2 ? 1 : 0, TB = k == 0 ? 0 : 1;
+  int row, col0, pos0;
+  if (w == 0) {
+    row = 8 * TA + 4 * (r & 1) + (r >> 1);  // pi(r)
+    col0 = 8 * TB + 4 * h;
+    pos0 = 4 * r;
+  } else {
+    const int tt = r >> 1, half = r & 1;
+    row = 8 * TB + 4 * h + tt;
+    col0 = 8 * TA + 4 * half;
+    pos0 = 8 * tt + 4 * half;
+  }
+  return (uint32_t)(row * 16 + col0) | (uint32_t)(128 * sl + 4 * pos0) << 16;
 }
 
 template <int P, bool B16 = false, bool NL = false>
@@ -213,6 +236,10 @@ __device__ __forceinline__ void frag_prologue(unsigned char *smem) {
       tabB[i] = (a < NN && q < NQ) ? dN(a, q) : make_double2(0.0, 0.0);
     }
   }
+  if constexpr (P == 3) {
+    for (int i = threadIdx.x; i < 64; i += blockDim.x)
+      reinterpret_cast<uint32_t *>(smem + L::tabR)[i] = frag_run(i >> 3, i & 7);
+  }
   // sum_a dN(a, q): zero in exact arithmetic, a few ulp of the table entries in
   // FP64; summed with Neumaier compensation (error ~1e-30 absolute) over the J-stage
   // table entries written above instead of evaluating the basis again
@@ -239,24 +266,53 @@ __device__ __forceinline__ void frag_prologue(unsigned char *smem) {
 // direct (0) / transposed (1) blocks.
 __host__ __device__ constexpr int frag_slot(int k, int h, int w) { return k == 0 ? h : (k == 1 ? 2 + 2 * h + w : 6 + h); }
 
-// The block (a, b) of element el (or its transpose (b, a) with w = 1): plan mode
-// stores it when this element is its first contributor; otherwise (and in
-// drop-in mode always) it goes to its staging position for frag_issue_run.
+// The block (a, b) of element el (or its transpose (b, a) with w = 1), where `act`: plan
+// mode stores it when this element is its first contributor (code bit 7, where `m80`
+// has it); otherwise (and in drop-in mode always) it goes to its staging position for
+// frag_issue_run.
+// Predicated, without a branch: the lanes of a warp mix the two.  Returns the code (0 in
+// drop-in mode), so that the caller knows whether any block was staged.
 template <int P, bool PLAN>
-__device__ __forceinline__ void frag_put(const Out &O, int el, int a, int b, int w, double kxx, double kxy,
-                                         double kyx, double kyy, double *stg) {
+__device__ __forceinline__ uint32_t frag_put(const Out &O, int el, int a, int b, int w, bool act, uint32_t m80, double kxx,
+                                             double kxy, double kyx, double kyy, double *stg) {
   constexpr int NN = Dims<P>::NN, CS = Dims<P>::CS;
   const int r0 = w ? b : a, c0 = w ? a : b;
   const double v0 = kxx, v1 = w ? kyx : kxy, v2 = w ? kxy : kyx, v3 = kyy;
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(stg);
   if constexpr (PLAN) {
-    const uint8_t code = O.codes[el * CS + r0 * NN + c0];
-    if (code & 0x80) {
-      store_block(O.mat + 4 * ((int64_t)O.rbase[el * NN + r0] + (code & 0x7f)), v0, v1, v2, v3);
-      return;
+    const uint32_t code = O.codes[el * CS + r0 * NN + c0];
+    double *blk = O.mat + 4 * ((int64_t)O.rbase[el * NN + r0] + (code & 0x7f));
+    asm volatile("{\n\t.reg .pred f, s;\n\t"
+                 "setp.ne.u32 f, %6, 0;\n\t"
+                 "setp.eq.and.u32 s, %7, 0, f;\n\t"
+                 "setp.ne.and.u32 f, %7, 0, f;\n\t"
+                 "@f st.global.v4.f64 [%0], {%2, %3, %4, %5};\n\t"
+                 "@s st.shared.v2.f64 [%1], {%2, %3};\n\t"
+                 "@s st.shared.v2.f64 [%1 + 16], {%4, %5};\n\t}" ::"l"(blk),
+                 "r"(sa), "d"(v0), "d"(v1), "d"(v2), "d"(v3), "r"((uint32_t)act), "r"(code & m80)
+                 : "memory");
+    return act ? code : 0x80u;
+  } else {
+    if (act) {
+      reinterpret_cast<double2 *>(stg)[0] = make_double2(v0, v1);
+      reinterpret_cast<double2 *>(stg)[1] = make_double2(v2, v3);
     }
+    return 0;
   }
-  reinterpret_cast<double2 *>(stg)[0] = make_double2(v0, v1);
-  reinterpret_cast<double2 *>(stg)[1] = make_double2(v2, v3);
+}
+
+// frag_put at order 3 with the code and the row's address in registers: one predicate.
+template <int OFF>
+__device__ __forceinline__ void frag_put_row(const double *row, uint32_t code, uint32_t m80, unsigned stg, double v0,
+                                             double v1, double v2, double v3) {
+  const double *blk = row + 4 * (code & 0x7f);
+  asm volatile("{\n\t.reg .pred f;\n\t"
+               "setp.ne.u32 f, %6, 0;\n\t"
+               "@f st.global.v4.f64 [%0], {%2, %3, %4, %5};\n\t"
+               "@!f st.shared.v2.f64 [%1 + %7], {%2, %3};\n\t"
+               "@!f st.shared.v2.f64 [%1 + %8], {%4, %5};\n\t}" ::"l"(blk),
+               "r"(stg), "d"(v0), "d"(v1), "d"(v2), "d"(v3), "r"(code & m80), "n"(OFF), "n"(OFF + 16)
+               : "memory");
 }
 
 // Before the second element of a step writes.  In a plan's pair layout it shares an
@@ -278,6 +334,19 @@ __device__ __forceinline__ void pair_order_fence() {
   pair_first_visible();
 }
 
+// A node's residual row: `act` lanes store it (first writer) or add to it, without a branch.
+__device__ __forceinline__ void residual_put(double *dst, bool act, bool first, double x, double y) {
+  asm volatile("{\n\t.reg .pred f, s;\n\t"
+               "setp.ne.u32 f, %3, 0;\n\t"
+               "setp.eq.and.u32 s, %4, 0, f;\n\t"
+               "setp.ne.and.u32 f, %4, 0, f;\n\t"
+               "@f st.global.v2.f64 [%0], {%1, %2};\n\t"
+               "@s red.global.add.f64 [%0], %1;\n\t"
+               "@s red.global.add.f64 [%0 + 8], %2;\n\t}" ::"l"(dst),
+               "d"(x), "d"(y), "r"((uint32_t)act), "r"((uint32_t)first)
+               : "memory");
+}
+
 __device__ __forceinline__ void bulk_add(double *gdst, const double *src, int bytes) {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(src);
   asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f64 [%0], [%1], %2;" ::"l"(gdst), "r"(sa),
@@ -285,51 +354,49 @@ __device__ __forceinline__ void bulk_add(double *gdst, const double *src, int by
                : "memory");
 }
 
-// Run r of staging slot sl (see frag_slot): four blocks of one matrix row with four
-// consecutive element-local columns.  Blocks to add: drop-in, every valid block;
-// plan, the valid blocks whose code is not a first store.  One 128-byte reduction
-// when all four are added and adjacent in the matrix, else 32 bytes per block
-// (four FP64 atomics for a block whose address is not 16-byte aligned).
+// Blocks of a run to add: drop-in, every block; plan, the blocks whose code is not a
+// first store.  One 128-byte reduction when all four are added and adjacent in the
+// matrix, else 32 bytes per block (four FP64 atomics for a block whose address is not
+// 16-byte aligned).  Order 3 (16 nodes: a run's four code bytes are one word).
 template <int P, bool PLAN>
-__device__ __forceinline__ void frag_issue_run(const Out &O, int el, int sl, int r, const double *redsW) {
+__device__ __forceinline__ void frag_issue_run(const Out &O, int el, uint32_t run, const double *redsW) {
   constexpr int NN = Dims<P>::NN, CS = Dims<P>::CS;
-  const int k = sl < 2 ? 0 : (sl < 6 ? 1 : 2);
-  const int h = sl < 2 ? sl : (sl < 6 ? (sl - 2) >> 1 : sl - 6);
-  const int w = (sl >= 2 && sl < 6) ? ((sl - 2) & 1) : 0;
-  const int TA = k == 2 ? 1 : 0, TB = k == 0 ? 0 : 1;
-  int row, col0, pos0;
-  if (w == 0) {
-    row = 8 * TA + 4 * (r & 1) + (r >> 1);  // pi(r)
-    col0 = 8 * TB + 4 * h;
-    pos0 = 4 * r;
-  } else {
-    const int tt = r >> 1, half = r & 1;
-    row = 8 * TB + 4 * h + tt;
-    col0 = 8 * TA + 4 * half;
-    pos0 = 8 * tt + 4 * half;
+  static_assert(NN == 16, "runs: order 3");
+  const int off = run & 0xffff, row = off >> 4, col0 = off & 15;
+  const double *src = redsW + (run >> 16);
+  if constexpr (PLAN) {
+    // most runs hold first stores only, most of the others add four adjacent blocks (or,
+    // where a strip leaves the run's last block to its right neighbour, three)
+    const uint32_t w4 = *reinterpret_cast<const uint32_t *>(O.codes + el * CS + off);
+    const uint32_t addm = ~w4 & 0x80808080u;
+    double *d0 = O.mat + 4 * ((int64_t)O.rbase[el * NN + row] + (w4 & 0x7f));
+    const bool four = addm == 0x80808080u && w4 == (w4 & 0xff) * 0x01010101u + 0x03020100u;
+    const bool three = addm == 0x00808080u && (w4 & 0xffffffu) == (w4 & 0xff) * 0x010101u + 0x020100u;
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "setp.ne.s32 p, %2, 0;\n\t"
+                 "@p cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f64 [%0], [%1], %2;\n\t}" ::"l"(d0),
+                 "r"((unsigned)__cvta_generic_to_shared(src)), "r"(four ? 128 : three ? 96 : 0)
+                 : "memory");
+    if (!__any_sync(0xffffffffu, addm != 0 && !four && !three)) return;
+    if (addm == 0 || four || three) return;
   }
-  if (row >= NN) return;
   double *dst[4];
   bool add[4];
   bool all = true, adj = true;
 #pragma unroll
   for (int j = 0; j < 4; j++) {
     const int col = col0 + j;
-    add[j] = col < NN;
-    dst[j] = O.mat;
-    if (add[j]) {
-      if constexpr (PLAN) {
-        const uint8_t code = O.codes[el * CS + row * NN + col];
-        add[j] = !(code & 0x80);
-        dst[j] = O.mat + 4 * ((int64_t)O.rbase[el * NN + row] + (code & 0x7f));
-      } else {
-        dst[j] = O.mat + O.map[(el * NN + row) * NN + col];
-      }
+    if constexpr (PLAN) {
+      const uint8_t code = O.codes[el * CS + row * NN + col];
+      add[j] = !(code & 0x80);
+      dst[j] = O.mat + 4 * ((int64_t)O.rbase[el * NN + row] + (code & 0x7f));
+    } else {
+      add[j] = true;
+      dst[j] = O.mat + O.map[(el * NN + row) * NN + col];
     }
     all = all && add[j];
     if (j > 0) adj = adj && dst[j] == dst[0] + 4 * j;
   }
-  const double *src = redsW + 128 * sl + 4 * pos0;
   if (all && adj && (reinterpret_cast<uintptr_t>(dst[0]) & 15u) == 0) {
     bulk_add(dst[0], src, 128);
     return;
@@ -348,83 +415,55 @@ __device__ __forceinline__ void frag_issue_run(const Out &O, int el, int sl, int
   }
 }
 
-// Per-block writers (order 2, where four consecutive element-local nodes straddle
-// grid rows and row runs never merge).  One 2x2 block of element `el` (staged codes /
-// row bases in O): a 256-bit store
-// when this element is the block's first contributor, else a 32-byte bulk
-// reduction from `slot` (this lane's staging slot; the caller has waited for the
-// slot's previous bulk read).  `which` = 1 writes the transposed block (b, a).
-template <int P>
-__device__ __forceinline__ void frag_write(const Out &O, int el, int a, int b, int which, double kxx, double kxy,
-                                           double kyx, double kyy, double *slot) {
+// Per-block writers (orders 2 and 4, where four consecutive element-local nodes straddle
+// grid rows and row runs rarely merge): block (r0, c0) of element `el`, where `act`.
+// Plan: the first contributor stores it, a later one stages it in `slot` (this lane's,
+// its previous bulk read complete) for bulk_add_block.  Drop-in: staged for the offset
+// of the reference map (accumulate-into contract; elements of one launch share blocks),
+// or added with four FP64 atomics when the block is not 16-byte aligned.  Without a
+// branch but for that case.  Returns whether it staged the block, with its address.
+template <int P, bool PLAN>
+__device__ __forceinline__ bool frag_put_block(const Out &O, int el, int r0, int c0, bool act, double v0, double v1,
+                                               double v2, double v3, double *slot, double *&blk) {
   constexpr int NN = Dims<P>::NN, CS = Dims<P>::CS;
-  const int r0 = which ? b : a, c0 = which ? a : b;
-  const double v0 = kxx, v1 = which ? kyx : kxy, v2 = which ? kxy : kyx, v3 = kyy;
-  const uint8_t code = O.codes[el * CS + r0 * NN + c0];
-  double *blk = O.mat + 4 * ((int64_t)O.rbase[el * NN + r0] + (code & 0x7f));
-  if (code & 0x80) {
-    store_block(blk, v0, v1, v2, v3);
+  if (!act) r0 = c0 = 0;
+  uint32_t first = 0;
+  bool add = act;
+  if constexpr (PLAN) {
+    const uint32_t code = O.codes[el * CS + r0 * NN + c0];
+    blk = O.mat + 4 * ((int64_t)O.rbase[el * NN + r0] + (code & 0x7f));
+    first = code & 0x80;
+    add = act && !first;
   } else {
-    reinterpret_cast<double2 *>(slot)[0] = make_double2(v0, v1);
-    reinterpret_cast<double2 *>(slot)[1] = make_double2(v2, v3);
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(slot);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f64 [%0], [%1], 32;" ::"l"(blk), "r"(sa)
-                 : "memory");
-    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    blk = O.mat + O.map[(el * NN + r0) * NN + c0];
+    if ((reinterpret_cast<uintptr_t>(blk) & 15u) != 0) {
+      if (act) {
+        atomicAdd(blk + 0, v0);
+        atomicAdd(blk + 1, v1);
+        atomicAdd(blk + 2, v2);
+        atomicAdd(blk + 3, v3);
+      }
+      add = false;
+    }
   }
-}
-
-// frag_write without its fence and bulk reduction: a first store goes out at once
-// (returns nullptr); a block to add is staged in `slot` and its destination
-// returned, for the caller to issue after one proxy fence for all its slots.
-template <int P>
-__device__ __forceinline__ double *frag_stage(const Out &O, int el, int a, int b, int which, double kxx, double kxy,
-                                              double kyx, double kyy, double *slot) {
-  constexpr int NN = Dims<P>::NN, CS = Dims<P>::CS;
-  const int r0 = which ? b : a, c0 = which ? a : b;
-  const double v0 = kxx, v1 = which ? kyx : kxy, v2 = which ? kxy : kyx, v3 = kyy;
-  const uint8_t code = O.codes[el * CS + r0 * NN + c0];
-  double *blk = O.mat + 4 * ((int64_t)O.rbase[el * NN + r0] + (code & 0x7f));
-  if (code & 0x80) {
-    store_block(blk, v0, v1, v2, v3);
-    return nullptr;
-  }
-  reinterpret_cast<double2 *>(slot)[0] = make_double2(v0, v1);
-  reinterpret_cast<double2 *>(slot)[1] = make_double2(v2, v3);
-  return blk;
-}
-
-__device__ __forceinline__ void bulk_add32(double *blk, const double *slot) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(slot);
-  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f64 [%0], [%1], 32;" ::"l"(blk), "r"(sa)
+  asm volatile("{\n\t.reg .pred f, s;\n\t"
+               "setp.ne.u32 f, %6, 0;\n\t"
+               "setp.ne.u32 s, %7, 0;\n\t"
+               "@f st.global.v4.f64 [%0], {%2, %3, %4, %5};\n\t"
+               "@s st.shared.v2.f64 [%1], {%2, %3};\n\t"
+               "@s st.shared.v2.f64 [%1 + 16], {%4, %5};\n\t}" ::"l"(blk),
+               "r"((unsigned)__cvta_generic_to_shared(slot)), "d"(v0), "d"(v1), "d"(v2), "d"(v3),
+               "r"(act ? first : 0u), "r"((uint32_t)add)
                : "memory");
+  return add;
 }
 
-// Drop-in mode: element `el`'s 2x2 block added at the reference map's offset
-// (accumulate-into contract; elements of one launch share blocks), one 32-byte bulk
-// reduction when the block address is 16-byte aligned, else four FP64 atomics.
-template <int P>
-__device__ __forceinline__ void frag_add_mapped(const Out &O, int el, int a, int b, int which, double kxx,
-                                                double kxy, double kyx, double kyy, double *slot) {
-  constexpr int NN = Dims<P>::NN;
-  const int r0 = which ? b : a, c0 = which ? a : b;
-  const double v0 = kxx, v1 = which ? kyx : kxy, v2 = which ? kxy : kyx, v3 = kyy;
-  double *blk = O.mat + O.map[(el * NN + r0) * NN + c0];
-  if ((reinterpret_cast<uintptr_t>(blk) & 15u) == 0) {
-    reinterpret_cast<double2 *>(slot)[0] = make_double2(v0, v1);
-    reinterpret_cast<double2 *>(slot)[1] = make_double2(v2, v3);
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(slot);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f64 [%0], [%1], 32;" ::"l"(blk), "r"(sa)
-                 : "memory");
-    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-  } else {
-    atomicAdd(blk + 0, v0);
-    atomicAdd(blk + 1, v1);
-    atomicAdd(blk + 2, v2);
-    atomicAdd(blk + 3, v3);
-  }
+__device__ __forceinline__ void bulk_add_block(double *blk, const double *slot, bool add) {
+  asm volatile("{\n\t.reg .pred p;\n\t"
+               "setp.ne.u32 p, %2, 0;\n\t"
+               "@p cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f64 [%0], [%1], 32;\n\t}" ::"l"(blk),
+               "r"((unsigned)__cvta_generic_to_shared(slot)), "r"((uint32_t)add)
+               : "memory");
 }
 
 // The element pairs a warp assembles, in order.
@@ -434,11 +473,13 @@ struct PairCursor {
   int64_t k0;
   int tile = -1;      // dependency-ordered launches: the pair's tile
   bool last = false;  // ... and whether it is the tile's last pair
+  int fl = 0;         // strips: kHalo | kCarry | kRight
 };
+
 
 // Single mesh: pairs p, p + stride, ... of list positions [begin, end).
 struct PairStride {
-  static constexpr bool kBatched = false, kSched = false;
+  static constexpr bool kBatched = false, kSched = false, kStrip = false;
   int64_t begin, end, p, stride;
   __device__ PairCursor next(int) {
     PairCursor c{0, 0, begin + 2 * p};
@@ -452,7 +493,7 @@ struct PairStride {
 // launches of fem_plan_assemble_host that share a schedule step): pairs p, p +
 // stride, ... of their concatenation; a pair never straddles two ranges.
 struct PairRanges {
-  static constexpr bool kBatched = false, kSched = false;
+  static constexpr bool kBatched = false, kSched = false, kStrip = false;
   RangeList r;
   int64_t p, stride;
   __device__ PairCursor next(int) {
@@ -472,11 +513,55 @@ struct PairRanges {
   }
 };
 
+// One mesh, strips (HostPlan::strips) of up to kMaxRanges ranges of one launch: a warp
+// takes strips p, p + stride, ... of their concatenation whole, two listed elements per
+// step; the next strip's header is read one strip ahead.
+struct StripRanges {
+  static constexpr bool kBatched = false, kSched = false, kStrip = true;
+  const Strip *strips;
+  const RangeList &r;  // the kernel's __grid_constant__ parameter
+  int64_t p, stride;
+  Strip ahead{0, 0, 0, 0};
+  int pos = 0, end = 0, flags = 0;
+  __device__ void fetch() {
+    ahead.count = 0;
+    int64_t q = p;
+#pragma unroll
+    for (int i = 0; i < kMaxRanges; i++) {
+      if (i >= r.n) break;
+      if (q < r.count[i]) {
+        const int4 v = __ldg(reinterpret_cast<const int4 *>(strips + r.begin[i] + q));
+        ahead = Strip{v.x, v.y, v.z, v.w};
+        break;
+      }
+      q -= r.count[i];
+    }
+    p += stride;
+  }
+  __device__ PairCursor next(int) {
+    PairCursor c{0, 0, 0};
+    int fl = kCarry;
+    if (pos >= end) {
+      if (ahead.count == 0) return c;
+      pos = ahead.begin;
+      end = ahead.begin + ahead.count;
+      flags = ahead.flags;
+      fl = (flags & kHalo);
+      fetch();
+    }
+    c.k0 = pos;
+    c.ne = min(2, end - pos);
+    pos += c.ne;
+    c.fl = fl | ((pos < end || (flags & kRight)) ? kRight : 0);
+    return c;
+  }
+};
+
 // Many meshes: the pairs of the tiles this warp pulls from the launch's queue
 // (one atomic counter per launch; tiles hold even element counts except at the
 // end of a colour range, so pairs never straddle tiles).
 struct PairQueue {
-  static constexpr bool kBatched = true, kSched = false;
+  static constexpr bool kBatched = true, kSched = false, kStrip = false;
   const Tile *tiles;
   int ntiles;
   int *counter;
@@ -557,7 +642,7 @@ __device__ __noinline__ void sched_wait(const SchedArgs *S, int g) {
 // every CTA of the grid is resident.
 template <bool BATCHED>
 struct PairSchedT {
-  static constexpr bool kBatched = BATCHED, kSched = true;
+  static constexpr bool kBatched = BATCHED, kSched = true, kStrip = false;
   const SchedArgs *S;  // the kernel's __grid_constant__ parameter
   int tile = -1, held = -1, mesh = 0;
   int64_t pos = 0, tend = 0;
@@ -618,6 +703,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
   constexpr bool NL = (MODE & kNL) != 0;
   constexpr bool B16 = (MODE & kB16) != 0;  // BF16x6 element stiffness
   using F = FragDims<P>;
+  constexpr bool STRIP = Gen::kStrip;
   using L = FragLayout<P, !PLAN, NL, B16, (MODE & kJac) != 0>;
   constexpr int NN = F::NN, NQ = F::NQ, K4 = F::K4, QT = F::QT, NTN = F::NTN, NQP = F::NQP, PS = L::PS, CS = F::CS;
   constexpr int STG = L::CS;  // staged bytes per element: plan code record or map rows
@@ -625,6 +711,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
   constexpr bool RUNS = (P == 3);  // order 3: staged row runs, one bulk reduction per adjacent run
   static_assert(!NL || !F::IL, "NONLINEAR strain: orders 2 and 3");
   static_assert(PLAN || !Gen::kBatched, "drop-in mode assembles one mesh");
+  static_assert(!STRIP || (PLAN && JAC && !NL && P == kStripOrder), "strips: LINEAR Jacobians of plans, order 3");
   static_assert(!B16 || (!NL && P == 3), "BF16x6 stiffness: LINEAR, order 3");
   // LINEAR FP64: mu is folded into the gradients (G-hat carries sqrt|s mu|), so a block
   // is four FMAs of M with the one constant lam / mu.  (B16 keeps sqrt|s|: the BF16
@@ -639,6 +726,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
   const double *wqs = reinterpret_cast<const double *>(smem + L::wq);
   const double2 *csum = reinterpret_cast<const double2 *>(smem + L::csum);
   const double2 *tabB = reinterpret_cast<const double2 *>(smem + L::tabB);
+  const uint32_t *tabR = reinterpret_cast<const uint32_t *>(smem + L::tabR);
   unsigned char *ws = smem + L::warps + warp * L::warp_bytes;
   double2 *WI0 = reinterpret_cast<double2 *>(ws + L::WI0);
   double2 *WI1 = reinterpret_cast<double2 *>(ws + L::WI1);
@@ -651,6 +739,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
   unsigned char *stage = ws + L::STAGE;
   double *redsW = reinterpret_cast<double *>(ws + L::REDS);  // staging slot s at redsW + 128 s
   double *ATs = reinterpret_cast<double *>(ws + L::AT);      // NONLINEAR tangent
+  double crx = 0.0, cry = 0.0;                               // strips: carried residual rows
 
   // Mesh arguments are read through `mtab` (for one mesh, a pointer to the kernel
   // parameter).  At p = 4 it is laundered once per step: the compiler then reloads
@@ -689,7 +778,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
         const AsmArgs &M = args(c);
         const double *src = c_ld < 2 ? M.coords : M.states;
         val[ks] = __ldg(src + 2 * (int64_t)node[ks] + (c_ld & 1));
-        if (PLAN && JAC && c_ld == 1) rbv[ks] = __ldg(M.rowp + node[ks]);
+        if (PLAN && JAC) rbv[ks] = __ldg(M.rowp + node[ks]);
       }
     }
   };
@@ -751,10 +840,9 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
     for (int ks = 0; ks < K4; ks++) {
       val[ks] = valB[ks];
       const int a = 4 * ks + t;
-      if (nodeB[ks] >= 0) {
-        if (c_ld == 0) nid[e_ld * NN + a] = nodeB[ks];
-        if (PLAN && JAC && c_ld == 1) rb[e_ld * NN + a] = rbB[ks];
-      }
+      // nid by the lanes of component 0, rb by those of component 1
+      if (nodeB[ks] >= 0 && c_ld < (PLAN && JAC ? 2 : 1))
+        (c_ld == 0 ? nid : rb)[e_ld * NN + a] = c_ld == 0 ? nodeB[ks] : rbB[ks];
     }
     cp_async_wait_all();
     __syncwarp();
@@ -928,6 +1016,36 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
         kyx = lam * myx + mu * mxy, kyy = c11 * myy + mu * mxx;
       }
     };
+    // order 3: the staged blocks of an element leave as row runs, two per lane, after one
+    // proxy fence; nothing to do when no lane staged any (a launch of first contributors)
+    auto issue_runs = [&](const Out &out, int el, bool staged) {
+      if (!__any_sync(0xffffffffu, staged)) return;
+      if (PLAN && !STRIP && el > 0) pair_first_landed();
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (PLAN && !STRIP && el > 0) pair_first_visible();
+#pragma unroll
+      for (int u = 0; u < 2; u++) if constexpr (RUNS) frag_issue_run<P, PLAN>(out, el, tabR[lane + 32 * u], redsW);
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    };
+    // all k-steps; the form with the points' signs is rarely run and stays rolled
+    auto kstep_all = [&](auto &kstep, bool neg) {
+      if (SCALED && neg) {
+        kstep(0, std::true_type{}, std::true_type{});
+#pragma unroll 1
+        for (int ks = 1; ks < K4; ks++) kstep(ks, std::false_type{}, std::true_type{});
+      } else {
+        kstep(0, std::true_type{}, std::false_type{});
+#pragma unroll
+        for (int ks = 1; ks < K4; ks++) kstep(ks, std::false_type{}, std::false_type{});
+      }
+    };
+    // strips: the right edge's residual rows go to the next element's left edge
+    auto residual_carry = [&](double &sx, double &sy, bool in) {
+      if (in && g < 2) sx += crx, sy += cry;
+      crx = __shfl_down_sync(0xffffffffu, sx, 24);
+      cry = __shfl_down_sync(0xffffffffu, sy, 24);
+    };
     if constexpr (!F::IL) {
       // node tiles on the tensor cores: both at p = 3; at p = 2 only tile 0 (nodes 0-7),
       // node 8 (alone in tile 1) has its row and column on the FP64 pipe (12 instead of
@@ -936,8 +1054,20 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
       constexpr int NPAIR = NTM * (NTM + 1) / 2;
       const int pa = 4 * (g & 1) + (g >> 1);  // pi(g)
       for (int el = 0; el < ne; el++) {
+        // Strips: the blocks of an edge's nodes among themselves and their residual rows
+        // belong to the element right of it; lanes (g = 6, 7; t = 3) hold exactly those
+        // blocks of an element's right edge, lanes (g = 0, 1; t = 0) its left edge's, in
+        // the same order.
+        const bool halo = STRIP && el == 0 && (cur.fl & kHalo);
+        const bool cin = STRIP && (el > 0 || (cur.fl & kCarry));
+        const bool right = STRIP && (el + 1 < ne || (cur.fl & kRight));
+        // The give lanes stage their blocks like blocks to add (which the codes say they are
+        // not, so no run takes them), the take lanes of the next element add them from
+        // there; a halo stages everything and issues nothing.
+        const bool give = STRIP && right && (lane & ~4) == 27, take = STRIP && cin && (lane & ~4) == 0;
+        const uint32_t m80 = give || halo ? 0u : 0x80u;
         // pair layout: the first element's residual writes before the second's
-        if (PLAN && el > 0) __syncwarp();
+        if (PLAN && !STRIP && el > 0) __syncwarp();
         if constexpr (B16) {
           // BF16x6 element stiffness: M_ij = sum_q s G_i(q, a) G_j(q, b) as m16n8k16
           // products (k = quadrature points 0-15; rows a and columns b of the two node
@@ -982,15 +1112,12 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
               ry[h] += __shfl_xor_sync(0xffffffffu, ry[h], 2);
             }
             const int a = 8 * t + pa;
-            if (t < 2 && a < NN) {
-              const double sx = t ? rx[1] : rx[0], sy = t ? ry[1] : ry[0];
-              double *dst = M.residual + 2 * (int64_t)nid[el * NN + a];
-              if (PLAN && O.codes[el * CS + NN * NN + a]) {
-                *reinterpret_cast<double2 *>(dst) = make_double2(sx, sy);
-              } else {
-                atomicAdd(dst, sx);
-                atomicAdd(dst + 1, sy);
-              }
+            double sx = t ? rx[1] : rx[0], sy = t ? ry[1] : ry[0];
+            if constexpr (STRIP) residual_carry(sx, sy, cin);
+            {
+              const bool act = t < 2 && !halo && !(right && g >= 6);
+              const int an = t < 2 ? a : 0;
+              residual_put(M.residual + 2 * (int64_t)nid[el * NN + an], act, PLAN && O.codes[el * CS + NN * NN + an], sx, sy);
             }
           }
           if constexpr (JAC) {
@@ -1042,6 +1169,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
             // the pair (1, 0) is the transposed half of (0, 1)) and leave as row runs.
             asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
             __syncwarp();
+            uint32_t allfirst = 0x80u;
 #pragma unroll
             for (int r = 0; r < 2; r++)
 #pragma unroll
@@ -1049,26 +1177,24 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
 #pragma unroll
                 for (int u = 0; u < 2; u++) {
                   const int a = 8 * r + pa, b = 8 * h + 4 * u + t, c = 2 * r + u;
-                  if (a < NN && b < NN) {
+                  {
                     const double mxx = acc[0][0][h][c], mxy = acc[0][1][h][c];
                     const double myx = acc[1][0][h][c], myy = acc[1][1][h][c];
                     double kxx, kxy, kyx, kyy;
                     block(mxx, mxy, myx, myy, kxx, kxy, kyx, kyy);
                     const int sl = (r == 1 && h == 0) ? frag_slot(1, g & 1, 1) : frag_slot(r + h, u, 0);
                     const int pos = (r == 1 && h == 0) ? 8 * (g >> 1) + 4 * u + t : 4 * g + t;
-                    frag_put<P, PLAN>(O, el, a, b, 0, kxx, kxy, kyx, kyy, redsW + 128 * sl + 4 * pos);
+                    double *stg = redsW + 128 * sl + 4 * pos;
+                    if (take) {  // from lane + 27's staging position
+                      const double *cs = stg + 4 * (r == 1 && h == 0 ? 8 * 3 + 3 : 27);
+                      kxx += cs[0], kxy += cs[1];
+                      kyx += cs[2], kyy += cs[3];
+                    }
+                    if constexpr (STRIP) __syncwarp();
+                    allfirst &= frag_put<P, PLAN>(O, el, a, b, 0, true, m80, kxx, kxy, kyx, kyy, stg);
                   }
                 }
-            if (PLAN && el > 0) pair_first_landed();
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (PLAN && el > 0) pair_first_visible();
-#pragma unroll
-            for (int v = 0; v < 2; v++) {
-              const int run = lane + 32 * v;
-              frag_issue_run<P, PLAN>(O, el, run >> 3, run & 7, redsW);
-            }
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            issue_runs(O, el, !halo && (allfirst & 0x80u) == 0);
           }
           continue;
         }
@@ -1078,19 +1204,13 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
         double acc[NPAIR][4][2];
         double rp[NTN][2];
         double n8[4] = {0.0, 0.0, 0.0, 0.0}, d8[4] = {0.0, 0.0, 0.0, 0.0};  // p = 2: M[8][pi(g)], M[8][8]
-        if constexpr (NL) {
-  #pragma unroll
-          for (int k = 0; k < NPAIR; k++)
-  #pragma unroll
-            for (int c = 0; c < 4; c++) acc[k][c][0] = acc[k][c][1] = 0.0;
-        }
   #pragma unroll
         for (int T = 0; T < NTN; T++) rp[T][0] = rp[T][1] = 0.0;
         // whether a point of this element has s (mu) < 0 (inverted element or negative
         // thickness or modulus): only then do the A fragments take the points' signs
         const bool neg = SCALED && (negm & (el ? 0xccccccccu : 0x33333333u)) != 0;
-  #pragma unroll
-        for (int ks = 0; ks < K4; ks++) {
+        auto kstep = [&](int ks, auto firstc, auto negc) {
+          constexpr bool FIRST = decltype(firstc)::value, NEG = decltype(negc)::value;
           const int o = el * PS + L::slot(4 * ks) + t;
           const double2 w0 = WI0[o], w1 = WI1[o];
           double fr[NTN][2];
@@ -1136,7 +1256,8 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
 #pragma unroll
                   for (int ik = 0; ik < 4; ik++) {
                     const double bv = fma(C[ik >> 1][ik & 1][0], fr[TB][0], C[ik >> 1][ik & 1][1] * fr[TB][1]);
-                    dmma(acc[k][ik][0], acc[k][ik][1], fr[TA][ll], bv);
+                    if (FIRST && ll == 0) dmma_first(acc[k][ik][0], acc[k][ik][1], fr[TA][ll], bv);
+                    else dmma(acc[k][ik][0], acc[k][ik][1], fr[TA][ll], bv);
                   }
                 }
               }
@@ -1153,7 +1274,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
           if constexpr (JAC && P == 2 && !NL) {
             // G-hat_i(q, 8) sits in lane (g = 0, t), tile 1
             const double h0 = __shfl_sync(0xffffffffu, fr[1][0], t), h1 = __shfl_sync(0xffffffffu, fr[1][1], t);
-            const double s0 = neg ? SGs[el * NQP + 4 * ks + t] * h0 : h0, s1 = neg ? SGs[el * NQP + 4 * ks + t] * h1 : h1;
+            const double s0 = NEG ? SGs[el * NQP + 4 * ks + t] * h0 : h0, s1 = NEG ? SGs[el * NQP + 4 * ks + t] * h1 : h1;
             n8[0] = fma(s0, fr[0][0], n8[0]);
             n8[1] = fma(s0, fr[0][1], n8[1]);
             n8[2] = fma(s1, fr[0][0], n8[2]);
@@ -1168,13 +1289,13 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
   #pragma unroll
             for (int TA = 0; TA < NTM; TA++) {
               double a0 = fr[TA][0], a1 = fr[TA][1];
-              if (neg) {
+              if constexpr (NEG) {
                 a0 *= SGs[el * NQP + 4 * ks + t];
                 a1 *= SGs[el * NQP + 4 * ks + t];
               }
   #pragma unroll
               for (int TB = TA; TB < NTM; TB++, k++) {
-                if (ks == 0) {
+                if constexpr (FIRST) {
                   dmma_first(acc[k][0][0], acc[k][0][1], a0, fr[TB][0]);
                   dmma_first(acc[k][1][0], acc[k][1][1], a0, fr[TB][1]);
                   dmma_first(acc[k][2][0], acc[k][2][1], a1, fr[TB][0]);
@@ -1188,7 +1309,8 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
               }
             }
           }
-        }
+        };
+        kstep_all(kstep, neg);
         // residual: sum over the four lanes t of a node (reduce-scatter over node tiles)
         if constexpr (RES) {
           const int Tm = t >> 1, To = Tm ^ 1;
@@ -1196,91 +1318,143 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
           double sy = (Tm ? rp[1][1] : rp[0][1]) + __shfl_xor_sync(0xffffffffu, To ? rp[1][1] : rp[0][1], 2);
           sx += __shfl_xor_sync(0xffffffffu, sx, 1);
           sy += __shfl_xor_sync(0xffffffffu, sy, 1);
+          if constexpr (STRIP) residual_carry(sx, sy, cin);
           const int a = 8 * Tm + pa;
-          if ((t & 1) == 0 && a < NN) {
-            double *dst = M.residual + 2 * (int64_t)nid[el * NN + a];
-            if (PLAN && O.codes[el * CS + NN * NN + a]) {
-              *reinterpret_cast<double2 *>(dst) = make_double2(sx, sy);
-            } else {
-              atomicAdd(dst, sx);
-              atomicAdd(dst + 1, sy);
-            }
-          }
+          const bool act = (t & 1) == 0 && a < NN && !halo && !(right && g >= 6);
+          const int an = a < NN ? a : 0;
+          residual_put(M.residual + 2 * (int64_t)nid[el * NN + an], act, PLAN && O.codes[el * CS + NN * NN + an], sx, sy);
         }
-        // stiffness blocks, order 3: lane (g, t) holds (a = 8TA + pi(g), b = 8TB + 4h + t).  Blocks that
-        // are added (drop-in: all; plan: later colours) are staged so that each row run of
-        // four consecutive columns is contiguous in shared memory -- slot s = (pair, h,
-        // direct/transposed), direct position 4g + t (row a, columns 8TB + 4h + 0..3),
-        // transposed position 8t + pi(g) (row b, columns 8TA + 4*half + 0..3) -- and then
-        // reduced with one 128-byte bulk operation per run whose four blocks are adjacent in
-        // the matrix, else one 32-byte operation per block.
         if constexpr (JAC && RUNS) {
+          // acc becomes the blocks (xx, xy, yx, yy)
+  #pragma unroll
+          for (int k = 0; k < NPAIR; k++)
+  #pragma unroll
+            for (int h = 0; h < 2; h++) {
+              double kxx, kxy, kyx, kyy;
+              block(acc[k][0][h], acc[k][1][h], acc[k][2][h], acc[k][3][h], kxx, kxy, kyx, kyy);
+              acc[k][0][h] = kxx, acc[k][1][h] = kxy, acc[k][2][h] = kyx, acc[k][3][h] = kyy;
+            }
           // every lane's previous bulk reads of the staging slots are complete
           asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
           __syncwarp();
-          int k = 0;
+          double *stg = redsW + 4 * lane;  // direct blocks: position 4g + t of their slot
+          if constexpr (STRIP) {
+            if (take) {
   #pragma unroll
-          for (int TA = 0; TA < NTN; TA++) {
+              for (int k = 0; k < NPAIR; k++)
   #pragma unroll
-            for (int TB = TA; TB < NTN; TB++, k++) {
-              const int a = 8 * TA + pa;
+                for (int h = 0; h < 2; h++) {
+                  const double2 *cs = reinterpret_cast<const double2 *>(stg + 128 * frag_slot(k, h, 0) + 4 * 27);
+                  acc[k][0][h] += cs[0].x, acc[k][1][h] += cs[0].y;
+                  acc[k][2][h] += cs[1].x, acc[k][3][h] += cs[1].y;
+                }
+            }
+            __syncwarp();
+          }
+          uint32_t allfirst = 0x80u;
+          if constexpr (PLAN && !NL) {
+            // the lane's code bytes and row addresses first: rows pi(g) and 8 + pi(g) hold
+            // its direct blocks, rows 8 + 4h + t the transposed ones of pair (0, 1)
+            const uint8_t *rec = O.codes + el * CS;
+            const int *rbe = O.rbase + el * NN;
+            uint32_t cd[NPAIR][2], ct[2];
   #pragma unroll
-              for (int h = 0; h < 2; h++) {
-                const int b = 8 * TB + 4 * h + t;
-                if (a < NN && b < NN) {
-                  const double mxx = acc[k][0][h], mxy = acc[k][1][h], myx = acc[k][2][h], myy = acc[k][3][h];
-                  double kxx, kxy, kyx, kyy;
-                  block(mxx, mxy, myx, myy, kxx, kxy, kyx, kyy);
-                  const int s0 = frag_slot(k, h, 0);
+            for (int k = 0; k < NPAIR; k++)
+  #pragma unroll
+              for (int h = 0; h < 2; h++) cd[k][h] = rec[pa * NN + t + (k == 2 ? 8 * NN : 0) + (k == 0 ? 0 : 8) + 4 * h];
+  #pragma unroll
+            for (int h = 0; h < 2; h++) ct[h] = rec[t * NN + pa + (8 + 4 * h) * NN];
+            const double *r0 = O.mat + 4 * (int64_t)rbe[pa], *r1 = O.mat + 4 * (int64_t)rbe[8 + pa];
+            const double *rt0 = O.mat + 4 * (int64_t)rbe[8 + t], *rt1 = O.mat + 4 * (int64_t)rbe[12 + t];
+            const unsigned sd = (unsigned)__cvta_generic_to_shared(stg);
+            const unsigned st = (unsigned)__cvta_generic_to_shared(redsW + 4 * (8 * t + pa));
+            auto direct = [&](auto kc, auto hc) {
+              constexpr int k = decltype(kc)::value, h = decltype(hc)::value;
+              frag_put_row<1024 * frag_slot(k, h, 0)>(k == 2 ? r1 : r0, cd[k][h], m80, sd, acc[k][0][h], acc[k][1][h],
+                                                      acc[k][2][h], acc[k][3][h]);
+              allfirst &= cd[k][h];
+            };
+            direct(IC<0>{}, IC<0>{});
+            direct(IC<0>{}, IC<1>{});
+            direct(IC<1>{}, IC<0>{});
+            direct(IC<1>{}, IC<1>{});
+            frag_put_row<1024 * frag_slot(1, 0, 1)>(rt0, ct[0], m80, st, acc[1][0][0], acc[1][2][0], acc[1][1][0], acc[1][3][0]);
+            frag_put_row<1024 * frag_slot(1, 1, 1)>(rt1, ct[1], m80, st, acc[1][0][1], acc[1][2][1], acc[1][1][1], acc[1][3][1]);
+            direct(IC<2>{}, IC<0>{});
+            direct(IC<2>{}, IC<1>{});
+            allfirst &= ct[0] & ct[1];
+          } else {
+            int k = 0;
+  #pragma unroll
+            for (int TA = 0; TA < NTN; TA++) {
+  #pragma unroll
+              for (int TB = TA; TB < NTN; TB++, k++) {
+                const int a = 8 * TA + pa;
+  #pragma unroll
+                for (int h = 0; h < 2; h++) {
+                  const int b = 8 * TB + 4 * h + t;
+                  const double kxx = acc[k][0][h], kxy = acc[k][1][h], kyx = acc[k][2][h], kyy = acc[k][3][h];
+                  // NONLINEAR diagonal tiles: (a, b) for a <= b and, for a < b, its exact
+                  // transpose (b, a) at the staging position the (b, a) lane would use
+                  const bool diag = NL && TA == TB;
+                  allfirst &= frag_put<P, PLAN>(O, el, a, b, 0, !diag || a <= b, m80, kxx, kxy, kyx, kyy,
+                                                stg + 128 * frag_slot(k, h, 0));
                   if (TA < TB) {
-                    const int s1 = frag_slot(k, h, 1);
-                    frag_put<P, PLAN>(O, el, a, b, 0, kxx, kxy, kyx, kyy, redsW + 128 * s0 + 4 * (4 * g + t));
-                    frag_put<P, PLAN>(O, el, a, b, 1, kxx, kxy, kyx, kyy, redsW + 128 * s1 + 4 * (8 * t + pa));
-                  } else if (!NL) {
-                    frag_put<P, PLAN>(O, el, a, b, 0, kxx, kxy, kyx, kyy, redsW + 128 * s0 + 4 * (4 * g + t));
-                  } else if (a <= b) {
-                    // NONLINEAR diagonal tile: (a, b) for a <= b and, for a < b, its exact
-                    // transpose (b, a) at the staging position the (b, a) lane would use
-                    frag_put<P, PLAN>(O, el, a, b, 0, kxx, kxy, kyx, kyy, redsW + 128 * s0 + 4 * (4 * g + t));
-                    if (a < b) {
-                      const int xb = b - 8 * TA, xa = a - 8 * TA;  // pi(g') = xb; a = 8T + 4h' + t'
-                      const int gb = 2 * (xb & 3) + (xb >> 2);
-                      const int st = frag_slot(k, xa >> 2, 0);
-                      frag_put<P, PLAN>(O, el, a, b, 1, kxx, kxy, kyx, kyy, redsW + 128 * st + 4 * (4 * gb + (xa & 3)));
-                    }
+                    allfirst &= frag_put<P, PLAN>(O, el, a, b, 1, true, m80, kxx, kxy, kyx, kyy,
+                                                  redsW + 128 * frag_slot(k, h, 1) + 4 * (8 * t + pa));
+                  } else if (diag) {
+                    const int xb = b - 8 * TA, xa = a - 8 * TA;  // pi(g') = xb; a = 8T + 4h' + t'
+                    const int gb = 2 * (xb & 3) + (xb >> 2);
+                    allfirst &= frag_put<P, PLAN>(O, el, a, b, 1, a < b, m80, kxx, kxy, kyx, kyy,
+                                                  redsW + 128 * frag_slot(k, xa >> 2, 0) + 4 * (4 * gb + (xa & 3)));
                   }
                 }
               }
             }
           }
-          if (PLAN && el > 0) pair_first_landed();
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          __syncwarp();
-          if (PLAN && el > 0) pair_first_visible();
-          // 64 runs (8 slots x 8 runs), two per lane
-  #pragma unroll
-          for (int u = 0; u < 2; u++) {
-            const int run = lane + 32 * u;
-            frag_issue_run<P, PLAN>(O, el, run >> 3, run & 7, redsW);
-          }
-          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          issue_runs(O, el, !halo && (allfirst & 0x80u) == 0);
         }
-        // stiffness blocks, order 2 (plan, LINEAR): lane (g, t) writes (pi(g), 4h + t),
-        // h = 0, 1, and lanes t < 2 / (g = 0, t = 2) a node-8 block; first stores go out
-        // at once, the blocks to add are staged in slots 0-2 and leave after one proxy
-        // fence, as one bulk group (a fence per block cost 5 % of the order-2 time)
-        if constexpr (JAC && !RUNS && PLAN && !NL && P == 2) {
-          if (el > 0) pair_order_fence();
+        // stiffness blocks, order 2: lane (g, t) writes (pi(g), 4h + t), h = 0, 1 (NONLINEAR:
+        // for a <= b, and the exact transpose), and lanes t < 2 / (g = 0, t = 2) a node-8
+        // block: (8, pi(g)), its transpose, (8, 8); first stores go out at once, the blocks
+        // to add are staged and leave after one proxy fence, as one bulk group (a fence
+        // per block cost 5 % of the order-2 time; NONLINEAR: three groups, for registers)
+        if constexpr (JAC && P == 2) {
           asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
           double *reds = redsW + 4 * lane;
-          double *dst[3] = {nullptr, nullptr, nullptr};
+          double *dst[3];
+          bool add[3] = {false, false, false};
+          double kxx, kxy, kyx, kyy;
+          auto issue = [&](int s0, int s1) {  // the staged blocks of slots [s0, s1)
+            bool any = false;
+#pragma unroll
+            for (int x = 0; x < 3; x++) any = any || (x >= s0 && x < s1 && add[x]);
+            if (!__any_sync(0xffffffffu, any)) return;
+            if (PLAN && el > 0) pair_first_landed();
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            if (PLAN && el > 0) {
+              __syncwarp();
+              pair_first_visible();
+            }
+#pragma unroll
+            for (int x = 0; x < 3; x++)
+              if (x >= s0 && x < s1) bulk_add_block(dst[x], reds + 128 * x, add[x]);
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          };
 #pragma unroll
           for (int h = 0; h < 2; h++) {
-            const double mxx = acc[0][0][h], mxy = acc[0][1][h], myx = acc[0][2][h], myy = acc[0][3][h];
-            double kxx, kxy, kyx, kyy;
-            block(mxx, mxy, myx, myy, kxx, kxy, kyx, kyy);
-            dst[h] = frag_stage<P>(O, el, pa, 4 * h + t, 0, kxx, kxy, kyx, kyy, reds + 128 * h);
+            const int b = 4 * h + t;
+            block(acc[0][0][h], acc[0][1][h], acc[0][2][h], acc[0][3][h], kxx, kxy, kyx, kyy);
+            if constexpr (NL) {
+              if (h) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+              add[0] = frag_put_block<P, PLAN>(O, el, pa, b, pa <= b, kxx, kxy, kyx, kyy, reds, dst[0]);
+              add[1] = frag_put_block<P, PLAN>(O, el, b, pa, pa < b, kxx, kyx, kxy, kyy, reds + 128, dst[1]);
+              issue(0, 2);
+            } else {
+              add[h] = frag_put_block<P, PLAN>(O, el, pa, b, true, kxx, kxy, kyx, kyy, reds + 128 * h, dst[h]);
+            }
           }
+          // sum the node-8 partials over the four lanes t
 #pragma unroll
           for (int c = 0; c < 4; c++) {
             n8[c] += __shfl_xor_sync(0xffffffffu, n8[c], 1);
@@ -1288,79 +1462,11 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
             d8[c] += __shfl_xor_sync(0xffffffffu, d8[c], 1);
             d8[c] += __shfl_xor_sync(0xffffffffu, d8[c], 2);
           }
-          const bool diag = (g == 0 && t == 2);
-          if (t < 2 || diag) {
-            const double mxx = diag ? d8[0] : n8[0], mxy = diag ? d8[1] : n8[1];
-            const double myx = diag ? d8[2] : n8[2], myy = diag ? d8[3] : n8[3];
-            double kxx, kxy, kyx, kyy;
-            block(mxx, mxy, myx, myy, kxx, kxy, kyx, kyy);
-            dst[2] = frag_stage<P>(O, el, 8, diag ? 8 : pa, diag ? 0 : t, kxx, kxy, kyx, kyy, reds + 128 * 2);
-          }
-          if (dst[0] || dst[1] || dst[2]) {
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-#pragma unroll
-            for (int s2 = 0; s2 < 3; s2++)
-              if (dst[s2]) bulk_add32(dst[s2], reds + 128 * s2);
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-          }
-        }
-        // stiffness blocks, order 2 (drop-in or NONLINEAR): lane (g, t) holds
-        // (a = 8TA + pi(g), b = 8TB + 4h + t), each written (or added) on its own
-        if constexpr (JAC && !RUNS && !(PLAN && !NL && P == 2)) {
-          if (PLAN && el > 0) pair_order_fence();
-          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-          int k = 0, slot = 0;
-          double *reds = redsW + 4 * lane;
-  #pragma unroll
-          for (int TA = 0; TA < NTM; TA++) {
-  #pragma unroll
-            for (int TB = TA; TB < NTM; TB++, k++) {
-              const int a = 8 * TA + pa;
-  #pragma unroll
-              for (int h = 0; h < 2; h++) {
-                const int b = 8 * TB + 4 * h + t;
-                if (a < NN && b < NN) {
-                  const double mxx = acc[k][0][h], mxy = acc[k][1][h], myx = acc[k][2][h], myy = acc[k][3][h];
-                  double kxx, kxy, kyx, kyy;
-                  block(mxx, mxy, myx, myy, kxx, kxy, kyx, kyy);
-                  // NONLINEAR diagonal tiles: (a, b) for a <= b and its exact transpose
-                  const bool dir = TA < TB || !NL || a <= b;
-                  const bool trn = TA < TB || (NL && a < b);
-                  if constexpr (PLAN) {
-                    if (dir) frag_write<P>(O, el, a, b, 0, kxx, kxy, kyx, kyy, reds + 128 * slot++);
-                    if (trn) frag_write<P>(O, el, a, b, 1, kxx, kxy, kyx, kyy, reds + 128 * slot++);
-                  } else {
-                    if (dir) frag_add_mapped<P>(O, el, a, b, 0, kxx, kxy, kyx, kyy, reds + 128 * slot++);
-                    if (trn) frag_add_mapped<P>(O, el, a, b, 1, kxx, kxy, kyx, kyy, reds + 128 * slot++);
-                  }
-                }
-              }
-            }
-          }
-          if constexpr (P == 2) {
-            // node 8: sum the partials over the four lanes t; lane t = 0 writes (8, pi(g)),
-            // t = 1 its transpose (pi(g), 8), lane (g = 0, t = 2) the diagonal block (8, 8)
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-              n8[c] += __shfl_xor_sync(0xffffffffu, n8[c], 1);
-              n8[c] += __shfl_xor_sync(0xffffffffu, n8[c], 2);
-              d8[c] += __shfl_xor_sync(0xffffffffu, d8[c], 1);
-              d8[c] += __shfl_xor_sync(0xffffffffu, d8[c], 2);
-            }
-            const bool diag = (g == 0 && t == 2);
-            if (t < 2 || diag) {
-              const double mxx = diag ? d8[0] : n8[0], mxy = diag ? d8[1] : n8[1];
-              const double myx = diag ? d8[2] : n8[2], myy = diag ? d8[3] : n8[3];
-              double kxx, kxy, kyx, kyy;
-              block(mxx, mxy, myx, myy, kxx, kxy, kyx, kyy);
-              const int b = diag ? 8 : pa, w = diag ? 0 : t;
-              if constexpr (PLAN) {
-                frag_write<P>(O, el, 8, b, w, kxx, kxy, kyx, kyy, reds + 128 * slot);
-              } else {
-                frag_add_mapped<P>(O, el, 8, b, w, kxx, kxy, kyx, kyy, reds + 128 * slot);
-              }
-            }
-          }
+          const bool diag = t == 2;
+          block(diag ? d8[0] : n8[0], diag ? d8[1] : n8[1], diag ? d8[2] : n8[2], diag ? d8[3] : n8[3], kxx, kxy, kyx, kyy);
+          add[2] = frag_put_block<P, PLAN>(O, el, t == 1 ? pa : 8, t == 0 ? pa : 8, t < 2 || (g == 0 && diag), kxx,
+                                           t == 1 ? kyx : kxy, t == 1 ? kxy : kyx, kyy, reds + 128 * 2, dst[2]);
+          issue(NL ? 2 : 0, 3);
         }
       }
     } else {
@@ -1373,7 +1479,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
       const double2 *WIi = ii ? WI1 : WI0;
       const double2 *WSi = ii ? WS1 : WS0;
       double *reds = redsW + 4 * lane;
-      int nw = 0;  // writes so far: ring position of the staging slot
+      int half = 0;  // half of the lane's staging slots the next batch uses
       for (int el = 0; el < ne; el++) {
         if (PLAN && el > 0) pair_order_fence();
         const bool neg = (negm & (el ? 0xccccccccu : 0x33333333u)) != 0;
@@ -1405,15 +1511,9 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
 #pragma unroll
           for (int mm = 0; mm < 2; mm++) {
             const int a = 4 * (2 * t + mm) + ah;
-            if (ii == 0 && a < NN) {
-              double *dst = M.residual + 2 * (int64_t)nid[el * NN + a];
-              if (PLAN && O.codes[el * CS + NN * NN + a]) {
-                *reinterpret_cast<double2 *>(dst) = make_double2(z[mm][0], z[mm][1]);
-              } else {
-                atomicAdd(dst, z[mm][0]);
-                atomicAdd(dst + 1, z[mm][1]);
-              }
-            }
+            const int an = a < NN ? a : 0;
+            residual_put(M.residual + 2 * (int64_t)nid[el * NN + an], ii == 0 && a < NN,
+                         PLAN && O.codes[el * CS + NN * NN + an], z[mm][0], z[mm][1]);
           }
         };
         if constexpr (RES && !JAC) {
@@ -1475,7 +1575,24 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
             }
           }
           // blocks: lane pair (l, l^4) exchanges rows; lane i = 0 writes (a, b), lane
-          // i = 1 writes (b, a) = (a, b)^T
+          // i = 1 writes (b, a) = (a, b)^T; the blocks to add leave in batches of two, from
+          // two halves of the lane's four slots in turn
+          constexpr int H = 2;
+          double *dst[H];
+          bool add[H];
+          int n = 0;
+          auto flush = [&](int m) {
+            bool any = add[0];
+            if (m > 1) any = any || add[1];
+            if (__any_sync(0xffffffffu, any)) {
+              asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+#pragma unroll
+              for (int x = 0; x < H; x++)
+                if (x < m) bulk_add_block(dst[x], reds + 128 * (H * half + x), add[x]);
+              half ^= 1;
+            }
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          };
 #pragma unroll
           for (int R = R0; R < R1; R++) {
             const int a = 4 * R + ah;
@@ -1486,21 +1603,19 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
               const double mxx = ii ? o0 : acc[R - R0][C - C0][0], mxy = ii ? o1 : acc[R - R0][C - C0][1];
               const double myx = ii ? acc[R - R0][C - C0][0] : o0, myy = ii ? acc[R - R0][C - C0][1] : o1;
               const int b = 4 * C + t;
-              if (a < NN && b < NN && a <= b && (ii == 0 || a < b)) {
-                double kxx, kxy, kyx, kyy;
-                block(mxx, mxy, myx, myy, kxx, kxy, kyx, kyy);
-                // the ring slot's previous bulk read (NSLOT writes ago) is complete
-                asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(L::NSLOT - 1) : "memory");
-                double *slot = reds + 128 * (nw % L::NSLOT);
-                nw++;
-                if constexpr (PLAN) {
-                  frag_write<P>(O, el, a, b, ii, kxx, kxy, kyx, kyy, slot);
-                } else {
-                  frag_add_mapped<P>(O, el, a, b, ii, kxx, kxy, kyx, kyy, slot);
-                }
+              double kxx, kxy, kyx, kyy;
+              block(mxx, mxy, myx, myy, kxx, kxy, kyx, kyy);
+              // the half's previous bulk reads are complete
+              if (n == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+              add[n] = frag_put_block<P, PLAN>(O, el, ii ? b : a, ii ? a : b, a < NN && b < NN && (ii ? a < b : a <= b), kxx,
+                                               ii ? kyx : kxy, ii ? kxy : kyx, kyy, reds + 128 * (H * half + n), dst[n]);
+              if (++n == H) {
+                flush(H);
+                n = 0;
               }
             }
           }
+          if (n) flush(n);
         };
         if constexpr (JAC) {
           static_assert(K4 == 7, "tile-pair groups of the order-4 layout");
@@ -1552,6 +1667,23 @@ __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB)
   frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) != 0>(smem);
   const int warp = threadIdx.x >> 5;
   PairRanges gen{R, (int64_t)blockIdx.x * FragDims<P>::WARPS + warp, (int64_t)gridDim.x * FragDims<P>::WARPS};
+  frag_loop<P, MODE>(smem, gen, A, &A);
+}
+
+// One mesh, strips of several ranges of its strip list (plan mode, LINEAR Jacobian).  The
+// order-3 assembly is bound by its writes: a probe that stores every block once at its
+// real address took 568 us for 512^2 in the pair layout's order (four colours, x-neighbours
+// written in different launches: lines leave L2 half written), 466 us with each element row
+// in one launch (linear fill: 378-400).  512^2: 668 -> 576 us, 1024^2 2.63 -> 2.21 ms.
+template <int P, int MODE>
+__global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB)
+    frag_strip_kernel(const __grid_constant__ AsmArgs A, const __grid_constant__ RangeList R,
+                      const Strip *__restrict__ strips) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) != 0>(smem);
+  const int warp = threadIdx.x >> 5;
+  StripRanges gen{strips, R, (int64_t)blockIdx.x * FragDims<P>::WARPS + warp, (int64_t)gridDim.x * FragDims<P>::WARPS};
+  gen.fetch();
   frag_loop<P, MODE>(smem, gen, A, &A);
 }
 
@@ -1665,6 +1797,32 @@ int launch_frag_ranges_p(const AsmArgs &a, const RangeList &r, cudaStream_t s, b
     err = cudaGetLastError();
   }
   if (err != cudaSuccess) return cuda_fail(err, "frag_ranges_kernel launch");
+  return FEM_SUCCESS;
+}
+
+template <int P, int MODE>
+int launch_frag_strips_p(const AsmArgs &a, const RangeList &r, const Strip *strips, cudaStream_t s, bool chained) {
+  using F = FragDims<P>;
+  constexpr int NT = 32 * F::WARPS;
+  auto kernel = frag_strip_kernel<P, MODE>;
+  const size_t smem = FragLayout<P, false, (MODE & kNL) != 0, (MODE & kB16) != 0, (MODE & kJac) != 0>::total;
+  LaunchInfo li;
+  int st = launch_info(kernel, NT, smem, li);
+  if (st) return st;
+  int64_t n = 0;
+  for (int i = 0; i < r.n; i++) n += r.count[i];
+  const int64_t need = (n + F::WARPS - 1) / F::WARPS;
+  const int64_t cap = (int64_t)li.grid_per_sm * li.num_sms;
+  const int grid = (int)(need < cap ? need : cap);
+  if (grid <= 0) return FEM_SUCCESS;
+  cudaError_t err;
+  if (chained) {
+    err = pdl_launch(kernel, grid, NT, smem, s, a, r, strips);
+  } else {
+    kernel<<<grid, NT, smem, s>>>(a, r, strips);
+    err = cudaGetLastError();
+  }
+  if (err != cudaSuccess) return cuda_fail(err, "frag_strip_kernel launch");
   return FEM_SUCCESS;
 }
 
@@ -1818,6 +1976,23 @@ int launch_frag_ranges(int order, int precision, int mode, const dev::AsmArgs &a
     case kNL | kPlan | kRes: return go(IC<kNL | kPlan | kRes>{});
     case kNL | kPlan | kRes | kJac: return go(IC<kNL | kPlan | kRes | kJac>{});
     default: return fail(FEM_ERR_INVALID_ARGUMENT, "fragment kernel, ranges: mode %d", mode);
+  }
+}
+
+// Strips: LINEAR Jacobians of order-kStripOrder plans.
+int launch_frag_strips(int order, int precision, int mode, const dev::AsmArgs &a, const dev::RangeList &r,
+                       const dev::Strip *strips, cudaStream_t s, int strain, bool chained) {
+  using namespace dev;
+  if (order != kStripOrder || strain != FEM_STRAIN_LINEAR)
+    return fail(FEM_ERR_INVALID_ORDER, "fragment kernel, strips: order %d, strain %d", order, strain);
+  if (b16_stiffness(order, precision, strain) && (mode & kJac)) mode |= kB16;
+  switch (mode) {
+    case kPlan | kJac: return launch_frag_strips_p<kStripOrder, kPlan | kJac>(a, r, strips, s, chained);
+    case kPlan | kRes | kJac: return launch_frag_strips_p<kStripOrder, kPlan | kRes | kJac>(a, r, strips, s, chained);
+    case kPlan | kJac | kB16: return launch_frag_strips_p<kStripOrder, kPlan | kJac | kB16>(a, r, strips, s, chained);
+    case kPlan | kRes | kJac | kB16:
+      return launch_frag_strips_p<kStripOrder, kPlan | kRes | kJac | kB16>(a, r, strips, s, chained);
+    default: return fail(FEM_ERR_INVALID_ARGUMENT, "fragment kernel, strips: mode %d", mode);
   }
 }
 

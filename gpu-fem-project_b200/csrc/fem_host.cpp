@@ -4,6 +4,7 @@
 // result does not depend on the schedule).
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <cstdarg>
 #include <cstring>
 #include <string>
@@ -175,34 +176,192 @@ static void build_row_plan(HostPlan &hp) {
   hp.rowChunk.swap(chunk);
 }
 
-// Pair layout (HostPlan::pairColourPtr ...).  Element f is e's right neighbour when
-// f's nodes (0, ly) are e's nodes (P, ly) for every ly (tensor order: local node
-// a = ly (P + 1) + lx); elements are paired greedily in id order.  Units (pairs
-// and unpaired elements) are coloured greedily like the elements of the colour
-// layout; codes are computed per colour with the units in parallel (they share no
-// node) and the two elements of a pair in order.  Leaves the layout empty when
-// the units need more than 64 colours.
-static void build_pair_plan(const int *connPtr, const int *conn, HostPlan &hp) {
-  const int P = hp.order, P1 = P + 1, nn = hp.nn, nE = hp.numElements;
+// Element f is e's right neighbour when f's nodes (0, ly) are e's nodes (P, ly) for
+// every ly (tensor order: local node a = ly (P + 1) + lx) and no other element has that
+// left edge.  right[e] = f, or -1.
+static void right_neighbours(const int *connPtr, const int *conn, const HostPlan &hp, std::vector<int> &right) {
+  const int P = hp.order, P1 = P + 1, nE = hp.numElements;
   auto node = [&](int e, int lx, int ly) { return conn[connPtr[e] + ly * P1 + lx]; };
   auto key = [](int a, int b) { return ((uint64_t)(uint32_t)a << 32) | (uint32_t)b; };
   // left edge (corner nodes (0, 0), (0, P)) -> element, sorted for lookup
   std::vector<std::pair<uint64_t, int>> left((size_t)nE);
   for (int e = 0; e < nE; e++) left[e] = {key(node(e, 0, 0), node(e, 0, P)), e};
   std::sort(left.begin(), left.end());
-  std::vector<int> partner((size_t)nE, -1);
-  std::vector<char> lead((size_t)nE, 0);
+  right.assign((size_t)nE, -1);
+#pragma omp parallel for schedule(static)
   for (int e = 0; e < nE; e++) {
-    if (partner[e] >= 0) continue;
     const uint64_t k = key(node(e, P, 0), node(e, P, P));
     auto it = std::lower_bound(left.begin(), left.end(), std::make_pair(k, INT_MIN));
     if (it == left.end() || it->first != k) continue;
     if (it + 1 != left.end() && (it + 1)->first == k) continue;  // two elements share that left edge
     const int f = it->second;
-    if (f == e || partner[f] >= 0) continue;
+    if (f == e) continue;
     bool same = true;
     for (int ly = 0; ly <= P && same; ly++) same = node(e, P, ly) == node(f, 0, ly);
-    if (!same) continue;
+    if (same) right[e] = f;
+  }
+}
+
+// Elements per strip (odd: with the halo, whole steps of two).  A launch of a colour
+// (about half of the elements) runs its strips in waves over the resident warps, so a
+// strip's steps times the waves are what it takes, and half a step is lost to a strip's
+// halo.  Measured (order 3, us; 5 / 7 / 11 / 15 / 23 elements): 128^2 55 / 65 / 77 / 74 /
+// 104, 200^2 123 / 120 / 137 / 121 / 154, 256^2 177 / 175 / 176 / 189 / 175, 512^2 622 /
+// 593 / 582 / 576 / 596, 1024^2 2454 / 2338 / 2252 / 2218 / 2209; the last wave is partly
+// overlapped, hence the mean of whole and exact waves.
+// chainPtr, colour: the chains and their colours (nc).
+static int strip_length(const std::vector<int> &chainPtr, const std::vector<int> &colour, int nc) {
+  int best = 1;
+  double cost = 1e300;
+  std::vector<int64_t> strips((size_t)nc);
+  for (int n = 1; n <= 31; n += 2) {
+    std::fill(strips.begin(), strips.end(), 0);
+    for (size_t i = 0; i < colour.size(); i++)  // a chain's first strip takes n + 1
+      strips[colour[i]] += std::max(1, (chainPtr[i + 1] - chainPtr[i] - 1 + n - 1) / n);
+    double c = 0.0;
+    for (int64_t k : strips) {
+      const double waves = (double)k / kStripWarps;
+      c += (std::ceil(waves) + waves) * (n + 1);
+    }
+    if (c < cost) {
+      cost = c;
+      best = n;
+    }
+  }
+  return best;
+}
+
+// Strip layout (HostPlan::strips ...), left empty when the mesh's chains are short, meet
+// themselves, or need more than 64 colours.
+static void build_strip_plan(const int *connPtr, const int *conn, const std::vector<int> &right, HostPlan &hp) {
+  const int P = hp.order, P1 = P + 1, nn = hp.nn, nE = hp.numElements;
+  if (P != kStripOrder || nE == 0) return;
+  // chains of right neighbours (an element is the right neighbour of one at most)
+  std::vector<int> left((size_t)nE, -1), next(right);
+  for (int e = 0; e < nE; e++) {
+    if (next[e] < 0) continue;
+    if (left[next[e]] >= 0) next[e] = -1;
+    else left[next[e]] = e;
+  }
+  std::vector<int> chain, chainPtr(1, 0);  // elements chain by chain
+  chain.reserve((size_t)nE);
+  for (int e = 0; e < nE; e++) {
+    if (left[e] >= 0) continue;
+    for (int x = e; x >= 0; x = next[x]) chain.push_back(x);
+    chainPtr.push_back((int)chain.size());
+  }
+  const int nch = (int)chainPtr.size() - 1;
+  if ((int)chain.size() != nE || nE / nch < 4) return;  // a ring, or short chains
+  // a chain's elements may share nodes only across the edge of two consecutive ones
+  std::vector<int> seen((size_t)hp.numNodes, -1);
+  for (int i = 0; i < nch; i++)
+    for (int k = chainPtr[i]; k < chainPtr[i + 1]; k++)
+      for (int a = 0; a < nn; a++) {
+        int &m = seen[conn[connPtr[chain[k]] + a]];
+        if (m == i && (k == chainPtr[i] || a % P1 != 0)) return;
+        m = i;
+      }
+  // chains coloured greedily over node bit masks
+  std::vector<uint64_t> used((size_t)hp.numNodes, 0);
+  std::vector<int> colour((size_t)nch);
+  int nc = 0;
+  for (int i = 0; i < nch; i++) {
+    uint64_t m = 0;
+    for (int k = chainPtr[i]; k < chainPtr[i + 1]; k++)
+      for (int a = 0; a < nn; a++) m |= used[conn[connPtr[chain[k]] + a]];
+    if (~m == 0) return;
+    colour[i] = __builtin_ctzll(~m);
+    nc = std::max(nc, colour[i] + 1);
+    for (int k = chainPtr[i]; k < chainPtr[i + 1]; k++)
+      for (int a = 0; a < nn; a++) used[conn[connPtr[chain[k]] + a]] |= 1ull << colour[i];
+  }
+  // strips, chain by chain: the first of a chain has no halo and takes one element more
+  const int len = strip_length(chainPtr, colour, nc);
+  std::vector<int> stripPtr(1, 0), chainOf;
+  std::vector<dev::Strip> strips;
+  std::vector<int> listed;  // element ids, halos included
+  for (int i = 0; i < nch; i++) {
+    for (int k = chainPtr[i]; k < chainPtr[i + 1];) {
+      const bool first = k == chainPtr[i];
+      const int n = std::min(len + (first ? 1 : 0), chainPtr[i + 1] - k);
+      strips.push_back({(int)listed.size(), n + (first ? 0 : 1),
+                        (first ? 0 : dev::kHalo) | (k + n < chainPtr[i + 1] ? dev::kRight : 0), chain[k]});
+      if (!first) listed.push_back(chain[k - 1]);
+      listed.insert(listed.end(), chain.begin() + k, chain.begin() + k + n);
+      k += n;
+    }
+    stripPtr.push_back((int)strips.size());
+  }
+  hp.stripConn.resize(listed.size() * nn);
+  hp.stripCode.assign(listed.size() * (size_t)hp.codeStride, 0);
+  std::vector<uint8_t> blockWritten((size_t)hp.nnzb, 0), nodeWritten((size_t)hp.numNodes, 0);
+  std::vector<std::vector<int>> byColour((size_t)nc);
+  for (int i = 0; i < nch; i++) byColour[colour[i]].push_back(i);
+  for (int c = 0; c < nc; c++) {
+    const std::vector<int> &chains = byColour[c];
+    // the chains of one colour share no node, hence no block
+#pragma omp parallel for schedule(dynamic, 1)
+    for (int64_t y = 0; y < (int64_t)chains.size(); y++) {
+      for (int x = stripPtr[chains[y]]; x < stripPtr[chains[y] + 1]; x++) {
+        const dev::Strip &st = strips[x];
+        for (int k = st.begin; k < st.begin + st.count; k++) {
+          const int *en = conn + connPtr[listed[k]];
+          std::copy(en, en + nn, &hp.stripConn[(size_t)k * nn]);
+          if ((st.flags & dev::kHalo) && k == st.begin) continue;
+          const bool give = k + 1 < st.begin + st.count || (st.flags & dev::kRight);
+          uint8_t *rec = &hp.stripCode[(size_t)k * hp.codeStride];
+          for (int a = 0; a < nn; a++) {
+            const int r = en[a];
+            const bool ra = give && a % P1 == P;
+            rec[nn * nn + a] = nodeWritten[r] ? 0 : 1;
+            if (!ra) nodeWritten[r] = 1;
+            const int *c0 = hp.cols.data() + hp.rowp[r], *c1 = hp.cols.data() + hp.rowp[r + 1];
+            for (int b = 0; b < nn; b++) {
+              const int *pos = std::lower_bound(c0, c1, en[b]);  // present: the colour layout found it
+              uint8_t &bf = blockWritten[(size_t)(pos - hp.cols.data())];
+              const bool rb = ra && b % P1 == P;
+              rec[a * nn + b] = (uint8_t)((pos - c0) | (rb || !bf ? 0x80 : 0));
+              if (!rb) bf = 1;
+            }
+          }
+        }
+      }
+    }
+  }
+  // by colour, ascending lead
+  hp.stripColourPtr.assign(1, 0);
+  for (int c = 0; c < nc; c++) {
+    const size_t s0 = hp.strips.size();
+    for (int i : byColour[c]) hp.strips.insert(hp.strips.end(), strips.begin() + stripPtr[i], strips.begin() + stripPtr[i + 1]);
+    std::sort(hp.strips.begin() + s0, hp.strips.end(), [](const dev::Strip &a, const dev::Strip &b) { return a.lead < b.lead; });
+    hp.stripColourPtr.push_back((int)hp.strips.size());
+  }
+  hp.stripLo.resize(hp.strips.size());
+  hp.stripHi.resize(hp.strips.size());
+#pragma omp parallel for schedule(static)
+  for (int64_t x = 0; x < (int64_t)hp.strips.size(); x++) {
+    const int *c0 = &hp.stripConn[(size_t)hp.strips[x].begin * nn];
+    const auto mm = std::minmax_element(c0, c0 + (size_t)hp.strips[x].count * nn);
+    hp.stripLo[x] = *mm.first;
+    hp.stripHi[x] = *mm.second;
+  }
+  hp.numStripColours = nc;
+}
+
+// Pair layout (HostPlan::pairColourPtr ...): elements paired with their right neighbour
+// greedily in id order.  Units (pairs
+// and unpaired elements) are coloured greedily like the elements of the colour
+// layout; codes are computed per colour with the units in parallel (they share no
+// node) and the two elements of a pair in order.  Leaves the layout empty when
+// the units need more than 64 colours.
+static void build_pair_plan(const int *connPtr, const int *conn, const std::vector<int> &right, HostPlan &hp) {
+  const bool tables = hp.numStripColours == 0;  // else the counts alone
+  const int nn = hp.nn, nE = hp.numElements;
+  std::vector<int> partner((size_t)nE, -1);
+  std::vector<char> lead((size_t)nE, 0);
+  for (int e = 0; e < nE; e++) {
+    const int f = right[e];
+    if (partner[e] >= 0 || f < 0 || partner[f] >= 0) continue;
     partner[e] = f;
     partner[f] = e;
     lead[e] = 1;
@@ -253,6 +412,9 @@ static void build_pair_plan(const int *connPtr, const int *conn, HostPlan &hp) {
       hp.pairList[fillS[c]++] = e;
     }
   }
+  hp.numPairColours = nc;
+  for (int c = 0; c < nc; c++) hp.numPairs += pairsOf[c];
+  if (!tables) return;
   hp.pairConnList.resize((size_t)nE * nn);
   hp.pairCode.assign((size_t)nE * hp.codeStride, 0);
   std::vector<uint8_t> blockWritten((size_t)hp.nnzb, 0), nodeWritten((size_t)hp.numNodes, 0);
@@ -288,15 +450,12 @@ static void build_pair_plan(const int *connPtr, const int *conn, HostPlan &hp) {
       }
     }
   }
-  hp.numPairColours = nc;
   hp.pairRegionEnd.resize((size_t)nc);
   for (int c = 0; c < nc; c++) hp.pairRegionEnd[c] = hp.pairColourPtr[c] + (int)(2 * pairsOf[c]);
-  int64_t np = 0;
-  for (int c = 0; c < nc; c++) np += pairsOf[c];
-  hp.numPairs = np;
 }
 
-int build_host_plan(int order, int numNodes, const int *connPtr, const int *conn, int numElements, HostPlan &hp) {
+int build_host_plan(int order, int numNodes, const int *connPtr, const int *conn, int numElements, HostPlan &hp,
+                    bool strips) {
   const int nn = (order + 1) * (order + 1);
   int st = validate_mesh(numNodes, connPtr, conn, numElements);
   if (st) return st;
@@ -363,7 +522,12 @@ int build_host_plan(int order, int numNodes, const int *connPtr, const int *conn
   }
   if (bad) return fail(FEM_ERR_UNSUPPORTED, "a BSR row holds more than 128 blocks; use the map-based entry points");
   if (order == 1) build_row_plan(hp);
-  if (order >= 2) build_pair_plan(connPtr, conn, hp);
+  if (order >= 2) {
+    std::vector<int> right;
+    right_neighbours(connPtr, conn, hp, right);
+    if (strips) build_strip_plan(connPtr, conn, right, hp);
+    build_pair_plan(connPtr, conn, right, hp);
+  }
   return FEM_SUCCESS;
 }
 
@@ -445,7 +609,7 @@ int fem_pair_layout(int elementOrder, int numNodes, const int *connPtr, const in
   if (elementOrder < 2 || elementOrder > 4)
     return fem::fail(FEM_ERR_INVALID_ORDER, "pair layout: orders 2..4 (order %d)", elementOrder);
   fem::HostPlan hp;
-  int st = fem::build_host_plan(elementOrder, numNodes, connPtr, conn, numElements, hp);
+  int st = fem::build_host_plan(elementOrder, numNodes, connPtr, conn, numElements, hp, /*strips=*/false);
   if (st) return st;
   *numColours = hp.numPairColours;
   *numPairs = hp.numPairs;

@@ -175,6 +175,9 @@ void plan_free(fem_plan *p) {
   cudaFree(p->d_blockCode);
   cudaFree(p->d_pairConnList);
   cudaFree(p->d_pairCode);
+  cudaFree(p->d_strips);
+  cudaFree(p->d_stripConn);
+  cudaFree(p->d_stripCode);
   cudaFree(p->d_rowElemPtr);
   cudaFree(p->d_rowElem);
   cudaFree(p->d_rowChunk);
@@ -356,6 +359,17 @@ int build_schedule(fem_plan *p, int band, int tile) {
   return FEM_SUCCESS;
 }
 
+// How the fragment kernel's single-mesh launches run a plan in its pair layout.  A plan
+// with a strip layout runs the LINEAR Jacobian by strips (order 3, us, before / strips:
+// 1024^2 2630 / 2210, 515 x 509 MIXED 698 / 640) and the rest by the element colours:
+// NONLINEAR strain and the residual alone are bound by their arithmetic, which a strip's
+// halo adds to (400 x 397 NONLINEAR: 707 colours, 710 pairs, 789 strips; 600 x 590
+// residual: 249, 248, 281).  The other plans run their pairs.
+bool plan_strips(const fem_plan *p, int strain, const double *matEntries) {
+  return p->usePairs && p->numStripColours > 0 && strain == FEM_STRAIN_LINEAR && matEntries;
+}
+bool plan_pairs(const fem_plan *p) { return p->usePairs && p->numPairColours > 0 && p->numStripColours == 0; }
+
 // Whether fem_plan_assemble runs `p` as one dependency-ordered launch.
 bool plan_sched(const fem_plan *p, int precision, int strain) {
   return p->schedGroups > 0 && fem::frag_supported(p->order, precision, strain, true) &&
@@ -467,7 +481,23 @@ int fem_plan_create(int elementOrder, int numNodes, const int *connPtr, const in
     }
     p->numChunks = (int)hp.rowChunk.size() - 1;
   }
-  if (hp.numPairColours > 0) {
+  if (hp.numStripColours > 0) {
+    if ((st = upload(hp.strips, &p->d_strips, p->deviceBytes)) ||
+        (st = upload(hp.stripConn, &p->d_stripConn, p->deviceBytes)) ||
+        (st = upload(hp.stripCode, &p->d_stripCode, p->deviceBytes))) {
+      plan_free(p);
+      return st;
+    }
+    p->stripColourPtr = hp.stripColourPtr;
+    p->stripLo = hp.stripLo;
+    p->stripHi = hp.stripHi;
+    p->stripLead.resize(hp.strips.size());
+    for (size_t x = 0; x < hp.strips.size(); x++) p->stripLead[x] = hp.strips[x].lead;
+    p->numStripColours = hp.numStripColours;
+    p->numPairColours = hp.numPairColours;
+    p->numPairs = hp.numPairs;
+    p->usePairs = hp.numPairColours > 0;
+  } else if (hp.numPairColours > 0) {
     if ((st = upload(hp.pairConnList, &p->d_pairConnList, p->deviceBytes)) ||
         (st = upload(hp.pairCode, &p->d_pairCode, p->deviceBytes))) {
       plan_free(p);
@@ -670,7 +700,20 @@ int fem_plan_assemble_ex(const fem_plan *plan, const double *states, const doubl
   }
   // the fragment kernel runs the pair layout (a step's two elements share an edge,
   // so the lines of the rows they share are written while they are still in L2)
-  const bool pairs = frag && plan->usePairs && plan->numPairColours > 0;
+  if (frag && plan_strips(plan, strainType, matEntries)) {
+    a.connList = plan->d_stripConn;
+    a.blockCode = plan->d_stripCode;
+    return fem::timed(s, elapsedSeconds, [&] {
+      for (int c = 0; c < plan->numStripColours; c++) {
+        fem::dev::RangeList r{1, {plan->stripColourPtr[c]}, {plan->stripColourPtr[c + 1] - plan->stripColourPtr[c]}};
+        int st = fem::launch_frag_strips(plan->order, precision, mode, a, r, plan->d_strips, s, strainType,
+                                         /*chained=*/c > 0);
+        if (st) return st;
+      }
+      return (int)FEM_SUCCESS;
+    });
+  }
+  const bool pairs = frag && plan_pairs(plan);
   if (pairs) {
     a.connList = plan->d_pairConnList;
     a.blockCode = plan->d_pairCode;
@@ -697,6 +740,14 @@ int fem_plan_set_layout(fem_plan *plan, int layout) {
   if (layout == FEM_LAYOUT_PAIRS && plan->numPairColours == 0)
     return fem::fail(FEM_ERR_UNSUPPORTED, "this plan has no pair layout (order 1, or its pairs need > 64 colours)");
   plan->usePairs = layout == FEM_LAYOUT_PAIRS;
+  return FEM_SUCCESS;
+}
+
+int fem_plan_get_strips(const fem_plan *plan, int *numStrips, int *numStripColours) {
+  fem::clear_error();
+  if (!plan) return fem::fail(FEM_ERR_INVALID_ARGUMENT, "plan is NULL");
+  if (numStrips) *numStrips = (int)plan->stripLead.size();
+  if (numStripColours) *numStripColours = plan->numStripColours;
   return FEM_SUCCESS;
 }
 
@@ -746,13 +797,15 @@ int fem_plan_assemble_host(const fem_plan *plan, const double *hostStates, doubl
   const bool rows = fem::plan_rows(plan) && strainType == FEM_STRAIN_LINEAR;
   // the fragment kernel runs the pair layout when the plan uses it (each band's pairs
   // and unpaired elements are two ranges of a colour), else the colour layout
-  const bool pairs = frag && !rows && plan->usePairs && plan->numPairColours > 0;
+  const bool strips = frag && !rows && plan_strips(plan, strainType, matEntries);
+  const bool pairs = frag && !rows && !strips && plan_pairs(plan);
   const int N = plan->numNodes, nE = plan->numElements;
-  const int nc = pairs ? plan->numPairColours : plan->numColours;
-  const std::vector<int> &cptr = pairs ? plan->pairColourPtr : plan->colourPtr;
-  const std::vector<int> &list = pairs ? plan->pairList : plan->elemList;
-  const std::vector<int> &nlo = pairs ? plan->pairNodeLo : plan->nodeLo;
-  const std::vector<int> &nhi = pairs ? plan->pairNodeHi : plan->nodeHi;
+  const int nc = strips ? plan->numStripColours : pairs ? plan->numPairColours : plan->numColours;
+  // strips: list positions are strips, each in the band of its lead element
+  const std::vector<int> &cptr = strips ? plan->stripColourPtr : pairs ? plan->pairColourPtr : plan->colourPtr;
+  const std::vector<int> &list = strips ? plan->stripLead : pairs ? plan->pairList : plan->elemList;
+  const std::vector<int> &nlo = strips ? plan->stripLo : pairs ? plan->pairNodeLo : plan->nodeLo;
+  const std::vector<int> &nhi = strips ? plan->stripHi : pairs ? plan->pairNodeHi : plan->nodeHi;
   const int B = std::min(numBands, std::max(1, std::min(N, nE)));
   // node chunk j = [nstart[j], nstart[j + 1]); chunk_of inverts exactly that split
   std::vector<int64_t> nstart((size_t)B + 1);
@@ -870,7 +923,10 @@ int fem_plan_assemble_host(const fem_plan *plan, const double *hostStates, doubl
 
   fem::dev::AsmArgs a{};
   fem::plan_args(a, plan);
-  if (pairs) {
+  if (strips) {
+    a.connList = plan->d_stripConn;
+    a.blockCode = plan->d_stripCode;
+  } else if (pairs) {
     a.connList = plan->d_pairConnList;
     a.blockCode = plan->d_pairCode;
   }
@@ -916,6 +972,9 @@ int fem_plan_assemble_host(const fem_plan *plan, const double *hostStates, doubl
         a.begin = 0;
         a.count = plan->numChunks;
         r = fem::launch_rows(mode, a, s);
+      } else if (strips) {
+        r = fem::launch_frag_strips(plan->order, precision, mode, a, g.r, plan->d_strips, s, strainType,
+                                    /*chained=*/i > 0);
       } else if (frag) {
         // after the first launch each one follows this call's previous launch (a state
         // chunk it waits for still gates it through the stream's event wait)

@@ -127,6 +127,9 @@ int launch_frag(int order, int precision, int mode, const dev::AsmArgs &a, cudaS
 // kMaxRanges list-position ranges of one mesh in one launch.
 int launch_frag_ranges(int order, int precision, int mode, const dev::AsmArgs &a, const dev::RangeList &r,
                        cudaStream_t s, int strain = FEM_STRAIN_LINEAR, bool chained = false);
+// Strips of one plan (plan mode): ranges of its strip list.
+int launch_frag_strips(int order, int precision, int mode, const dev::AsmArgs &a, const dev::RangeList &r,
+                       const dev::Strip *strips, cudaStream_t s, int strain = FEM_STRAIN_LINEAR, bool chained = false);
 // All colours of one plan in one dependency-ordered persistent launch (plan mode).
 int launch_frag_sched(int order, int precision, int mode, const dev::AsmArgs &a, const dev::SchedArgs &sa,
                       cudaStream_t s, int strain = FEM_STRAIN_LINEAR);
@@ -213,6 +216,13 @@ struct fem_plan {
   int numPairColours = 0;
   int64_t numPairs = 0;
   bool usePairs = false;
+  // large meshes of order kStripOrder: strip layout, the pair layout's other form
+  // (HostPlan::strips); numStripColours == 0: none
+  fem::dev::Strip *d_strips = nullptr;
+  int *d_stripConn = nullptr;
+  uint8_t *d_stripCode = nullptr;
+  std::vector<int> stripColourPtr, stripLead, stripLo, stripHi;
+  int numStripColours = 0;
   // order 1: row assembly tables (HostPlan::rowElemPtr/rowElem/rowChunk); numChunks == 0: none
   int *d_rowElemPtr = nullptr, *d_rowElem = nullptr, *d_rowChunk = nullptr;
   int numChunks = 0;

@@ -175,7 +175,11 @@ int fem_plan_row_chunks(const fem_plan *plan, int *numChunks);
  *                       pairs share no node, and a warp assembles a pair in one
  *                       step, the second element adding to the shared edge's
  *                       blocks the first one stored, so that the rows the two
- *                       share are written while their lines are in L2;
+ *                       share are written while their lines are in L2.  Order-3
+ *                       plans whose elements form chains of such neighbours run the
+ *                       LINEAR Jacobian (with or without the residual) by strips of
+ *                       these chains instead, one launch per colour of the chains
+ *                       (fem_plan_get_strips), and everything else by FEM_LAYOUT_COLOURS;
  *   FEM_LAYOUT_COLOURS  the element colouring above (what every other path runs).
  * The results agree to rounding: a block's contributions are added in another
  * order where more than two elements share it.  fem_plan_get_layout also reports
@@ -185,6 +189,8 @@ int fem_plan_row_chunks(const fem_plan *plan, int *numChunks);
 #define FEM_LAYOUT_PAIRS 1
 int fem_plan_set_layout(fem_plan *plan, int layout);
 int fem_plan_get_layout(const fem_plan *plan, int *layout, int64_t *numPairs, int *numPairColours);
+/* Strips of an order-3 plan and their colours (launches); 0, 0 when it has none. */
+int fem_plan_get_strips(const fem_plan *plan, int *numStrips, int *numStripColours);
 /* Device pointers of the plan's rowp/cols (owned by the plan). */
 int fem_plan_device_pattern(const fem_plan *plan, const int **rowp, const int **cols);
 /* states/nodeCoords/residual/matEntries are device pointers; residual or
