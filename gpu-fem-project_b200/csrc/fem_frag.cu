@@ -14,33 +14,36 @@
 //
 //   1. gather    lane (g, t) (g = lane/4, t = lane%4) loads component c = g%4
 //                (x, y, u, v) of node 4ks + t of element g/4: that register IS
-//                the A fragment of step 2 (rows = 2 elements x 4 components,
+//                the B fragment of step 2 (columns = 2 elements x 4 components,
 //                k = element nodes).  Node ids are read two steps ahead, the
 //                coordinates/states one step ahead.
-//   2. J stage   C[(e,c)][(q,d)] = sum_a X[(e,c)][a] dN_d(a, q): the isoparametric
+//   2. J stage   C_d[q][(e,c)] = sum_a dN_d(a, q) X[a][(e,c)]: the isoparametric
 //                Jacobian and the reference-space state gradient of both
-//                elements at every quadrature point (K4 x K4 MMAs), with the
-//                derivative table as B fragments (shared memory, lane order).
-//   3. transpose three xor-shuffle rounds per group of four column tiles give each
-//                lane all eight values of one quadrature point q = 4(4m + c) + t
-//                (one point per lane at p <= 3, two at p = 4); it forms det J, J^-1,
-//                s = w det J t, the weak stress and sqrt|s| J^-1 (FP64) and
-//                stores the ~10 doubles of q to shared memory.
+//                elements at every quadrature point (8 points per tile), with the
+//                derivative table as A fragments (shared memory, lane order).
+//   3. points    lane (g, t) holds J (t even) or grad u (t odd) of element t/2 at its
+//                tiles' points q = 8tm + g; one xor-1 exchange per pair of tiles hands
+//                each lane all eight values of one point.  It forms det J, sqrt|s| J^-1
+//                (s = w det J t) and the weak stress in FP64 and stores the ~8 doubles
+//                of q to shared memory.
 //   4. fragments lane (g, t) builds G-hat_i(q, a) = sqrt|s| (dN(a,q) J^-1)_i for
 //                q = 4ks + t from sqrt|s| J^-1 and the table: the A and B fragments
 //                of M_ij[a][b] = sum_q s G_ai G_bj.
 //   5. residual  R_(a,i) = sum_q sum_j G-hat_j S-hat_ij on the FP64 pipe from the
 //                same fragments, reduced over the lanes of a node by shuffles.
-//   6. stiffness p = 2, 3: component-major node tiles (a = 8T + pi(g), pi(g) =
-//                4(g%2) + g/2; pairs TA <= TB, four (i, j) tiles sharing
-//                fragments, k-steps outermost): lane (g, t) ends with WHOLE 2x2
-//                blocks (a, b = 8TB + 4h + t), so the plane-stress combination
-//                needs no shuffle and a warp store covers eight runs of four
-//                consecutive blocks.  p = 4: interleaved rows r = 2a + i in seven
-//                tiles (a = 4T + g/2), one pass per group of tile pairs with the
-//                group's fragments rebuilt from the table (the residual rides on
-//                the first three groups); lanes l, l^4 exchange the two rows of a
-//                block.  Blocks above the diagonal are also written transposed.
+//   6. stiffness component-major node tiles (a = 8T + pi(g), pi(g) = 4(g%2) + g/2;
+//                pairs TA <= TB, four (i, j) tiles sharing fragments, k-steps
+//                outermost): lane (g, t) ends with WHOLE 2x2 blocks (a, b = 8TB +
+//                4h + t), so the plane-stress combination needs no shuffle and a
+//                warp store covers eight runs of four consecutive blocks.  Orders 2
+//                and 4 (9 and 25 nodes) leave the last node out of the tiles; its row
+//                and column take the FP64 pipe.  Order 4 runs its six tile pairs in
+//                two passes of twelve accumulator tiles (an earlier form, 28 tiles of
+//                interleaved rows r = 2a + i in five groups, formed 19 instead of 5
+//                fragment pairs per k-step and exchanged the two rows of every block
+//                between lanes: 256^2 703 -> 507 us; the same at two CTAs per SM and 255
+//                registers: 537 us).  Blocks above the diagonal are also written
+//                transposed.
 //
 // Writes.  Plan mode: a launch is one colour; the first contributor of a block
 // stores it (one 256-bit store); a later colour adds its 2x2 blocks with
@@ -78,16 +81,17 @@ struct FragDims {
   static constexpr int K4 = (NN + 3) / 4;   // node k-steps = quadrature k-steps
   static constexpr int NQP = 4 * K4;        // padded quadrature points
   static constexpr int QT = 2 * ((NQ + 15) / 16);  // J-stage row tiles (8 quadrature points each), in pairs
-  static constexpr int NTN = (NN + 7) / 8;  // node tiles of the component-major stiffness product
+  static constexpr int NTM = NN / 8;        // node tiles of the component-major stiffness product
+  static constexpr bool EX = NN % 8 == 1;   // orders 2, 4: the last node is in no tile (FP64 pipe)
+  static constexpr int NPASS = NTM == 3 ? 2 : 1;  // stiffness passes (at most 12 accumulator tiles each)
   static constexpr int CS = Dims<P>::CS;    // plan code record bytes per element
   static constexpr int WARPS = 4;           // warps per CTA
-  // Stiffness layout: component-major node tiles at p = 2, 3 (two tiles of 8 nodes),
-  // interleaved rows r = 2a + i at p = 4 (50 rows in seven tiles, where node tiles
-  // would pad 25 nodes to 32 and need 280 instead of 196 MMAs per element).
-  static constexpr bool IL = (P == 4);
-  static constexpr int NTAB = IL ? K4 : NTN;  // table tiles per k-step
-  static constexpr int TABW = IL ? 16 : 32;   // table entries per (k-step, tile): lane, or (g/2, t)
-  static_assert(P >= 2 && P <= 4 && (IL || NTN == 2), "fragment kernel: orders 2 to 4");
+  static_assert(P >= 2 && P <= 4 && (NN == 8 * NTM || EX), "fragment kernel: orders 2 to 4");
+  // Node-tile pair k = (ta, tb) of a pass: pass 0 the pairs of tiles 0 and 1 (order 2: of
+  // tile 0), pass 1 those of tile 2.
+  static constexpr int NPAIR = NTM == 1 ? 1 : 3;
+  __host__ __device__ static constexpr int ta(int pass, int k) { return pass ? k : (k == 2 ? 1 : 0); }
+  __host__ __device__ static constexpr int tb(int pass, int k) { return pass ? 2 : (k == 0 ? 0 : 1); }
 };
 
 template <int V>
@@ -100,7 +104,7 @@ using IC = std::integral_constant<int, V>;
 template <int P, bool DROP = false, bool NL = false, bool B16 = false, bool JAC = true>
 struct FragLayout {
   using F = FragDims<P>;
-  static constexpr int K4 = F::K4, NTN = F::NTN, NQP = F::NQP, NN = F::NN;
+  static constexpr int K4 = F::K4, NQP = F::NQP, NN = F::NN;
   static constexpr int CS = DROP ? 4 * NN * NN : F::CS;  // staged bytes per element
   // Slot of quadrature point q of an element's arrays, and the slots between the two
   // elements: a quarter-warp of the quadrature stage stores points q, q + 1 of two
@@ -109,8 +113,9 @@ struct FragLayout {
   static constexpr int PS = (NQP + 2 * ((NQP - 1) / 8) + 11) / 8 * 8 - 4;
   __host__ __device__ static constexpr int slot(int q) { return q + 2 * (q >> 3); }
   static constexpr size_t tabJ = 0;                          // double2 [K4][QT][32]
-  static constexpr size_t tabF = tabJ + 16 * K4 * F::QT * 32;  // double2 [K4][NTAB][TABW]
-  static constexpr size_t wq = tabF + 16 * K4 * F::NTAB * F::TABW;  // double [NQP]
+  static constexpr size_t tabF = tabJ + 16 * K4 * F::QT * 32;  // double2 [K4][NTM][32]
+  static constexpr size_t tabX = tabF + 16 * K4 * F::NTM * 32;  // double2 [NQP]: dN of the node outside the tiles
+  static constexpr size_t wq = tabX + (F::EX ? 16 * NQP : 0);  // double [NQP]
   static constexpr size_t csum = align16(wq + 8 * NQP);       // double2 [NQP]: sum_a dN(a, q)
   static constexpr size_t tabB = align16(csum + 16 * NQP);    // double2 [8][32]: BF16x6 stiffness operands
   static constexpr size_t tabR = align16(tabB + (B16 ? 16 * 8 * 32 : 0));  // uint32 [64]: runs (order 3)
@@ -125,9 +130,9 @@ struct FragLayout {
   static constexpr size_t NID = MC + 16;            // int [2][NN]: node ids
   static constexpr size_t RB = align16(NID + 4 * 2 * NN);  // int [2][NN]: rowp[node]
   static constexpr size_t STAGE = align16(RB + 4 * 2 * NN);  // [2 buffers][2 elements][CS] code records
-  // staging slots: p = 3, 3 node-tile pairs x 2 halves, direct and transposed; p = 2,
-  // the (at most 8) blocks one lane writes per element; p = 4, a ring of 4 per lane
-  static constexpr int NSLOT = F::IL ? 4 : 8;
+  // staging slots: p = 3, 3 node-tile pairs x 2 halves, direct and transposed; p = 2, 4, the
+  // blocks one lane has in flight
+  static constexpr int NSLOT = P == 3 ? 8 : 4;
   static constexpr size_t REDS = align16(STAGE + 2 * 2 * CS);  // double4 [NSLOT][32]: bulk-reduction sources
   // NONLINEAR: sign(s) x tangent modulus, double [2][NQP][2 (l)][8 (i, k, n)]
   static constexpr size_t AT = align16(REDS + (JAC ? 32 * NSLOT * 32 : 0));
@@ -188,7 +193,7 @@ template <int P, bool B16 = false, bool NL = false>
 __device__ __forceinline__ void frag_prologue(unsigned char *smem) {
   using F = FragDims<P>;
   using L = FragLayout<P, false, false, B16>;
-  constexpr int P1 = F::P1, NN = F::NN, NQ = F::NQ, K4 = F::K4, QT = F::QT, NTAB = F::NTAB, TABW = F::TABW;
+  constexpr int P1 = F::P1, NN = F::NN, NQ = F::NQ, K4 = F::K4, QT = F::QT, NTM = F::NTM;
   double2 *tabJ = reinterpret_cast<double2 *>(smem + L::tabJ);
   double2 *tabF = reinterpret_cast<double2 *>(smem + L::tabF);
   double *wq = reinterpret_cast<double *>(smem + L::wq);
@@ -205,20 +210,15 @@ __device__ __forceinline__ void frag_prologue(unsigned char *smem) {
     const int a = 4 * ks + (lane & 3), q = 8 * tm + (lane >> 2);
     tabJ[i] = (a < NN && q < NQ) ? dN(a, q) : make_double2(0.0, 0.0);
   }
-  // stiffness fragments at (ks, T), q = 4ks + t: component-major, lane (g, t) holds
-  // dN(a = 8T + pi(g), q); interleaved, entry 4(g/2) + t holds dN(a = 4T + g/2, q)
-  for (int i = threadIdx.x; i < K4 * NTAB * TABW; i += blockDim.x) {
-    const int e = i % TABW, blk = i / TABW, ks = blk / NTAB, T = blk - ks * NTAB;
-    int a, q;
-    if constexpr (F::IL) {
-      a = 4 * T + (e >> 2);
-      q = 4 * ks + (e & 3);
-    } else {
-      const int g = e >> 2, t = e & 3;
-      a = 8 * T + 4 * (g & 1) + (g >> 1);
-      q = 4 * ks + t;
-    }
-    tabF[i] = (a < NN && q < NQ) ? dN(a, q) : make_double2(0.0, 0.0);
+  // stiffness fragments at (ks, T): lane (g, t) holds dN(a = 8T + pi(g), q = 4ks + t)
+  for (int i = threadIdx.x; i < K4 * NTM * 32; i += blockDim.x) {
+    const int lane = i & 31, blk = i >> 5, ks = blk / NTM, T = blk - ks * NTM;
+    const int g = lane >> 2, t = lane & 3, a = 8 * T + 4 * (g & 1) + (g >> 1), q = 4 * ks + t;
+    tabF[i] = q < NQ ? dN(a, q) : make_double2(0.0, 0.0);
+  }
+  if constexpr (F::EX) {
+    double2 *tabX = reinterpret_cast<double2 *>(smem + L::tabX);
+    for (int q = threadIdx.x; q < F::NQP; q += blockDim.x) tabX[q] = q < NQ ? dN(NN - 1, q) : make_double2(0.0, 0.0);
   }
   // Gauss weights (NONLINEAR), their square roots (LINEAR)
   for (int q = threadIdx.x; q < F::NQP; q += blockDim.x) {
@@ -453,8 +453,7 @@ __device__ __forceinline__ bool frag_put_block(const Out &O, int el, int r0, int
                "@s st.shared.v2.f64 [%1], {%2, %3};\n\t"
                "@s st.shared.v2.f64 [%1 + 16], {%4, %5};\n\t}" ::"l"(blk),
                "r"((unsigned)__cvta_generic_to_shared(slot)), "d"(v0), "d"(v1), "d"(v2), "d"(v3),
-               "r"(act ? first : 0u), "r"((uint32_t)add)
-               : "memory");
+               "r"(act ? first : 0u), "r"((uint32_t)add));
   return add;
 }
 
@@ -705,11 +704,13 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
   using F = FragDims<P>;
   constexpr bool STRIP = Gen::kStrip;
   using L = FragLayout<P, !PLAN, NL, B16, (MODE & kJac) != 0>;
-  constexpr int NN = F::NN, NQ = F::NQ, K4 = F::K4, QT = F::QT, NTN = F::NTN, NQP = F::NQP, PS = L::PS, CS = F::CS;
+  constexpr int NN = F::NN, NQ = F::NQ, K4 = F::K4, QT = F::QT, NTM = F::NTM, NQP = F::NQP, PS = L::PS, CS = F::CS;
+  constexpr bool EX = F::EX;  // node XN is in no tile
+  constexpr int XN = NN - 1, NPAIR = F::NPAIR;
   constexpr int STG = L::CS;  // staged bytes per element: plan code record or map rows
   constexpr bool RES = (MODE & kRes) != 0, JAC = (MODE & kJac) != 0;
   constexpr bool RUNS = (P == 3);  // order 3: staged row runs, one bulk reduction per adjacent run
-  static_assert(!NL || !F::IL, "NONLINEAR strain: orders 2 and 3");
+  static_assert(!NL || P < 4, "NONLINEAR strain: orders 2 and 3");
   static_assert(PLAN || !Gen::kBatched, "drop-in mode assembles one mesh");
   static_assert(!STRIP || (PLAN && JAC && !NL && P == kStripOrder), "strips: LINEAR Jacobians of plans, order 3");
   static_assert(!B16 || (!NL && P == 3), "BF16x6 stiffness: LINEAR, order 3");
@@ -723,6 +724,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
   const int e_ld = g >> 2, c_ld = g & 3;  // element / component this lane gathers
   const double2 *tabJ = reinterpret_cast<const double2 *>(smem + L::tabJ);
   const double2 *tabF = reinterpret_cast<const double2 *>(smem + L::tabF);
+  const double2 *tabX = reinterpret_cast<const double2 *>(smem + L::tabX);
   const double *wqs = reinterpret_cast<const double *>(smem + L::wq);
   const double2 *csum = reinterpret_cast<const double2 *>(smem + L::csum);
   const double2 *tabB = reinterpret_cast<const double2 *>(smem + L::tabB);
@@ -1046,13 +1048,9 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
       crx = __shfl_down_sync(0xffffffffu, sx, 24);
       cry = __shfl_down_sync(0xffffffffu, sy, 24);
     };
-    if constexpr (!F::IL) {
-      // node tiles on the tensor cores: both at p = 3; at p = 2 only tile 0 (nodes 0-7),
-      // node 8 (alone in tile 1) has its row and column on the FP64 pipe (12 instead of
-      // 36 MMAs per element)
-      constexpr int NTM = (P == 2) ? 1 : NTN;
-      constexpr int NPAIR = NTM * (NTM + 1) / 2;
+    {
       const int pa = 4 * (g & 1) + (g >> 1);  // pi(g)
+      int half = 0;  // orders 2 and 4: half of the lane's staging slots the next blocks use
       for (int el = 0; el < ne; el++) {
         // Strips: the blocks of an edge's nodes among themselves and their residual rows
         // belong to the element right of it; lanes (g = 6, 7; t = 3) hold exactly those
@@ -1200,45 +1198,56 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
         }
         // 3.-5. quadrature k-steps outermost: per step each lane forms its fragments
         // G-hat_i(q = 4ks + t, a = 8T + pi(g)), adds its residual partials and issues
-        // the 4 NPAIR independent stiffness MMAs of all node-tile pairs
-        double acc[NPAIR][4][2];
-        double rp[NTN][2];
-        double n8[4] = {0.0, 0.0, 0.0, 0.0}, d8[4] = {0.0, 0.0, 0.0, 0.0};  // p = 2: M[8][pi(g)], M[8][8]
-  #pragma unroll
-        for (int T = 0; T < NTN; T++) rp[T][0] = rp[T][1] = 0.0;
+        // the 4 NPAIR independent stiffness MMAs of the pass's node-tile pairs.  Orders 2
+        // and 4: the node outside the tiles has its row and column on the FP64 pipe, each
+        // lane forming its G-hat(q, XN) itself (order 4: 168 instead of the 280 MMAs of a
+        // fourth node tile).
         // whether a point of this element has s (mu) < 0 (inverted element or negative
         // thickness or modulus): only then do the A fragments take the points' signs
         const bool neg = SCALED && (negm & (el ? 0xccccccccu : 0x33333333u)) != 0;
+        auto pass = [&](auto passc) {
+        constexpr int PASS = decltype(passc)::value;
+        // fragments of tiles [0, NF); residual slots: tiles RT0 and RT1, NTM = node XN;
+        // xs[0], xs[1]: M[XN][tile] (orders 2: tile 0; 4: tiles 0, 1 | 2) and M[XN][XN]
+        constexpr int NF = PASS ? 3 : (NTM == 1 ? 1 : 2);
+        [[maybe_unused]] constexpr int RT0 = PASS ? 2 : 0, RT1 = PASS || NTM == 1 ? NTM : 1;
+        constexpr bool XD = EX && RT1 == NTM;  // this pass has XN's own row
+        double acc[NPAIR][4][2];
+        double rp[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+        double xs[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
         auto kstep = [&](int ks, auto firstc, auto negc) {
           constexpr bool FIRST = decltype(firstc)::value, NEG = decltype(negc)::value;
           const int o = el * PS + L::slot(4 * ks) + t;
           const double2 w0 = WI0[o], w1 = WI1[o];
-          double fr[NTN][2];
+          double fr[NTM][2];
   #pragma unroll
-          for (int T = 0; T < NTN; T++) {
-            const double2 d = tabF[(ks * NTN + T) * 32 + lane];
+          for (int T = 0; T < NF; T++) {
+            const double2 d = tabF[(ks * NTM + T) * 32 + lane];
             fr[T][0] = fma(w0.x, d.x, w0.y * d.y);
             fr[T][1] = fma(w1.x, d.x, w1.y * d.y);
+          }
+          double h0 = 0.0, h1 = 0.0;  // G-hat(q, XN)
+          if constexpr (EX && (JAC || XD)) {
+            const double2 d = tabX[4 * ks + t];
+            h0 = fma(w0.x, d.x, w0.y * d.y);
+            h1 = fma(w1.x, d.x, w1.y * d.y);
           }
           if constexpr (RES) {
             // LINEAR: the stress is symmetric, S-hat_yx = S-hat_xy
             const double2 s0 = WS0[o];
             const double s1y = WS1[o].y, s1x = NL ? WS1[o].x : s0.y;
   #pragma unroll
-            for (int T = 0; T < NTN; T++) {
-              rp[T][0] = fma(fr[T][0], s0.x, fma(fr[T][1], s1x, rp[T][0]));
-              rp[T][1] = fma(fr[T][0], s0.y, fma(fr[T][1], s1y, rp[T][1]));
+            for (int x = 0; x < 2; x++) {
+              const int T = x ? RT1 : RT0;
+              const double f0 = T == NTM ? h0 : fr[T < NTM ? T : 0][0], f1 = T == NTM ? h1 : fr[T < NTM ? T : 0][1];
+              rp[x][0] = fma(f0, s0.x, fma(f1, s1x, rp[x][0]));
+              rp[x][1] = fma(f0, s0.y, fma(f1, s1y, rp[x][1]));
             }
           }
           if constexpr (JAC && NL) {
             // K_ik[a][b] = sum over (q, l) of G-hat_l(q, a) B_ikl(q, b),
             // B_ikl = sign(s) sum_n A_{il,kn} G-hat_n(q, b): 4 (i, k) x 2 (l) MMAs per pair
             const double *at = ATs + (el * NQP + 4 * ks + t) * 16;
-            double h0 = 0.0, h1 = 0.0;
-            if constexpr (P == 2) {
-              h0 = __shfl_sync(0xffffffffu, fr[1][0], t);
-              h1 = __shfl_sync(0xffffffffu, fr[1][1], t);
-            }
 #pragma unroll
             for (int ll = 0; ll < 2; ll++) {
               double C[2][2][2];  // [i][k][n]
@@ -1248,80 +1257,66 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
                 C[j >> 1][j & 1][0] = v.x;
                 C[j >> 1][j & 1][1] = v.y;
               }
-              int k = 0;
 #pragma unroll
-              for (int TA = 0; TA < NTM; TA++) {
+              for (int k = 0; k < NPAIR; k++) {
+                const int TA = F::ta(PASS, k), TB = F::tb(PASS, k);
 #pragma unroll
-                for (int TB = TA; TB < NTM; TB++, k++) {
-#pragma unroll
-                  for (int ik = 0; ik < 4; ik++) {
-                    const double bv = fma(C[ik >> 1][ik & 1][0], fr[TB][0], C[ik >> 1][ik & 1][1] * fr[TB][1]);
-                    if (FIRST && ll == 0) dmma_first(acc[k][ik][0], acc[k][ik][1], fr[TA][ll], bv);
-                    else dmma(acc[k][ik][0], acc[k][ik][1], fr[TA][ll], bv);
-                  }
+                for (int ik = 0; ik < 4; ik++) {
+                  const double bv = fma(C[ik >> 1][ik & 1][0], fr[TB][0], C[ik >> 1][ik & 1][1] * fr[TB][1]);
+                  if (FIRST && ll == 0) dmma_first(acc[k][ik][0], acc[k][ik][1], fr[TA][ll], bv);
+                  else dmma(acc[k][ik][0], acc[k][ik][1], fr[TA][ll], bv);
                 }
               }
-              if constexpr (P == 2) {
+              if constexpr (EX) {
                 const double hl = ll ? h1 : h0;
 #pragma unroll
                 for (int ik = 0; ik < 4; ik++) {
-                  n8[ik] = fma(hl, fma(C[ik >> 1][ik & 1][0], fr[0][0], C[ik >> 1][ik & 1][1] * fr[0][1]), n8[ik]);
-                  d8[ik] = fma(hl, fma(C[ik >> 1][ik & 1][0], h0, C[ik >> 1][ik & 1][1] * h1), d8[ik]);
+                  xs[0][ik] = fma(hl, fma(C[ik >> 1][ik & 1][0], fr[0][0], C[ik >> 1][ik & 1][1] * fr[0][1]), xs[0][ik]);
+                  xs[1][ik] = fma(hl, fma(C[ik >> 1][ik & 1][0], h0, C[ik >> 1][ik & 1][1] * h1), xs[1][ik]);
                 }
               }
             }
           }
-          if constexpr (JAC && P == 2 && !NL) {
-            // G-hat_i(q, 8) sits in lane (g = 0, t), tile 1
-            const double h0 = __shfl_sync(0xffffffffu, fr[1][0], t), h1 = __shfl_sync(0xffffffffu, fr[1][1], t);
-            const double s0 = NEG ? SGs[el * NQP + 4 * ks + t] * h0 : h0, s1 = NEG ? SGs[el * NQP + 4 * ks + t] * h1 : h1;
-            n8[0] = fma(s0, fr[0][0], n8[0]);
-            n8[1] = fma(s0, fr[0][1], n8[1]);
-            n8[2] = fma(s1, fr[0][0], n8[2]);
-            n8[3] = fma(s1, fr[0][1], n8[3]);
-            d8[0] = fma(s0, h0, d8[0]);
-            d8[1] = fma(s0, h1, d8[1]);
-            d8[2] = fma(s1, h0, d8[2]);
-            d8[3] = fma(s1, h1, d8[3]);
-          }
           if constexpr (JAC && !NL) {
-            int k = 0;
+            double sg = 1.0;
+            if constexpr (NEG) sg = SGs[el * NQP + 4 * ks + t];
+            double af[NTM][2];  // A fragments: times the point's sign
   #pragma unroll
-            for (int TA = 0; TA < NTM; TA++) {
-              double a0 = fr[TA][0], a1 = fr[TA][1];
-              if constexpr (NEG) {
-                a0 *= SGs[el * NQP + 4 * ks + t];
-                a1 *= SGs[el * NQP + 4 * ks + t];
+            for (int T = 0; T < NF; T++) af[T][0] = NEG ? sg * fr[T][0] : fr[T][0], af[T][1] = NEG ? sg * fr[T][1] : fr[T][1];
+  #pragma unroll
+            for (int k = 0; k < NPAIR; k++) {
+              const int TA = F::ta(PASS, k), TB = F::tb(PASS, k);
+  #pragma unroll
+              for (int ij = 0; ij < 4; ij++) {
+                if constexpr (FIRST) dmma_first(acc[k][ij][0], acc[k][ij][1], af[TA][ij >> 1], fr[TB][ij & 1]);
+                else dmma(acc[k][ij][0], acc[k][ij][1], af[TA][ij >> 1], fr[TB][ij & 1]);
               }
+            }
+            if constexpr (EX) {
+              const double s0 = NEG ? sg * h0 : h0, s1 = NEG ? sg * h1 : h1;
   #pragma unroll
-              for (int TB = TA; TB < NTM; TB++, k++) {
-                if constexpr (FIRST) {
-                  dmma_first(acc[k][0][0], acc[k][0][1], a0, fr[TB][0]);
-                  dmma_first(acc[k][1][0], acc[k][1][1], a0, fr[TB][1]);
-                  dmma_first(acc[k][2][0], acc[k][2][1], a1, fr[TB][0]);
-                  dmma_first(acc[k][3][0], acc[k][3][1], a1, fr[TB][1]);
-                } else {
-                  dmma(acc[k][0][0], acc[k][0][1], a0, fr[TB][0]);
-                  dmma(acc[k][1][0], acc[k][1][1], a0, fr[TB][1]);
-                  dmma(acc[k][2][0], acc[k][2][1], a1, fr[TB][0]);
-                  dmma(acc[k][3][0], acc[k][3][1], a1, fr[TB][1]);
-                }
+              for (int x = 0; x < 2; x++) {
+                const int T = x ? RT1 : RT0;
+                const double f0 = T == NTM ? h0 : fr[T < NTM ? T : 0][0], f1 = T == NTM ? h1 : fr[T < NTM ? T : 0][1];
+                xs[x][0] = fma(s0, f0, xs[x][0]);
+                xs[x][1] = fma(s0, f1, xs[x][1]);
+                xs[x][2] = fma(s1, f0, xs[x][2]);
+                xs[x][3] = fma(s1, f1, xs[x][3]);
               }
             }
           }
         };
         kstep_all(kstep, neg);
-        // residual: sum over the four lanes t of a node (reduce-scatter over node tiles)
+        // residual: sum over the four lanes t of a node (reduce-scatter over the two slots)
+        const int Tm = t >> 1, To = Tm ^ 1;
         if constexpr (RES) {
-          const int Tm = t >> 1, To = Tm ^ 1;
           double sx = (Tm ? rp[1][0] : rp[0][0]) + __shfl_xor_sync(0xffffffffu, To ? rp[1][0] : rp[0][0], 2);
           double sy = (Tm ? rp[1][1] : rp[0][1]) + __shfl_xor_sync(0xffffffffu, To ? rp[1][1] : rp[0][1], 2);
           sx += __shfl_xor_sync(0xffffffffu, sx, 1);
           sy += __shfl_xor_sync(0xffffffffu, sy, 1);
           if constexpr (STRIP) residual_carry(sx, sy, cin);
-          const int a = 8 * Tm + pa;
-          const bool act = (t & 1) == 0 && a < NN && !halo && !(right && g >= 6);
-          const int an = a < NN ? a : 0;
+          const int an = Tm == 0 ? 8 * RT0 + pa : (RT1 == NTM ? XN : 8 * RT1 + pa);
+          const bool act = (t & 1) == 0 && (Tm == 0 || RT1 < NTM || g == 0) && !halo && !(right && g >= 6);
           residual_put(M.residual + 2 * (int64_t)nid[el * NN + an], act, PLAN && O.codes[el * CS + NN * NN + an], sx, sy);
         }
         if constexpr (JAC && RUNS) {
@@ -1384,11 +1379,10 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
             direct(IC<2>{}, IC<1>{});
             allfirst &= ct[0] & ct[1];
           } else {
-            int k = 0;
   #pragma unroll
-            for (int TA = 0; TA < NTN; TA++) {
-  #pragma unroll
-              for (int TB = TA; TB < NTN; TB++, k++) {
+            for (int k = 0; k < NPAIR; k++) {
+              {
+                const int TA = F::ta(0, k), TB = F::tb(0, k);
                 const int a = 8 * TA + pa;
   #pragma unroll
                 for (int h = 0; h < 2; h++) {
@@ -1414,21 +1408,22 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
           }
           issue_runs(O, el, !halo && (allfirst & 0x80u) == 0);
         }
-        // stiffness blocks, order 2: lane (g, t) writes (pi(g), 4h + t), h = 0, 1 (NONLINEAR:
-        // for a <= b, and the exact transpose), and lanes t < 2 / (g = 0, t = 2) a node-8
-        // block: (8, pi(g)), its transpose, (8, 8); first stores go out at once, the blocks
-        // to add are staged and leave after one proxy fence, as one bulk group (a fence
-        // per block cost 5 % of the order-2 time; NONLINEAR: three groups, for registers)
-        if constexpr (JAC && P == 2) {
-          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        // stiffness blocks, orders 2 and 4: lane (g, t) writes (8TA + pi(g), 8TB + 4h + t) of
+        // each pair and, for TA < TB, its transpose (NONLINEAR diagonal pairs: for a <= b,
+        // and the exact transpose); then the row and column of node XN: of the two slots of
+        // xs, lanes t/2 = x take slot x, t even (XN, a), t odd its transpose.  First stores
+        // go out at once, the blocks to add are staged and leave FL at a time after one
+        // proxy fence, as one bulk group, from two halves of the lane's slots in turn.
+        if constexpr (JAC && EX) {
+          constexpr int FL = P == 2 && !NL ? 3 : 2, HALF = FL == 2 ? 2 : 0;
           double *reds = redsW + 4 * lane;
-          double *dst[3];
-          bool add[3] = {false, false, false};
-          double kxx, kxy, kyx, kyy;
-          auto issue = [&](int s0, int s1) {  // the staged blocks of slots [s0, s1)
+          double *dst[FL];
+          bool add[FL];
+          int n = 0;
+          auto flush = [&](int m) {
             bool any = false;
 #pragma unroll
-            for (int x = 0; x < 3; x++) any = any || (x >= s0 && x < s1 && add[x]);
+            for (int x = 0; x < FL; x++) any = any || (x < m && add[x]);
             if (!__any_sync(0xffffffffu, any)) return;
             if (PLAN && el > 0) pair_first_landed();
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1437,201 +1432,53 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
               pair_first_visible();
             }
 #pragma unroll
-            for (int x = 0; x < 3; x++)
-              if (x >= s0 && x < s1) bulk_add_block(dst[x], reds + 128 * x, add[x]);
+            for (int x = 0; x < FL; x++)
+              if (x < m) bulk_add_block(dst[x], reds + 128 * (HALF * half + x), add[x]);
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            half ^= 1;
           };
-#pragma unroll
-          for (int h = 0; h < 2; h++) {
-            const int b = 4 * h + t;
-            block(acc[0][0][h], acc[0][1][h], acc[0][2][h], acc[0][3][h], kxx, kxy, kyx, kyy);
-            if constexpr (NL) {
-              if (h) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-              add[0] = frag_put_block<P, PLAN>(O, el, pa, b, pa <= b, kxx, kxy, kyx, kyy, reds, dst[0]);
-              add[1] = frag_put_block<P, PLAN>(O, el, b, pa, pa < b, kxx, kyx, kxy, kyy, reds + 128, dst[1]);
-              issue(0, 2);
-            } else {
-              add[h] = frag_put_block<P, PLAN>(O, el, pa, b, true, kxx, kxy, kyx, kyy, reds + 128 * h, dst[h]);
+          auto put = [&](int r, int c, bool act, double v0, double v1, double v2, double v3) {
+            // the bulk reads of the slots used next are complete
+            if (n == 0) {
+              if constexpr (HALF) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+              else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
             }
-          }
-          // sum the node-8 partials over the four lanes t
+            add[n] = frag_put_block<P, PLAN>(O, el, r, c, act, v0, v1, v2, v3, reds + 128 * (HALF * half + n), dst[n]);
+            if (++n == FL) {
+              flush(FL);
+              n = 0;
+            }
+          };
+          double kxx, kxy, kyx, kyy;
+#pragma unroll
+          for (int k = 0; k < NPAIR; k++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+              const int TA = F::ta(PASS, k), TB = F::tb(PASS, k);
+              const int a = 8 * TA + pa, b = 8 * TB + 4 * h + t;
+              const bool diag = NL && TA == TB;
+              block(acc[k][0][h], acc[k][1][h], acc[k][2][h], acc[k][3][h], kxx, kxy, kyx, kyy);
+              put(a, b, !diag || a <= b, kxx, kxy, kyx, kyy);
+              if (TA < TB || diag) put(b, a, !diag || a < b, kxx, kyx, kxy, kyy);
+            }
+          double xv[4];
 #pragma unroll
           for (int c = 0; c < 4; c++) {
-            n8[c] += __shfl_xor_sync(0xffffffffu, n8[c], 1);
-            n8[c] += __shfl_xor_sync(0xffffffffu, n8[c], 2);
-            d8[c] += __shfl_xor_sync(0xffffffffu, d8[c], 1);
-            d8[c] += __shfl_xor_sync(0xffffffffu, d8[c], 2);
+            xv[c] = (Tm ? xs[1][c] : xs[0][c]) + __shfl_xor_sync(0xffffffffu, To ? xs[1][c] : xs[0][c], 2);
+            xv[c] += __shfl_xor_sync(0xffffffffu, xv[c], 1);
           }
-          const bool diag = t == 2;
-          block(diag ? d8[0] : n8[0], diag ? d8[1] : n8[1], diag ? d8[2] : n8[2], diag ? d8[3] : n8[3], kxx, kxy, kyx, kyy);
-          add[2] = frag_put_block<P, PLAN>(O, el, t == 1 ? pa : 8, t == 0 ? pa : 8, t < 2 || (g == 0 && diag), kxx,
-                                           t == 1 ? kyx : kxy, t == 1 ? kxy : kyx, kyy, reds + 128 * 2, dst[2]);
-          issue(NL ? 2 : 0, 3);
-        }
-      }
-    } else {
-      // interleaved rows r = 2a + i (p = 4): lane (g, t) builds G-hat_i(q = 4ks + t,
-      // a = 4T + g/2), i = g%2, the A fragment of row tile T and the B fragment of
-      // column tile T; lanes l and l^4 hold the two rows of a 2x2 block.  The stiffness
-      // takes one pass per group of tile pairs; the residual rides on the first three
-      // groups (a pass of its own when the Jacobian is not assembled).
-      const int ii = g & 1, ah = g >> 1;
-      const double2 *WIi = ii ? WI1 : WI0;
-      const double2 *WSi = ii ? WS1 : WS0;
-      double *reds = redsW + 4 * lane;
-      int half = 0;  // half of the lane's staging slots the next batch uses
-      for (int el = 0; el < ne; el++) {
-        if (PLAN && el > 0) pair_order_fence();
-        const bool neg = (negm & (el ? 0xccccccccu : 0x33333333u)) != 0;
-        // residual R_(a,i'): lane partials rp over its quadrature points (with the
-        // Jacobian, accumulated by the first three stiffness groups, which between them
-        // form every column tile's fragments; alone, in a pass of its own), then a full
-        // sum over the component pair (xor 4) and a reduce-scatter over the four lanes
-        // t (lane t ends with tiles 2t and 2t + 1)
-        double rp[8][2];
-#pragma unroll
-        for (int T = 0; T < 8; T++) rp[T][0] = rp[T][1] = 0.0;
-        auto res_write = [&]() {
-#pragma unroll
-          for (int T = 0; T < K4; T++)
-#pragma unroll
-            for (int c = 0; c < 2; c++) rp[T][c] += __shfl_xor_sync(0xffffffffu, rp[T][c], 4);
-          const int hi = t >> 1, lo = t & 1;
-          double w4[4][2], z[2][2];
-#pragma unroll
-          for (int k = 0; k < 4; k++)
-#pragma unroll
-            for (int c = 0; c < 2; c++)
-              w4[k][c] = (hi ? rp[4 + k][c] : rp[k][c]) + __shfl_xor_sync(0xffffffffu, hi ? rp[k][c] : rp[4 + k][c], 2);
-#pragma unroll
-          for (int mm = 0; mm < 2; mm++)
-#pragma unroll
-            for (int c = 0; c < 2; c++)
-              z[mm][c] = (lo ? w4[2 + mm][c] : w4[mm][c]) + __shfl_xor_sync(0xffffffffu, lo ? w4[mm][c] : w4[2 + mm][c], 1);
-#pragma unroll
-          for (int mm = 0; mm < 2; mm++) {
-            const int a = 4 * (2 * t + mm) + ah;
-            const int an = a < NN ? a : 0;
-            residual_put(M.residual + 2 * (int64_t)nid[el * NN + an], ii == 0 && a < NN,
-                         PLAN && O.codes[el * CS + NN * NN + an], z[mm][0], z[mm][1]);
-          }
-        };
-        if constexpr (RES && !JAC) {
-#pragma unroll
-          for (int ks = 0; ks < K4; ks++) {
-            const int o = el * PS + L::slot(4 * ks) + t;
-            const double2 w = WIi[o];
-            const double2 sj = WSi[o];  // (S-hat_xj, S-hat_yj), j = this lane's component
-#pragma unroll
-            for (int C = 0; C < K4; C++) {
-              const double2 d = tabF[(ks * K4 + C) * 16 + 4 * ah + t];
-              const double gv = fma(w.x, d.x, w.y * d.y);
-              rp[C][0] = fma(gv, sj.x, rp[C][0]);
-              rp[C][1] = fma(gv, sj.y, rp[C][1]);
-            }
-          }
-          res_write();
-        }
-        // stiffness: the 28 tile pairs (R, C >= R) in four groups, each a triangle
-        // {R0..R1-1}^2 or a rectangle {R0..R1-1} x {C0..C1-1} of the upper triangle
-        // (at most ten live accumulator tiles); within a group the k-steps are
-        // outermost and each fragment of the group's rows and columns is formed once
-        // per step: 17 fragment builds per k-step for the 28 tile pairs
-        auto group = [&](auto r0c, auto r1c, auto c0c, auto c1c, auto resc) {
-          constexpr int R0 = decltype(r0c)::value, R1 = decltype(r1c)::value;
-          constexpr int C0 = decltype(c0c)::value, C1 = decltype(c1c)::value;
-          constexpr bool GRES = RES && decltype(resc)::value;  // residual tiles C0..C1-1
-          double acc[R1 - R0][C1 - C0][2];
-#pragma unroll
-          for (int R = R0; R < R1; R++)
-#pragma unroll
-            for (int C = C0; C < C1; C++) acc[R - R0][C - C0][0] = acc[R - R0][C - C0][1] = 0.0;
-#pragma unroll
-          for (int ks = 0; ks < K4; ks++) {
-            const int o = el * PS + L::slot(4 * ks) + t;
-            const double2 w = WIi[o];
-            double fr[K4];
-#pragma unroll
-            for (int T = 0; T < K4; T++) {
-              if ((T >= R0 && T < R1) || (T >= C0 && T < C1)) {
-                const double2 d = tabF[(ks * K4 + T) * 16 + 4 * ah + t];
-                fr[T] = fma(w.x, d.x, w.y * d.y);
-              }
-            }
-            if constexpr (GRES) {
-              const double2 sj = WSi[o];
-#pragma unroll
-              for (int C = C0; C < C1; C++) {
-                rp[C][0] = fma(fr[C], sj.x, rp[C][0]);
-                rp[C][1] = fma(fr[C], sj.y, rp[C][1]);
-              }
-            }
-#pragma unroll
-            for (int R = R0; R < R1; R++) {
-              const double af = neg ? SGs[el * NQP + 4 * ks + t] * fr[R] : fr[R];
-#pragma unroll
-              for (int C = (R > C0 ? R : C0); C < C1; C++)
-                dmma(acc[R - R0][C - C0][0], acc[R - R0][C - C0][1], af, fr[C]);
-            }
-          }
-          // blocks: lane pair (l, l^4) exchanges rows; lane i = 0 writes (a, b), lane
-          // i = 1 writes (b, a) = (a, b)^T; the blocks to add leave in batches of two, from
-          // two halves of the lane's four slots in turn
-          constexpr int H = 2;
-          double *dst[H];
-          bool add[H];
-          int n = 0;
-          auto flush = [&](int m) {
-            bool any = add[0];
-            if (m > 1) any = any || add[1];
-            if (__any_sync(0xffffffffu, any)) {
-              asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-#pragma unroll
-              for (int x = 0; x < H; x++)
-                if (x < m) bulk_add_block(dst[x], reds + 128 * (H * half + x), add[x]);
-              half ^= 1;
-            }
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-          };
-#pragma unroll
-          for (int R = R0; R < R1; R++) {
-            const int a = 4 * R + ah;
-#pragma unroll
-            for (int C = (R > C0 ? R : C0); C < C1; C++) {
-              const double o0 = __shfl_xor_sync(0xffffffffu, acc[R - R0][C - C0][0], 4);
-              const double o1 = __shfl_xor_sync(0xffffffffu, acc[R - R0][C - C0][1], 4);
-              const double mxx = ii ? o0 : acc[R - R0][C - C0][0], mxy = ii ? o1 : acc[R - R0][C - C0][1];
-              const double myx = ii ? acc[R - R0][C - C0][0] : o0, myy = ii ? acc[R - R0][C - C0][1] : o1;
-              const int b = 4 * C + t;
-              double kxx, kxy, kyx, kyy;
-              block(mxx, mxy, myx, myy, kxx, kxy, kyx, kyy);
-              // the half's previous bulk reads are complete
-              if (n == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-              add[n] = frag_put_block<P, PLAN>(O, el, ii ? b : a, ii ? a : b, a < NN && b < NN && (ii ? a < b : a <= b), kxx,
-                                               ii ? kyx : kxy, ii ? kxy : kyx, kyy, reds + 128 * (H * half + n), dst[n]);
-              if (++n == H) {
-                flush(H);
-                n = 0;
-              }
-            }
-          }
+          block(xv[0], xv[1], xv[2], xv[3], kxx, kxy, kyx, kyy);
+          const int xa = Tm == 0 ? 8 * RT0 + pa : (RT1 == NTM ? XN : 8 * RT1 + pa);
+          const bool tr = t & 1;
+          put(tr ? xa : XN, tr ? XN : xa, Tm == 0 || RT1 < NTM || (g == 0 && !tr), kxx, tr ? kyx : kxy, tr ? kxy : kyx, kyy);
           if (n) flush(n);
+        }
         };
-        if constexpr (JAC) {
-          static_assert(K4 == 7, "tile-pair groups of the order-4 layout");
-          // compiler barriers keep each group's table loads inside the group (hoisting
-          // them across groups raises register pressure past the budget)
+        pass(IC<0>{});
+        if constexpr (F::NPASS == 2) {
+          // keeps each pass's table loads inside the pass (registers)
           asm volatile("" ::: "memory");
-          group(IC<0>{}, IC<3>{}, IC<0>{}, IC<3>{}, std::true_type{});
-          asm volatile("" ::: "memory");
-          group(IC<0>{}, IC<3>{}, IC<3>{}, IC<5>{}, std::true_type{});
-          asm volatile("" ::: "memory");
-          group(IC<0>{}, IC<3>{}, IC<5>{}, IC<7>{}, std::true_type{});
-          if constexpr (RES) res_write();
-          asm volatile("" ::: "memory");
-          group(IC<3>{}, IC<5>{}, IC<3>{}, IC<7>{}, std::false_type{});
-          asm volatile("" ::: "memory");
-          group(IC<5>{}, IC<7>{}, IC<5>{}, IC<7>{}, std::false_type{});
+          pass(IC<1>{});
         }
       }
     }
