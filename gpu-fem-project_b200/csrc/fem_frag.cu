@@ -67,9 +67,11 @@
 
 // Resident CTAs per SM the register budget is sized for: 3 (168 registers) at
 // p = 3, where the 12 live stiffness accumulators need them, and at p = 4; 4 (128)
-// at p = 2 and for the residual alone (no stiffness accumulators).
+// at p = 2.  The residual alone, without stiffness accumulators: 6 (85 registers) at
+// p = 2, 3 (800 x 512 p = 2: 175 / 159 / 152 us with 4 / 5 / 6; 600 x 590 p = 3: 172 / 162 /
+// 160 us), 4 at p = 4 (256^2: 102 / 107 / 115 us).
 #ifndef FEM_FRAG_MINB
-#define FEM_FRAG_MINB ((P == 2 || (MODE & kJac) == 0) ? 4 : 3)
+#define FEM_FRAG_MINB ((MODE & kJac) == 0 ? (P == 4 ? 4 : 6) : P == 2 ? 4 : 3)
 #endif
 
 namespace fem {
@@ -115,18 +117,20 @@ struct FragLayout {
   static constexpr size_t tabJ = 0;                          // double2 [K4][QT][32]
   static constexpr size_t tabF = tabJ + 16 * K4 * F::QT * 32;  // double2 [K4][NTM][32]
   static constexpr size_t tabX = tabF + 16 * K4 * F::NTM * 32;  // double2 [NQP]: dN of the node outside the tiles
-  static constexpr size_t wq = tabX + (F::EX ? 16 * NQP : 0);  // double [NQP]
-  static constexpr size_t csum = align16(wq + 8 * NQP);       // double2 [NQP]: sum_a dN(a, q)
-  static constexpr size_t tabB = align16(csum + 16 * NQP);    // double2 [8][32]: BF16x6 stiffness operands
+  static constexpr int NQT = 8 * F::QT;                       // points of the J stage's tiles
+  static constexpr size_t wq = tabX + (F::EX ? 16 * NQP : 0);  // double [NQT]
+  static constexpr size_t csum = align16(wq + 8 * NQT);       // double2 [NQT]: sum_a dN(a, q)
+  static constexpr size_t tabB = align16(csum + 16 * NQT);    // double2 [8][32]: BF16x6 stiffness operands
   static constexpr size_t tabR = align16(tabB + (B16 ? 16 * 8 * 32 : 0));  // uint32 [64]: runs (order 3)
   static constexpr size_t warps = align16(tabR + (P == 3 ? 4 * 64 : 0));
   // warp-relative; [2] = the two elements of the step, point q at slot(q) of PS
+  // (residual alone: s sigma J^-T, rows x and y, in WI0 and WI1, and no more)
   static constexpr size_t WI0 = 0;                  // double2 [2][PS]: sqrt|s| (J^-1_0x, J^-1_1x)
   static constexpr size_t WI1 = WI0 + 16 * 2 * PS;  // double2 [2][PS]: sqrt|s| (J^-1_0y, J^-1_1y)
   static constexpr size_t WS0 = WI1 + 16 * 2 * PS;  // double2 [2][PS]: (S-hat_xx, S-hat_xy)
-  static constexpr size_t WS1 = WS0 + 16 * 2 * PS;  // double2 [2][PS]: (S-hat_xy, S-hat_yy)
-  static constexpr size_t SG = WS1 + 16 * 2 * PS;   // double [2][NQP]: sign of s (0 on padding)
-  static constexpr size_t MC = align16(SG + 8 * 2 * NQP);  // double2: the mesh's (+-sqrt|t| or |t mu|, lam / mu)
+  static constexpr size_t WS1 = WS0 + (JAC ? 16 * 2 * PS : 0);  // double2 [2][PS]: (S-hat_xy, S-hat_yy)
+  static constexpr size_t SG = WS1 + (JAC ? 16 * 2 * PS : 0);   // double [2][NQP]: sign of s (0 on padding)
+  static constexpr size_t MC = align16(SG + (JAC ? 8 * 2 * NQP : 0));  // double2: the mesh's (+-sqrt|t| or |t mu|, lam / mu)
   static constexpr size_t NID = MC + 16;            // int [2][NN]: node ids
   static constexpr size_t RB = align16(NID + 4 * 2 * NN);  // int [2][NN]: rowp[node]
   static constexpr size_t STAGE = align16(RB + 4 * 2 * NN);  // [2 buffers][2 elements][CS] code records
@@ -136,7 +140,7 @@ struct FragLayout {
   static constexpr size_t REDS = align16(STAGE + 2 * 2 * CS);  // double4 [NSLOT][32]: bulk-reduction sources
   // NONLINEAR: sign(s) x tangent modulus, double [2][NQP][2 (l)][8 (i, k, n)]
   static constexpr size_t AT = align16(REDS + (JAC ? 32 * NSLOT * 32 : 0));
-  static constexpr size_t warp_bytes = align16(AT + (NL ? 8 * 2 * NQP * 16 : 0));
+  static constexpr size_t warp_bytes = align16(AT + (NL && JAC ? 8 * 2 * NQP * 16 : 0));
   static constexpr size_t total = warps + F::WARPS * warp_bytes;
 };
 
@@ -189,7 +193,8 @@ __device__ __forceinline__ uint32_t frag_run(int sl, int r) {
   return (uint32_t)(row * 16 + col0) | (uint32_t)(128 * sl + 4 * pos0) << 16;
 }
 
-template <int P, bool B16 = false, bool NL = false>
+// SQRTW: the square roots of the Gauss weights instead of the weights.
+template <int P, bool B16, bool SQRTW>
 __device__ __forceinline__ void frag_prologue(unsigned char *smem) {
   using F = FragDims<P>;
   using L = FragLayout<P, false, false, B16>;
@@ -220,10 +225,9 @@ __device__ __forceinline__ void frag_prologue(unsigned char *smem) {
     double2 *tabX = reinterpret_cast<double2 *>(smem + L::tabX);
     for (int q = threadIdx.x; q < F::NQP; q += blockDim.x) tabX[q] = q < NQ ? dN(NN - 1, q) : make_double2(0.0, 0.0);
   }
-  // Gauss weights (NONLINEAR), their square roots (LINEAR)
-  for (int q = threadIdx.x; q < F::NQP; q += blockDim.x) {
+  for (int q = threadIdx.x; q < L::NQT; q += blockDim.x) {
     const double w = q < NQ ? __dmul_rn(kGW[P][q % P1], kGW[P][q / P1]) : 0.0;
-    wq[q] = NL ? w : sqrt(w);
+    wq[q] = SQRTW ? sqrt(w) : w;
   }
   // BF16x6 stiffness (order 3): entry (2k + h, lane (g, t)) holds dN(a, q) for the
   // node a = 8h + pi(g) and quadrature point q = 2t + (k & 1) + 8 (k >> 1) that lane
@@ -245,7 +249,7 @@ __device__ __forceinline__ void frag_prologue(unsigned char *smem) {
   // table entries written above instead of evaluating the basis again
   __syncthreads();
   double2 *csum = reinterpret_cast<double2 *>(smem + L::csum);
-  for (int q = threadIdx.x; q < F::NQP; q += blockDim.x) {
+  for (int q = threadIdx.x; q < L::NQT; q += blockDim.x) {
     double s0 = 0.0, c0 = 0.0, s1 = 0.0, c1 = 0.0;
     if (q < NQ) {
       for (int a = 0; a < NN; a++) {
@@ -284,12 +288,11 @@ __device__ __forceinline__ uint32_t frag_put(const Out &O, int el, int a, int b,
     double *blk = O.mat + 4 * ((int64_t)O.rbase[el * NN + r0] + (code & 0x7f));
     asm volatile("{\n\t.reg .pred f, s;\n\t"
                  "setp.ne.u32 f, %6, 0;\n\t"
-                 "setp.eq.and.u32 s, %7, 0, f;\n\t"
-                 "setp.ne.and.u32 f, %7, 0, f;\n\t"
+                 "setp.ne.u32 s, %7, 0;\n\t"
                  "@f st.global.v4.f64 [%0], {%2, %3, %4, %5};\n\t"
                  "@s st.shared.v2.f64 [%1], {%2, %3};\n\t"
                  "@s st.shared.v2.f64 [%1 + 16], {%4, %5};\n\t}" ::"l"(blk),
-                 "r"(sa), "d"(v0), "d"(v1), "d"(v2), "d"(v3), "r"((uint32_t)act), "r"(code & m80)
+                 "r"(sa), "d"(v0), "d"(v1), "d"(v2), "d"(v3), "r"(act ? code & m80 : 0u), "r"((uint32_t)(act && !(code & m80)))
                  : "memory");
     return act ? code : 0x80u;
   } else {
@@ -338,12 +341,11 @@ __device__ __forceinline__ void pair_order_fence() {
 __device__ __forceinline__ void residual_put(double *dst, bool act, bool first, double x, double y) {
   asm volatile("{\n\t.reg .pred f, s;\n\t"
                "setp.ne.u32 f, %3, 0;\n\t"
-               "setp.eq.and.u32 s, %4, 0, f;\n\t"
-               "setp.ne.and.u32 f, %4, 0, f;\n\t"
+               "setp.ne.u32 s, %4, 0;\n\t"
                "@f st.global.v2.f64 [%0], {%1, %2};\n\t"
                "@s red.global.add.f64 [%0], %1;\n\t"
                "@s red.global.add.f64 [%0 + 8], %2;\n\t}" ::"l"(dst),
-               "d"(x), "d"(y), "r"((uint32_t)act), "r"((uint32_t)first)
+               "d"(x), "d"(y), "r"((uint32_t)(act && first)), "r"((uint32_t)(act && !first))
                : "memory");
 }
 
@@ -758,38 +760,44 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
     }
   };
   // node ids (two pairs ahead) and coordinate/state values (one pair ahead)
-  int nodeA[K4], nodeB[K4], rbB[K4];
-  double valB[K4];
+  int nodeA[K4] = {}, nodeB[K4] = {}, rbB[K4] = {};
+  double valB[K4] = {};
+  // Lanes past the element's nodes or the pair's elements read the last ones again: their
+  // values meet zero table entries, their ids are not kept.
   auto load_nodes = [&](const PairCursor &c, int *node) {
+    if (c.ne <= 0) return;
+    const int64_t k = c.k0 + (c.ne > 1 ? e_ld : 0);
+    const int *src;
+    if constexpr (PLAN) src = args(c).connList + k * NN;
+    else src = args(c).conn + __ldg(args(c).connPtr + k);
 #pragma unroll
-    for (int ks = 0; ks < K4; ks++) {
-      const int a = 4 * ks + t;
-      if constexpr (PLAN) {
-        node[ks] = (e_ld < c.ne && a < NN) ? __ldg(args(c).connList + (c.k0 + e_ld) * NN + a) : -1;
-      } else {
-        node[ks] = (e_ld < c.ne && a < NN) ? __ldg(args(c).conn + __ldg(args(c).connPtr + c.k0 + e_ld) + a) : -1;
-      }
-    }
+    for (int ks = 0; ks < K4; ks++) node[ks] = __ldg(src + (4 * ks + 3 < NN ? 4 * ks + t : min(4 * ks + t, NN - 1)));
   };
   auto load_values = [&](const PairCursor &c, const int *node, double *val, int *rbv) {
+    if (c.ne <= 0) return;
+    const AsmArgs &M = args(c);
+    const double *src = (c_ld < 2 ? M.coords : M.states) + (c_ld & 1);
 #pragma unroll
     for (int ks = 0; ks < K4; ks++) {
-      val[ks] = 0.0;
-      rbv[ks] = 0;
-      if (node[ks] >= 0) {
-        const AsmArgs &M = args(c);
-        const double *src = c_ld < 2 ? M.coords : M.states;
-        val[ks] = __ldg(src + 2 * (int64_t)node[ks] + (c_ld & 1));
-        if (PLAN && JAC) rbv[ks] = __ldg(M.rowp + node[ks]);
-      }
+      val[ks] = __ldg(src + 2 * (int64_t)node[ks]);
+      if (PLAN && JAC) rbv[ks] = __ldg(M.rowp + node[ks]);
     }
   };
   auto stage_codes = [&](const PairCursor &c, int buf) {
     if (c.ne > 0) {
       unsigned char *dst = stage + buf * 2 * STG;
-      if constexpr (PLAN) {
+      if constexpr (PLAN && JAC) {
         const unsigned char *src = args(c).blockCode + c.k0 * CS;
-        for (int i = lane; i < c.ne * CS / 16; i += 32) cp_async16(dst + 16 * i, src + 16 * i);
+#pragma unroll
+        for (int i0 = 0; i0 < 2 * CS / 16; i0 += 32) {
+          const int i = i0 + lane;
+          if (i < c.ne * CS / 16) cp_async16(dst + 16 * i, src + 16 * i);
+        }
+      } else if constexpr (PLAN) {
+        // the first-writer bytes of the residual rows alone
+        constexpr int B0 = NN * NN / 16, NB = (NN * NN + NN - 1) / 16 - B0 + 1;
+        const int e = lane / NB, i = B0 + lane - e * NB;
+        if (e < c.ne) cp_async16(dst + e * CS + 16 * i, args(c).blockCode + (c.k0 + e) * CS + 16 * i);
       } else if constexpr (JAC) {
         // element map rows: 16-byte copies when a row set is a multiple of 16 bytes
         const int *src = args(c).map + c.k0 * NN * NN;
@@ -814,6 +822,10 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
       __syncwarp();
     }
   };
+  if constexpr (NL && JAC && NQP > NQ) {  // the padded points' tangents: zero
+    for (int i = lane; i < 2 * (NQP - NQ) * 16; i += 32)
+      ATs[(i / ((NQP - NQ) * 16) * NQP + NQ) * 16 + i % ((NQP - NQ) * 16)] = 0.0;
+  }
   int meshC = -1;
   // a grid launched after this one with programmatic serialization may start its CTAs
   // as this one's retire; it waits (griddepcontrol.wait) before it writes
@@ -843,7 +855,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
       val[ks] = valB[ks];
       const int a = 4 * ks + t;
       // nid by the lanes of component 0, rb by those of component 1
-      if (nodeB[ks] >= 0 && c_ld < (PLAN && JAC ? 2 : 1))
+      if ((4 * ks + 3 < NN || a < NN) && c_ld < (PLAN && JAC ? 2 : 1))
         (c_ld == 0 ? nid : rb)[e_ld * NN + a] = c_ld == 0 ? nodeB[ks] : rbB[ks];
     }
     cp_async_wait_all();
@@ -901,96 +913,110 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
           um[d][c] = odd ? hi : r;
         }
       const int q = 16 * m + 8 * odd + g;
-      const bool valid = e_q < ne && q < NQ;
       const int o = e_q * PS + L::slot(q);
-      double2 wi0 = make_double2(0, 0), wi1 = make_double2(0, 0), ws0 = make_double2(0, 0), ws1 = make_double2(0, 0);
-      double sg = 0.0;
-      bool ng = false;
-      if (valid) {
-        const double2 cs = csum[q];
-        const double j00 = fma(xq, cs.x, jm[0][0]), j01 = fma(xq, cs.y, jm[1][0]);
-        const double j10 = fma(yq, cs.x, jm[0][1]), j11 = fma(yq, cs.y, jm[1][1]);
-        const double g00 = um[0][0], g01 = um[1][0], g10 = um[0][1], g11 = um[1][1];
-        const double det = j00 * j11 - j01 * j10;
+      const bool in = 8 * F::QT == NQ || q < NQ;  // a point of the rule: the others store zeros
+      const double2 cs = csum[q];
+      const double j00 = fma(xq, cs.x, jm[0][0]), j01 = fma(xq, cs.y, jm[1][0]);
+      const double j10 = fma(yq, cs.x, jm[0][1]), j11 = fma(yq, cs.y, jm[1][1]);
+      const double g00 = um[0][0], g01 = um[1][0], g10 = um[0][1], g11 = um[1][1];
+      const double det = j00 * j11 - j01 * j10;
+      const bool keep = q < NQP;  // the point has a slot
+      if constexpr (!JAC) {
+        // residual alone: R_(a,i) = sum_q sum_d T_id dN_d(a, q) with T = s sigma J^-T, so
+        // the nodal gradients are not formed: w t sigma adj(J)^T
+        const double inv = in ? 1.0 / det : 0.0;
+        const double ux0 = (g00 * j11 - g01 * j10) * inv, ux1 = (g01 * j00 - g00 * j01) * inv;
+        const double uy0 = (g10 * j11 - g11 * j10) * inv, uy1 = (g11 * j00 - g10 * j01) * inv;
+        double pxx, pxy, pyx, pyy;
         if constexpr (NL) {
-          const double inv = 1.0 / det;
-          const double i00 = j11 * inv, i01 = -j01 * inv, i10 = -j10 * inv, i11 = j00 * inv;
-          const double st = wqs[q] * det * M.t;
-          const double rs = sqrt(fabs(st));
-          sg = st < 0.0 ? -1.0 : 1.0;
-          const double sw = sg * rs;
-          const double uxx = g00 * i00 + g01 * i10, uxy = g00 * i01 + g01 * i11;
-          const double uyx = g10 * i00 + g11 * i10, uyy = g10 * i01 + g11 * i11;
-          wi0 = make_double2(rs * i00, rs * i10);
-          wi1 = make_double2(rs * i01, rs * i11);
-          // Green strain E = 1/2 (g + g^T + g^T g), S = 2 mu E + lam tr(E) I, first Piola
-          // P = F S (F = I + g); tangent A_{il,kn} = delta_ik S_ln + mu F_in F_kl
-          // + mu (F F^T)_ik delta_ln + lam F_il F_kn (element/FEKernels.h:286-315,
-          // NONLINEAR), stored times sign(s) as [l][i][k][n]
-          const double F[2][2] = {{1.0 + uxx, uxy}, {uyx, 1.0 + uyy}};
-          const double e00 = 0.5 * (2.0 * uxx + uxx * uxx + uyx * uyx);
-          const double e01 = 0.5 * (uxy + uyx + uxx * uxy + uyx * uyy);
-          const double e11 = 0.5 * (2.0 * uyy + uxy * uxy + uyy * uyy);
-          const double trE = e00 + e11;
-          const double Sm[2][2] = {{2.0 * mu * e00 + lam * trE, 2.0 * mu * e01}, {2.0 * mu * e01, 2.0 * mu * e11 + lam * trE}};
-          const double pxx = F[0][0] * Sm[0][0] + F[0][1] * Sm[1][0], pxy = F[0][0] * Sm[0][1] + F[0][1] * Sm[1][1];
-          const double pyx = F[1][0] * Sm[0][0] + F[1][1] * Sm[1][0], pyy = F[1][0] * Sm[0][1] + F[1][1] * Sm[1][1];
-          ws0 = make_double2(sw * pxx, sw * pyx);  // (P-hat_x0, P-hat_y0)
-          ws1 = make_double2(sw * pxy, sw * pyy);  // (P-hat_x1, P-hat_y1)
-          if constexpr (JAC) {
-            double *at = ATs + (e_q * NQP + q) * 16;
-#pragma unroll
-            for (int ll = 0; ll < 2; ll++)
-#pragma unroll
-              for (int ii2 = 0; ii2 < 2; ii2++)
-#pragma unroll
-                for (int kk = 0; kk < 2; kk++) {
-                  double v2[2];
-#pragma unroll
-                  for (int nn = 0; nn < 2; nn++) {
-                    const double bik = F[ii2][0] * F[kk][0] + F[ii2][1] * F[kk][1];
-                    double v = mu * F[ii2][nn] * F[kk][ll] + lam * F[ii2][ll] * F[kk][nn];
-                    if (ii2 == kk) v += Sm[ll][nn];
-                    if (ll == nn) v += mu * bik;
-                    v2[nn] = sg * v;
-                  }
-                  *reinterpret_cast<double2 *>(at + ll * 8 + ii2 * 4 + kk * 2) = make_double2(v2[0], v2[1]);
-                }
-          }
+          const double F[2][2] = {{1.0 + ux0, ux1}, {uy0, 1.0 + uy1}};
+          const double e00 = 0.5 * (2.0 * ux0 + ux0 * ux0 + uy0 * uy0);
+          const double e01 = 0.5 * (ux1 + uy0 + ux0 * ux1 + uy0 * uy1);
+          const double e11 = 0.5 * (2.0 * uy1 + ux1 * ux1 + uy1 * uy1);
+          const double tr = lam * (e00 + e11), s00 = 2.0 * mu * e00 + tr, s01 = 2.0 * mu * e01, s11 = 2.0 * mu * e11 + tr;
+          pxx = F[0][0] * s00 + F[0][1] * s01, pxy = F[0][0] * s01 + F[0][1] * s11;
+          pyx = F[1][0] * s00 + F[1][1] * s01, pyy = F[1][0] * s01 + F[1][1] * s11;
         } else {
-          // s = w det t, J^-1 = adj(J) / det: sqrt|s| J^-1 = +-c adj(J) with
-          // c = sqrt|w t| / sqrt|det| (the sign leaves every product of two gradients
-          // alone), grad u = g adj(J) / det, and s sigma G = (+-c sigma(g adj(J))) (c adj(J) dN):
-          // one reciprocal square root instead of a division and a square root.
-          // A singular point (det = 0) gives NaN.
-          const double2 mc = make_double2(MC->x, MC->y);
-          const double r = det != 0.0 ? rsqrt(fabs(det)) : __longlong_as_double(0x7ff8000000000000LL);
-          const double c = wqs[q] * fabs(mc.x) * r;
-          ng = (det < 0.0) != (mc.x < 0.0);
-          sg = ng ? -1.0 : 1.0;
-          const double cw = sg * c;
-          const double uxx = g00 * j11 - g01 * j10, uxy = g01 * j00 - g00 * j01;
-          const double uyx = g10 * j11 - g11 * j10, uyy = g11 * j00 - g10 * j01;
-          wi0 = make_double2(c * j11, -(c * j10));
-          wi1 = make_double2(-(c * j01), c * j00);
-          const double m1 = SCALED ? 1.0 : mu, lt = (SCALED ? mc.y : lam) * (uxx + uyy);
-          const double sxy = cw * (m1 * (uxy + uyx));
-          ws0 = make_double2(cw * fma(2.0 * m1, uxx, lt), sxy);
-          ws1 = make_double2(sxy, cw * fma(2.0 * m1, uyy, lt));
+          const double tr = lam * (ux0 + uy1);
+          pxx = 2.0 * mu * ux0 + tr, pyy = 2.0 * mu * uy1 + tr;
+          pxy = pyx = mu * (ux1 + uy0);
         }
-      } else if (NL && JAC && q < NQP) {
-        double2 *at = reinterpret_cast<double2 *>(ATs + (e_q * NQP + q) * 16);
+        const double wt = wqs[q] * M.t;
+        if (keep) {
+          WI0[o] = make_double2(wt * (pxx * j11 - pxy * j01), wt * (pxy * j00 - pxx * j10));
+          WI1[o] = make_double2(wt * (pyx * j11 - pyy * j01), wt * (pyy * j00 - pyx * j10));
+        }
+      } else if constexpr (NL) {
+        const double inv = in ? 1.0 / det : 0.0;
+        const double i00 = j11 * inv, i01 = -j01 * inv, i10 = -j10 * inv, i11 = j00 * inv;
+        const double st = wqs[q] * det * M.t;
+        const double rs = sqrt(fabs(st));
+        const double sg = st < 0.0 ? -1.0 : 1.0;
+        const double sw = sg * rs;
+        const double uxx = g00 * i00 + g01 * i10, uxy = g00 * i01 + g01 * i11;
+        const double uyx = g10 * i00 + g11 * i10, uyy = g10 * i01 + g11 * i11;
+        // Green strain E = 1/2 (g + g^T + g^T g), S = 2 mu E + lam tr(E) I, first Piola
+        // P = F S (F = I + g); tangent A_{il,kn} = delta_ik S_ln + mu F_in F_kl
+        // + mu (F F^T)_ik delta_ln + lam F_il F_kn (element/FEKernels.h:286-315,
+        // NONLINEAR), stored times sign(s) as [l][i][k][n]
+        const double F[2][2] = {{1.0 + uxx, uxy}, {uyx, 1.0 + uyy}};
+        const double e00 = 0.5 * (2.0 * uxx + uxx * uxx + uyx * uyx);
+        const double e01 = 0.5 * (uxy + uyx + uxx * uxy + uyx * uyy);
+        const double e11 = 0.5 * (2.0 * uyy + uxy * uxy + uyy * uyy);
+        const double trE = e00 + e11;
+        const double Sm[2][2] = {{2.0 * mu * e00 + lam * trE, 2.0 * mu * e01}, {2.0 * mu * e01, 2.0 * mu * e11 + lam * trE}};
+        if (keep) {
+          WI0[o] = make_double2(rs * i00, rs * i10);
+          WI1[o] = make_double2(rs * i01, rs * i11);
+          // (P-hat_x0, P-hat_y0), (P-hat_x1, P-hat_y1)
+          WS0[o] = make_double2(sw * (F[0][0] * Sm[0][0] + F[0][1] * Sm[1][0]), sw * (F[1][0] * Sm[0][0] + F[1][1] * Sm[1][0]));
+          WS1[o] = make_double2(sw * (F[0][0] * Sm[0][1] + F[0][1] * Sm[1][1]), sw * (F[1][0] * Sm[0][1] + F[1][1] * Sm[1][1]));
+          double *at = ATs + (e_q * NQP + q) * 16;
+          if (in) {
 #pragma unroll
-        for (int j = 0; j < 8; j++) at[j] = make_double2(0.0, 0.0);
+          for (int ll = 0; ll < 2; ll++)
+#pragma unroll
+            for (int ii2 = 0; ii2 < 2; ii2++)
+#pragma unroll
+              for (int kk = 0; kk < 2; kk++) {
+                double v2[2];
+#pragma unroll
+                for (int nn = 0; nn < 2; nn++) {
+                  const double bik = F[ii2][0] * F[kk][0] + F[ii2][1] * F[kk][1];
+                  double v = mu * F[ii2][nn] * F[kk][ll] + lam * F[ii2][ll] * F[kk][nn];
+                  if (ii2 == kk) v += Sm[ll][nn];
+                  if (ll == nn) v += mu * bik;
+                  v2[nn] = sg * v;
+                }
+                *reinterpret_cast<double2 *>(at + ll * 8 + ii2 * 4 + kk * 2) = make_double2(v2[0], v2[1]);
+              }
+          }
+        }
+      } else {
+        // s = w det t, J^-1 = adj(J) / det: sqrt|s| J^-1 = +-c adj(J) with
+        // c = sqrt|w t| / sqrt|det| (the sign leaves every product of two gradients
+        // alone), grad u = g adj(J) / det, and s sigma G = (+-c sigma(g adj(J))) (c adj(J) dN):
+        // one reciprocal square root instead of a division and a square root.
+        // A singular point (det = 0) gives NaN.
+        const double2 mc = make_double2(MC->x, MC->y);
+        const double r = det != 0.0 ? rsqrt(fabs(det)) : __longlong_as_double(0x7ff8000000000000LL);
+        const double c = in ? wqs[q] * fabs(mc.x) * r : 0.0;
+        const bool ng = in && e_q < ne && (det < 0.0) != (mc.x < 0.0);
+        const double sg = ng ? -1.0 : 1.0;
+        const double cw = sg * c;
+        const double uxx = g00 * j11 - g01 * j10, uxy = g01 * j00 - g00 * j01;
+        const double uyx = g10 * j11 - g11 * j10, uyy = g11 * j00 - g10 * j01;
+        const double m1 = SCALED ? 1.0 : mu, lt = (SCALED ? mc.y : lam) * (uxx + uyy);
+        const double sxy = cw * (m1 * (uxy + uyx));
+        if (keep) {
+          WI0[o] = make_double2(c * j11, -(c * j10));
+          WI1[o] = make_double2(-(c * j01), c * j00);
+          WS0[o] = make_double2(cw * fma(2.0 * m1, uxx, lt), sxy);
+          WS1[o] = make_double2(sxy, cw * fma(2.0 * m1, uyy, lt));
+          SGs[e_q * NQP + q] = sg;
+        }
+        if constexpr (SCALED) negm |= __ballot_sync(0xffffffffu, ng);
       }
-      if (q < NQP) {
-        WI0[o] = wi0;
-        WI1[o] = wi1;
-        WS0[o] = ws0;
-        WS1[o] = ws1;
-        if constexpr (!NL) SGs[e_q * NQP + q] = sg;
-      }
-      if constexpr (SCALED) negm |= __ballot_sync(0xffffffffu, ng);
     }
     __syncwarp();
 
@@ -1048,7 +1074,71 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
       crx = __shfl_down_sync(0xffffffffu, sx, 24);
       cry = __shfl_down_sync(0xffffffffu, sy, 24);
     };
-    {
+    if constexpr (!JAC) {
+      // residual alone: rows (element, component) m = g%4 (twice), columns the nodes of a
+      // tile, k = points: R_(a,i) = sum_(q,d) T_id(q) dN_d(a, q); the node outside the tiles
+      // on the FP64 pipe.  Forming the nodal gradients first, as the Jacobian does, took
+      // 8 shared loads and 16 FMAs per k-step and element instead of this pair's 3 loads
+      // and 4 MMAs (order 3; residual 600 x 590 order 3 248 -> 160 us, 800 x 512 order
+      // 2 239 -> 152, 256^2 order 4 170 -> 102).
+      const double2 *Ts = ((g & 1) ? WI1 : WI0) + ((g >> 1) & 1) * PS;
+      double c[NTM][2], xr = 0.0;
+#pragma unroll
+      for (int ks = 0; ks < K4; ks++) {
+        const double2 tv = Ts[L::slot(4 * ks) + t];
+#pragma unroll
+        for (int T = 0; T < NTM; T++) {
+          const double2 d = tabF[(ks * NTM + T) * 32 + lane];
+          if (ks == 0) dmma_first(c[T][0], c[T][1], tv.x, d.x);
+          else dmma(c[T][0], c[T][1], tv.x, d.x);
+          dmma(c[T][0], c[T][1], tv.y, d.y);
+        }
+        if constexpr (EX) {
+          const double2 d = tabX[4 * ks + t];
+          xr = fma(tv.x, d.x, fma(tv.y, d.y, xr));
+        }
+      }
+      // lane (g, t) holds component i = g%2 of nodes 8T + t, 8T + 4 + t; lanes g, g^1 swap,
+      // and each keeps node 8T + 4i + t; the copies g >= 4 take the odd tiles (the last
+      // one of orders 2 and 4: node XN)
+      const int i = g & 1, e = (g >> 1) & 1, up = g >> 2;
+      if constexpr (EX) {
+        xr += __shfl_xor_sync(0xffffffffu, xr, 1);
+        xr += __shfl_xor_sync(0xffffffffu, xr, 2);
+      }
+      constexpr int NR = (NTM + (EX ? 1 : 0) + 1) / 2;
+      double sx[NR], sy[NR];
+      double *dst[NR];
+      bool act[NR], first[NR];
+#pragma unroll
+      for (int x = 0; x < NR; x++) {
+        const int T = 2 * x;
+        double v0 = c[T][0], v1 = c[T][1];
+        if (up) {
+          v0 = T + 1 < NTM ? c[T + 1 < NTM ? T + 1 : T][0] : xr;
+          v1 = T + 1 < NTM ? c[T + 1 < NTM ? T + 1 : T][1] : xr;
+        }
+        const double r = __shfl_xor_sync(0xffffffffu, i ? v0 : v1, 4);
+        sx[x] = i ? r : v0;
+        sy[x] = i ? v1 : r;
+        const bool xl = EX && T + 1 == NTM && up;
+        const int a = xl ? XN : 8 * (T + up) + 4 * i + t;
+        act[x] = e < ne && (!xl || (i == 0 && t == 0));
+        dst[x] = M.residual + 2 * (int64_t)nid[e * NN + a];
+        first[x] = PLAN && O.codes[e * CS + NN * NN + a];
+      }
+      if constexpr (PLAN) {
+        // pair layout: the first element's rows before the second's
+#pragma unroll
+        for (int x = 0; x < NR; x++) residual_put(dst[x], act[x] && e == 0, first[x], sx[x], sy[x]);
+        __syncwarp();
+#pragma unroll
+        for (int x = 0; x < NR; x++) residual_put(dst[x], act[x] && e == 1, first[x], sx[x], sy[x]);
+      } else {
+#pragma unroll
+        for (int x = 0; x < NR; x++) residual_put(dst[x], act[x], false, sx[x], sy[x]);
+      }
+    } else {
       const int pa = 4 * (g & 1) + (g >> 1);  // pi(g)
       int half = 0;  // orders 2 and 4: half of the lane's staging slots the next blocks use
       for (int el = 0; el < ne; el++) {
@@ -1189,7 +1279,14 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
                       kyx += cs[2], kyy += cs[3];
                     }
                     if constexpr (STRIP) __syncwarp();
-                    allfirst &= frag_put<P, PLAN>(O, el, a, b, 0, true, m80, kxx, kxy, kyx, kyy, stg);
+                    if constexpr (PLAN) {
+                      const uint32_t code = O.codes[el * CS + a * NN + b];
+                      frag_put_row<0>(O.mat + 4 * (int64_t)O.rbase[el * NN + a], code, m80,
+                                      (unsigned)__cvta_generic_to_shared(stg), kxx, kxy, kyx, kyy);
+                      allfirst &= code;
+                    } else {
+                      allfirst &= frag_put<P, PLAN>(O, el, a, b, 0, true, m80, kxx, kxy, kyx, kyy, stg);
+                    }
                   }
                 }
             issue_runs(O, el, !halo && (allfirst & 0x80u) == 0);
@@ -1213,8 +1310,8 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
         [[maybe_unused]] constexpr int RT0 = PASS ? 2 : 0, RT1 = PASS || NTM == 1 ? NTM : 1;
         constexpr bool XD = EX && RT1 == NTM;  // this pass has XN's own row
         double acc[NPAIR][4][2];
-        double rp[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-        double xs[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
+        [[maybe_unused]] double rp[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+        [[maybe_unused]] double xs[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
         auto kstep = [&](int ks, auto firstc, auto negc) {
           constexpr bool FIRST = decltype(firstc)::value, NEG = decltype(negc)::value;
           const int o = el * PS + L::slot(4 * ks) + t;
@@ -1226,7 +1323,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
             fr[T][0] = fma(w0.x, d.x, w0.y * d.y);
             fr[T][1] = fma(w1.x, d.x, w1.y * d.y);
           }
-          double h0 = 0.0, h1 = 0.0;  // G-hat(q, XN)
+          [[maybe_unused]] double h0 = 0.0, h1 = 0.0;  // G-hat(q, XN)
           if constexpr (EX && (JAC || XD)) {
             const double2 d = tabX[4 * ks + t];
             h0 = fma(w0.x, d.x, w0.y * d.y);
@@ -1308,7 +1405,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
         };
         kstep_all(kstep, neg);
         // residual: sum over the four lanes t of a node (reduce-scatter over the two slots)
-        const int Tm = t >> 1, To = Tm ^ 1;
+        [[maybe_unused]] const int Tm = t >> 1, To = Tm ^ 1;
         if constexpr (RES) {
           double sx = (Tm ? rp[1][0] : rp[0][0]) + __shfl_xor_sync(0xffffffffu, To ? rp[1][0] : rp[0][0], 2);
           double sy = (Tm ? rp[1][1] : rp[0][1]) + __shfl_xor_sync(0xffffffffu, To ? rp[1][1] : rp[0][1], 2);
@@ -1499,7 +1596,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
 template <int P, int MODE>
 __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB) frag_kernel(const __grid_constant__ AsmArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
-  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) != 0>(smem);
+  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) == 0 && (MODE & kJac) != 0>(smem);
   const int warp = threadIdx.x >> 5;
   PairStride gen{A.begin, A.begin + A.count, (int64_t)blockIdx.x * FragDims<P>::WARPS + warp,
                  (int64_t)gridDim.x * FragDims<P>::WARPS};
@@ -1511,7 +1608,7 @@ template <int P, int MODE>
 __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB)
     frag_ranges_kernel(const __grid_constant__ AsmArgs A, const RangeList R) {
   extern __shared__ __align__(16) unsigned char smem[];
-  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) != 0>(smem);
+  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) == 0 && (MODE & kJac) != 0>(smem);
   const int warp = threadIdx.x >> 5;
   PairRanges gen{R, (int64_t)blockIdx.x * FragDims<P>::WARPS + warp, (int64_t)gridDim.x * FragDims<P>::WARPS};
   frag_loop<P, MODE>(smem, gen, A, &A);
@@ -1527,7 +1624,7 @@ __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB)
     frag_strip_kernel(const __grid_constant__ AsmArgs A, const __grid_constant__ RangeList R,
                       const Strip *__restrict__ strips) {
   extern __shared__ __align__(16) unsigned char smem[];
-  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) != 0>(smem);
+  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) == 0 && (MODE & kJac) != 0>(smem);
   const int warp = threadIdx.x >> 5;
   StripRanges gen{strips, R, (int64_t)blockIdx.x * FragDims<P>::WARPS + warp, (int64_t)gridDim.x * FragDims<P>::WARPS};
   gen.fetch();
@@ -1539,7 +1636,7 @@ template <int P, int MODE>
 __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB)
     frag_sched_kernel(const __grid_constant__ AsmArgs A, const __grid_constant__ SchedArgs S) {
   extern __shared__ __align__(16) unsigned char smem[];
-  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) != 0>(smem);
+  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) == 0 && (MODE & kJac) != 0>(smem);
   PairSched gen{&S};
   frag_loop<P, MODE>(smem, gen, A, &A);
 }
@@ -1551,7 +1648,7 @@ template <int P, int MODE>
 __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB)
     frag_batched_sched_kernel(const AsmArgs *__restrict__ meshes, const __grid_constant__ SchedArgs S) {
   extern __shared__ __align__(16) unsigned char smem[];
-  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) != 0>(smem);
+  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) == 0 && (MODE & kJac) != 0>(smem);
   PairSchedT<true> gen{&S};
   frag_loop<P, MODE>(smem, gen, meshes[0], meshes);
 }
@@ -1561,7 +1658,7 @@ template <int P, int MODE>
 __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB)
     frag_batched_kernel(const AsmArgs *__restrict__ meshes, const Tile *__restrict__ tiles, int ntiles, int *counter) {
   extern __shared__ __align__(16) unsigned char smem[];
-  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) != 0>(smem);
+  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) == 0 && (MODE & kJac) != 0>(smem);
   PairQueue gen{tiles, ntiles, counter, 0, 0, 0, false};
   frag_loop<P, MODE>(smem, gen, meshes[0], meshes);
 }
