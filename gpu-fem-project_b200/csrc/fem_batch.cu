@@ -168,6 +168,7 @@ struct fem_batch {
   bool args_dirty = true;
   int maxColours = 0;
   int tileBatches[kOrders] = {0, 16, 16, 16, 16};  // tile length in element batches, per order
+  int rowTileChunks = fem::kRowTileChunks;           // chunks per row tile
   int kernel[2][kOrders] = {};                       // [FP64, MIXED][order]: FEM_KERNEL_*
   std::vector<fem::dev::Tile> tiles;
   std::vector<int> tileOff;  // [kOrders][maxColours + 1]
@@ -224,6 +225,26 @@ void batch_free(fem_batch *b) {
 
 int order_of(const fem_batch *b, int m) { return b->plans[m]->order; }
 
+// Default tile lengths, by the elements n of a colour launch (about a quarter of the
+// order's): n / 2000 elements, 4 at least (a launch of few, long tiles leaves warps idle:
+// 12 meshes of 1e3-6e4 elements, 16 element batches per tile 826 us, 8 636, 4 611, 2 674, 1
+// 758; 20 of 1e3-8e3: 608 / - / 372 / 361 / 442; tiles of one pair ask for more CTAs, whose table setup
+// the other orders' launches wait for), 16 batches at most.  Row chunks likewise: one
+// tile per two resident warps' worth, 16 chunks at most.
+void default_tiles(fem_batch *b) {
+  int64_t elements[kOrders] = {}, chunks = 0;
+  for (const fem_plan *pl : b->plans) {
+    elements[pl->order] += pl->numElements;
+    chunks += pl->numChunks;
+  }
+  for (int p = 2; p < kOrders; p++) {
+    const int epg = fem::epg_of(p);
+    b->tileBatches[p] = (int)std::clamp<int64_t>(elements[p] / 4 / 2000 / epg, 4 / epg, 16);
+    if (epg == 1) b->tileBatches[p] &= ~1;  // whole pairs
+  }
+  b->rowTileChunks = (int)std::clamp<int64_t>(chunks / (2 * fem::kRowWarpsResident), 1, fem::kRowTileChunks);
+}
+
 // Colour tiles of every mesh (order-1 meshes with row tables last within each
 // colour, after rowSplit[c], so that row assembly can skip them) and the row
 // tiles of the order-1 meshes that have row tables.
@@ -257,11 +278,11 @@ void build_tiles(fem_batch *b) {
   for (size_t m = 0; m < b->plans.size(); m++) {
     const fem_plan *pl = b->plans[m];
     if (!fem::plan_rows(pl)) continue;
-    for (int k = 0; k < pl->numChunks; k += fem::kRowTileChunks) {
+    for (int k = 0; k < pl->numChunks; k += b->rowTileChunks) {
       fem::dev::Tile t;
       t.mesh = (int)m;
       t.begin = k;
-      t.count = std::min(fem::kRowTileChunks, pl->numChunks - k);
+      t.count = std::min(b->rowTileChunks, pl->numChunks - k);
       b->tiles.push_back(t);
     }
   }
@@ -497,6 +518,7 @@ int fem_batch_create(int numMeshes, fem_plan *const *plans, fem_batch **batch) {
     return st;
   }
   b->deviceBytes = (int64_t)(sizeof(fem::dev::AsmArgs) * numMeshes + sizeof(int) * kOrders * kMaxColours);
+  default_tiles(b);
   build_tiles(b);
   *batch = b;
   return FEM_SUCCESS;

@@ -488,7 +488,7 @@ struct StrideSource {
 
 // A tile of the batched work queue: `count` consecutive (colour-ordered) element
 // positions of mesh `mesh`, starting at `begin`.
-struct Tile {
+struct __align__(16) Tile {
   int mesh;
   int count;
   int64_t begin;

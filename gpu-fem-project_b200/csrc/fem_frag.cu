@@ -202,12 +202,20 @@ __device__ __forceinline__ void frag_prologue(unsigned char *smem) {
   double2 *tabJ = reinterpret_cast<double2 *>(smem + L::tabJ);
   double2 *tabF = reinterpret_cast<double2 *>(smem + L::tabF);
   double *wq = reinterpret_cast<double *>(smem + L::wq);
+  // the 1D basis at the 1D points, [point][node] (N, dN), in the first warp's region: a
+  // thread per entry, where evaluating it per 2D entry meant ten divergent constant loads
+  // and two polynomials each (a large part of a small launch's time)
+  double2 *b1 = reinterpret_cast<double2 *>(smem + L::warps);
+  for (int i = threadIdx.x; i < P1 * P1; i += blockDim.x) {
+    double N, dN1;
+    lag1d(P, kGX[P][i / P1], i % P1, N, dN1);
+    b1[i] = make_double2(N, dN1);
+  }
+  __syncthreads();
   // dN(a, q) = (N_y dN_x, N_x dN_y) with the rounding of the element kernel's table
   auto dN = [&](int a, int q) {
-    double Nx, dNx, Ny, dNy;
-    lag1d(P, kGX[P][q % P1], a % P1, Nx, dNx);
-    lag1d(P, kGX[P][q / P1], a / P1, Ny, dNy);
-    return make_double2(__dmul_rn(Ny, dNx), __dmul_rn(Nx, dNy));
+    const double2 x = b1[(q % P1) * P1 + a % P1], y = b1[(q / P1) * P1 + a / P1];
+    return make_double2(__dmul_rn(y.x, x.y), __dmul_rn(x.x, y.y));
   };
   // J-stage A fragments: lane (g, t) of (ks, tm) holds dN(a = 4ks + t, q = 8tm + g)
   for (int i = threadIdx.x; i < K4 * QT * 32; i += blockDim.x) {
@@ -252,6 +260,7 @@ __device__ __forceinline__ void frag_prologue(unsigned char *smem) {
   for (int q = threadIdx.x; q < L::NQT; q += blockDim.x) {
     double s0 = 0.0, c0 = 0.0, s1 = 0.0, c1 = 0.0;
     if (q < NQ) {
+#pragma unroll
       for (int a = 0; a < NN; a++) {
         const double2 d = tabJ[((a >> 2) * QT + (q >> 3)) * 32 + 4 * (q & 7) + (a & 3)];
         const double t0 = s0 + d.x, t1 = s1 + d.y;
@@ -558,43 +567,41 @@ struct StripRanges {
   }
 };
 
-// Many meshes: the pairs of the tiles this warp pulls from the launch's queue
-// (one atomic counter per launch; tiles hold even element counts except at the
-// end of a colour range, so pairs never straddle tiles).
+// Many meshes: the pairs of the warp's tiles -- tile w of the launch's list first, then
+// the ones it pulls from the launch's queue (one atomic counter per launch; tiles hold
+// even element counts except at the end of a colour range, so pairs never straddle
+// tiles).  A warp asks for its next tile when it hands out the last pair of the one it
+// has, no earlier: a small launch has about as many tiles as warps, and a warp that
+// holds tiles in advance (as every warp did, from its start) leaves others idle.
 struct PairQueue {
   static constexpr bool kBatched = true, kSched = false, kStrip = false;
   const Tile *tiles;
   int ntiles;
   int *counter;
-  int mesh;
-  int64_t pos, tend;
-  bool done;
-  // lane 0: the tile after the current one, taken one tile ahead so that the queue
-  // atomic's latency (long behind a later colour's reductions in L2) is hidden
-  int ahead = -1;
+  int warps;      // of the launch
+  int idx;        // lane 0: the next tile
+  int mesh = 0;
+  int64_t pos = 0, tend = 0;
+  bool done = false;
   __device__ PairCursor next(int lane) {
     PairCursor c{0, 0, 0};
-    while (!done && pos >= tend) {
-      int t = 0;
-      if (lane == 0) {
-        t = ahead < 0 ? atomicAdd(counter, 1) : ahead;
-        ahead = t < ntiles ? atomicAdd(counter, 1) : ntiles;
-      }
-      t = __shfl_sync(0xffffffffu, t, 0);
+    if (done) return c;
+    if (pos >= tend) {
+      const int t = __shfl_sync(0xffffffffu, idx, 0);
       if (t >= ntiles) {
         done = true;
-      } else {
-        const Tile tl = tiles[t];
-        mesh = tl.mesh;
-        pos = tl.begin;
-        tend = tl.begin + tl.count;
+        return c;
       }
+      const int4 tl = __ldg(reinterpret_cast<const int4 *>(tiles + t));  // mesh, count, begin
+      mesh = tl.x;
+      pos = ((int64_t)tl.w << 32) | (uint32_t)tl.z;
+      tend = pos + tl.y;
     }
-    if (done) return c;
     c.mesh = mesh;
     c.k0 = pos;
     c.ne = (int)min((int64_t)2, tend - pos);
     pos += 2;
+    if (pos >= tend && lane == 0) idx = warps + atomicAdd(counter, 1);
     return c;
   }
 };
@@ -1659,7 +1666,8 @@ __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB)
     frag_batched_kernel(const AsmArgs *__restrict__ meshes, const Tile *__restrict__ tiles, int ntiles, int *counter) {
   extern __shared__ __align__(16) unsigned char smem[];
   frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) == 0 && (MODE & kJac) != 0>(smem);
-  PairQueue gen{tiles, ntiles, counter, 0, 0, 0, false};
+  constexpr int W = FragDims<P>::WARPS;
+  PairQueue gen{tiles, ntiles, counter, (int)gridDim.x * W, (int)blockIdx.x * W + (int)(threadIdx.x >> 5)};
   frag_loop<P, MODE>(smem, gen, meshes[0], meshes);
 }
 

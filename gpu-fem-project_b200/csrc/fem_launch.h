@@ -109,8 +109,8 @@ int launch_batched(int p, int precision, const dev::AsmArgs *meshes, const dev::
 int launch_rows(int mode, const dev::AsmArgs &a, cudaStream_t s);
 int launch_rows_batched(const dev::AsmArgs *meshes, const dev::Tile *tiles, int ntiles, int *counter,
                         cudaStream_t s);
-// Chunks per row tile of the batched row kernel.
-constexpr int kRowTileChunks = 16;
+// Chunks per row tile of the batched row kernel (batches: at most), its resident warps.
+constexpr int kRowTileChunks = 16, kRowWarpsResident = 148 * 12;
 // Warp-fragment kernel (fem_frag.cu): LINEAR assembly at orders 2 to 4 and NONLINEAR
 // at orders 2 and 3 (frag_supported), plan mode (one colour, list positions
 // [a.begin, a.begin + a.count)) or drop-in mode (elements through the reference map,

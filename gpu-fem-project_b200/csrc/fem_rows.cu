@@ -261,18 +261,16 @@ __global__ void __launch_bounds__(32 * kRowWarps, 3) rows_p1_batched_kernel(cons
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double NP, NM;
   p1_basis(NP, NM);
-  int ahead = -1;  // lane 0: the next tile, taken one tile ahead (hides the queue atomic's latency)
-  for (;;) {
-    int t = 0;
-    if (lane == 0) {
-      t = ahead < 0 ? atomicAdd(counter, 1) : ahead;
-      ahead = t < ntiles ? atomicAdd(counter, 1) : ntiles;
-    }
-    t = __shfl_sync(0xffffffffu, t, 0);
-    if (t >= ntiles) break;
+  // the warp's first tile by its place in the grid, the next ones from the queue, each
+  // asked for when the one before it starts (hides the queue atomic's latency)
+  int t = (int)blockIdx.x * kRowWarps + warp;
+  while (t < ntiles) {
     const Tile tl = tiles[t];
+    int nt = 0;
+    if (lane == 0) nt = (int)gridDim.x * kRowWarps + atomicAdd(counter, 1);
     const AsmArgs &M = meshes[tl.mesh];
     row_stream<kRes | kJac>(M, tl.begin, tl.begin + tl.count, 1, acc[warp], lane, NP, NM);
+    t = __shfl_sync(0xffffffffu, nt, 0);
   }
 }
 
