@@ -114,7 +114,7 @@ int launch_batched_variant(int p, int v, const dev::AsmArgs *meshes, const dev::
 int launch_batched(int p, int precision, const dev::AsmArgs *meshes, const dev::Tile *tiles, int ntiles, int *counter,
                    cudaStream_t s) {
   // the same kernel as the single-mesh plan path, so batched results equal lone ones bit for bit
-  if (frag_supported(p, precision, FEM_STRAIN_LINEAR, true))
+  if (frag_supported(p, precision, FEM_STRAIN_LINEAR))
     return launch_frag_batched(p, precision, meshes, tiles, ntiles, counter, s);
   if (precision == FEM_PRECISION_FP64) return launch_batched_t<double>(p, meshes, tiles, ntiles, counter, s);
   if (precision == FEM_PRECISION_MIXED && p == 4 && umma_order4())
@@ -148,7 +148,7 @@ bool variant_allowed(int p, int precision, int v) {
 // mesh has row tables, the element kernel otherwise -- reported as ROWS).
 int default_variant(int p, int precision) {
   if (p == 1) return FEM_KERNEL_ROWS;
-  if (fem::frag_supported(p, precision, FEM_STRAIN_LINEAR, true))
+  if (fem::frag_supported(p, precision, FEM_STRAIN_LINEAR))
     return fem::b16_stiffness(p, precision, FEM_STRAIN_LINEAR) ? FEM_KERNEL_FRAGMENT_BF16X6 : FEM_KERNEL_FRAGMENT_FP64;
   if (precision == FEM_PRECISION_MIXED)
     return p == 4 && fem::umma_order4() ? FEM_KERNEL_ELEMENT_TCGEN05 : FEM_KERNEL_ELEMENT_FP32;

@@ -71,7 +71,7 @@
 // p = 2, 3 (800 x 512 p = 2: 175 / 159 / 152 us with 4 / 5 / 6; 600 x 590 p = 3: 172 / 162 /
 // 160 us), 4 at p = 4 (256^2: 102 / 107 / 115 us).
 #ifndef FEM_FRAG_MINB
-#define FEM_FRAG_MINB ((MODE & kJac) == 0 ? (P == 4 ? 4 : 6) : P == 2 ? 4 : 3)
+#define FEM_FRAG_MINB ((MODE & kJac) == 0 ? (P == 4 ? 4 : 6) : P == 2 ? 4 : P == 4 && (MODE & kPlan) == 0 ? 2 : 3)
 #endif
 
 namespace fem {
@@ -89,6 +89,14 @@ struct FragDims {
   static constexpr int CS = Dims<P>::CS;    // plan code record bytes per element
   static constexpr int WARPS = 4;           // warps per CTA
   static_assert(P >= 2 && P <= 4 && (NN == 8 * NTM || EX), "fragment kernel: orders 2 to 4");
+  // Local node at position m of the tiles: m, but at order 4, where four x-neighbours sit at
+  // positions 4r .. 4r + 3 (grid row r) and then the last column: the blocks of a row's
+  // four columns, and the residual rows of a quadruple of lanes, are adjacent in memory
+  // wherever the numbering follows the grid.  (Not the plan's Jacobian, whose blocks leave
+  // one by one: 381 x 379 1034 us, permuted 1075.)
+  __host__ __device__ static constexpr int node(int m) {
+    return P < 4 ? m : (m < 20 ? 5 * (m >> 2) + (m & 3) : (m < 24 ? 5 * (m - 20) + 4 : 24));
+  }
   // Node-tile pair k = (ta, tb) of a pass: pass 0 the pairs of tiles 0 and 1 (order 2: of
   // tile 0), pass 1 those of tile 2.
   static constexpr int NPAIR = NTM == 1 ? 1 : 3;
@@ -107,7 +115,8 @@ template <int P, bool DROP = false, bool NL = false, bool B16 = false, bool JAC 
 struct FragLayout {
   using F = FragDims<P>;
   static constexpr int K4 = F::K4, NQP = F::NQP, NN = F::NN;
-  static constexpr int CS = DROP ? 4 * NN * NN : F::CS;  // staged bytes per element
+  // staged bytes per element (drop-in order 4: none, the issuing lanes load their entries)
+  static constexpr int CS = !DROP ? F::CS : (P == 4 ? 0 : 4 * NN * NN);
   // Slot of quadrature point q of an element's arrays, and the slots between the two
   // elements: a quarter-warp of the quadrature stage stores points q, q + 1 of two
   // tiles of both elements (slots g, g + 10, g + PS, g + PS + 10 with PS = 4 mod 8:
@@ -121,8 +130,10 @@ struct FragLayout {
   static constexpr size_t wq = tabX + (F::EX ? 16 * NQP : 0);  // double [NQT]
   static constexpr size_t csum = align16(wq + 8 * NQT);       // double2 [NQT]: sum_a dN(a, q)
   static constexpr size_t tabB = align16(csum + 16 * NQT);    // double2 [8][32]: BF16x6 stiffness operands
-  static constexpr size_t tabR = align16(tabB + (B16 ? 16 * 8 * 32 : 0));  // uint32 [64]: runs (order 3)
-  static constexpr size_t warps = align16(tabR + (P == 3 ? 4 * 64 : 0));
+  // uint32: runs (order 3: 64; drop-in orders 2 and 4: DR per pass)
+  static constexpr int DR = !DROP || !JAC ? 0 : (P == 2 ? 32 : P == 4 ? 96 : 0);
+  static constexpr size_t tabR = align16(tabB + (B16 ? 16 * 8 * 32 : 0));
+  static constexpr size_t warps = align16(tabR + 4 * (P == 3 ? 64 : DR * F::NPASS));
   // warp-relative; [2] = the two elements of the step, point q at slot(q) of PS
   // (residual alone: s sigma J^-T, rows x and y, in WI0 and WI1, and no more)
   static constexpr size_t WI0 = 0;                  // double2 [2][PS]: sqrt|s| (J^-1_0x, J^-1_1x)
@@ -135,8 +146,8 @@ struct FragLayout {
   static constexpr size_t RB = align16(NID + 4 * 2 * NN);  // int [2][NN]: rowp[node]
   static constexpr size_t STAGE = align16(RB + 4 * 2 * NN);  // [2 buffers][2 elements][CS] code records
   // staging slots: p = 3, 3 node-tile pairs x 2 halves, direct and transposed; p = 2, 4, the
-  // blocks one lane has in flight
-  static constexpr int NSLOT = P == 3 ? 8 : 4;
+  // blocks one lane has in flight; drop-in p = 4 a pass's pairs and node XN's blocks
+  static constexpr int NSLOT = P == 3 ? 8 : (P == 4 && DROP ? 11 : 4);
   static constexpr size_t REDS = align16(STAGE + 2 * 2 * CS);  // double4 [NSLOT][32]: bulk-reduction sources
   // NONLINEAR: sign(s) x tangent modulus, double [2][NQP][2 (l)][8 (i, k, n)]
   static constexpr size_t AT = align16(REDS + (JAC ? 32 * NSLOT * 32 : 0));
@@ -193,11 +204,72 @@ __device__ __forceinline__ uint32_t frag_run(int sl, int r) {
   return (uint32_t)(row * 16 + col0) | (uint32_t)(128 * sl + 4 * pos0) << 16;
 }
 
-// SQRTW: the square roots of the Gauss weights instead of the weights.
-template <int P, bool B16, bool SQRTW>
-__device__ __forceinline__ void frag_prologue(unsigned char *smem) {
+// Drop-in orders 2 and 4, entry i of a pass: up to four staged blocks of one matrix row,
+// packed as row NN + first column | (columns 5 apart) << 10 | (blocks - 1) << 11 |
+// staged position << 13; 0xffffffff: none.  Staging slots: a pass's node-tile pairs
+// (direct: position 4r + t of row pi(r), transposed: 8t + pi(g)), then node XN's row and
+// column, (XN, m) and (m, XN), and its diagonal block.
+template <int P>
+__host__ __device__ __forceinline__ uint32_t drop_run(int pass, int i) {
   using F = FragDims<P>;
-  using L = FragLayout<P, false, false, B16>;
+  constexpr int NN = F::NN, XN = NN - 1;
+  auto pack = [](int row, int col0, bool five, int n, int src) {
+    return (uint32_t)(row * NN + col0) | (uint32_t)five << 10 | (uint32_t)(n - 1) << 11 | (uint32_t)src << 13;
+  };
+  auto pi = [](int r) { return 4 * (r & 1) + (r >> 1); };
+  auto quad = [&](int row, int m0, int src) { return pack(row, F::node(m0), m0 == 20, 4, src); };
+  if constexpr (P == 2) {
+    if (i < 16) return quad(pi(i & 7), 4 * (i >> 3), 32 * (i >> 3) + 4 * (i & 7));
+    if (i < 18) return quad(XN, 4 * (i - 16), 64 + 4 * (i - 16));
+    if (i < 26) return pack(i - 18, XN, false, 1, 64 + 8 + i - 18);
+    return i == 26 ? pack(XN, XN, false, 1, 64 + 16) : 0xffffffffu;
+  } else if constexpr (P == 4) {
+    const int s = i >> 3, r = i & 7, np = pass ? 80 : 64;
+    if (i < np) {
+      const int k = pass ? (s < 8 ? s >> 2 : 2) : (s < 2 ? 0 : s < 6 ? 1 : 2);
+      const int h = pass ? (s < 8 ? (s >> 1) & 1 : s - 8) : (s < 2 ? s : s < 6 ? (s - 2) >> 1 : s - 6);
+      const bool w = pass ? (s < 8 && (s & 1)) : (s >= 2 && s < 6 && (s & 1));
+      const int TA = F::ta(pass, k), TB = F::tb(pass, k);
+      if (!w) return quad(F::node(8 * TA + pi(r)), 8 * TB + 4 * h, 32 * s + 4 * r);
+      const int tt = r >> 1, half = r & 1;
+      return quad(F::node(8 * TB + 4 * h + tt), 8 * TA + 4 * half, 32 * s + 8 * tt + 4 * half);
+    }
+    const int j = i - np, sx = 4 * np;  // node XN's slot follows the pairs'
+    const int nq = pass ? 2 : 4, nm = pass ? 8 : 16, m0 = pass ? 16 : 0;
+    if (j < nq) return quad(XN, m0 + 4 * j, sx + 4 * j);
+    if (j < nq + nm) return pack(F::node(m0 + j - nq), XN, false, 1, sx + nm + j - nq);
+    return pass && j == nq + nm ? pack(XN, XN, false, 1, sx + 2 * nm) : 0xffffffffu;
+  }
+  return 0xffffffffu;
+}
+
+// Drop-in: the blocks staged from `src` on are added at map offsets m[0..3] (n = 1 or 4
+// of them), each maximal stretch of blocks adjacent in the matrix with one reduction;
+// FP64 atomics where the matrix is not 16-byte aligned.  n = 0: none.
+__device__ __forceinline__ void drop_issue(double *mat, const int (&m)[4], int n, const double *src) {
+  if ((reinterpret_cast<uintptr_t>(mat) & 15u) != 0) {
+    for (int j = 0; j < n; j++)
+      for (int c = 0; c < 4; c++) atomicAdd(mat + m[j] + c, src[4 * j + c]);
+    return;
+  }
+  const int c1 = n == 4 && m[1] == m[0] + 4, c2 = n == 4 && m[2] == m[1] + 4, c3 = n == 4 && m[3] == m[2] + 4;
+  const int b[4] = {n ? 32 * (1 + c1 * (1 + c2 * (1 + c3))) : 0, n == 4 && !c1 ? 32 * (1 + c2 * (1 + c3)) : 0,
+                    n == 4 && !c2 ? 32 * (1 + c3) : 0, n == 4 && !c3 ? 32 : 0};
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(src);
+#pragma unroll
+  for (int j = 0; j < 4; j++)
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "setp.ne.s32 p, %2, 0;\n\t"
+                 "@p cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f64 [%0], [%1], %2;\n\t}" ::"l"(mat + m[j]),
+                 "r"(sa + 32 * j), "r"(b[j])
+                 : "memory");
+}
+
+template <int P, int MODE>
+__device__ __forceinline__ void frag_prologue(unsigned char *smem) {
+  constexpr bool B16 = (MODE & kB16) != 0, SQRTW = (MODE & kNL) == 0 && (MODE & kJac) != 0;
+  using F = FragDims<P>;
+  using L = FragLayout<P, (MODE & kPlan) == 0, (MODE & kNL) != 0, B16, (MODE & kJac) != 0>;
   constexpr int P1 = F::P1, NN = F::NN, NQ = F::NQ, K4 = F::K4, QT = F::QT, NTM = F::NTM;
   double2 *tabJ = reinterpret_cast<double2 *>(smem + L::tabJ);
   double2 *tabF = reinterpret_cast<double2 *>(smem + L::tabF);
@@ -223,10 +295,11 @@ __device__ __forceinline__ void frag_prologue(unsigned char *smem) {
     const int a = 4 * ks + (lane & 3), q = 8 * tm + (lane >> 2);
     tabJ[i] = (a < NN && q < NQ) ? dN(a, q) : make_double2(0.0, 0.0);
   }
-  // stiffness fragments at (ks, T): lane (g, t) holds dN(a = 8T + pi(g), q = 4ks + t)
+  // stiffness fragments at (ks, T): lane (g, t) holds dN(node(8T + pi(g)), q = 4ks + t)
   for (int i = threadIdx.x; i < K4 * NTM * 32; i += blockDim.x) {
     const int lane = i & 31, blk = i >> 5, ks = blk / NTM, T = blk - ks * NTM;
-    const int g = lane >> 2, t = lane & 3, a = 8 * T + 4 * (g & 1) + (g >> 1), q = 4 * ks + t;
+    const int g = lane >> 2, t = lane & 3, m = 8 * T + 4 * (g & 1) + (g >> 1), q = 4 * ks + t;
+    const int a = (MODE & (kPlan | kJac)) == (kPlan | kJac) ? m : F::node(m);
     tabF[i] = q < NQ ? dN(a, q) : make_double2(0.0, 0.0);
   }
   if constexpr (F::EX) {
@@ -235,7 +308,7 @@ __device__ __forceinline__ void frag_prologue(unsigned char *smem) {
   }
   for (int q = threadIdx.x; q < L::NQT; q += blockDim.x) {
     const double w = q < NQ ? __dmul_rn(kGW[P][q % P1], kGW[P][q / P1]) : 0.0;
-    wq[q] = SQRTW ? sqrt(w) : w;
+    wq[q] = SQRTW ? sqrt(w) : w;  // LINEAR Jacobians: the square root
   }
   // BF16x6 stiffness (order 3): entry (2k + h, lane (g, t)) holds dN(a, q) for the
   // node a = 8h + pi(g) and quadrature point q = 2t + (k & 1) + 8 (k >> 1) that lane
@@ -252,6 +325,8 @@ __device__ __forceinline__ void frag_prologue(unsigned char *smem) {
     for (int i = threadIdx.x; i < 64; i += blockDim.x)
       reinterpret_cast<uint32_t *>(smem + L::tabR)[i] = frag_run(i >> 3, i & 7);
   }
+  for (int i = threadIdx.x; i < L::DR * F::NPASS; i += blockDim.x)
+    reinterpret_cast<uint32_t *>(smem + L::tabR)[i] = drop_run<P>(i / (L::DR ? L::DR : 1), i % (L::DR ? L::DR : 1));
   // sum_a dN(a, q): zero in exact arithmetic, a few ulp of the table entries in
   // FP64; summed with Neumaier compensation (error ~1e-30 absolute) over the J-stage
   // table entries written above instead of evaluating the basis again
@@ -426,37 +501,20 @@ __device__ __forceinline__ void frag_issue_run(const Out &O, int el, uint32_t ru
   }
 }
 
-// Per-block writers (orders 2 and 4, where four consecutive element-local nodes straddle
-// grid rows and row runs rarely merge): block (r0, c0) of element `el`, where `act`.
-// Plan: the first contributor stores it, a later one stages it in `slot` (this lane's,
-// its previous bulk read complete) for bulk_add_block.  Drop-in: staged for the offset
-// of the reference map (accumulate-into contract; elements of one launch share blocks),
-// or added with four FP64 atomics when the block is not 16-byte aligned.  Without a
-// branch but for that case.  Returns whether it staged the block, with its address.
-template <int P, bool PLAN>
+// Per-block writer of plans at orders 2 and 4, where four consecutive element-local nodes
+// straddle grid rows and row runs rarely merge: block (r0, c0) of element `el`, where
+// `act`.  The first contributor stores it, a later one stages it in `slot` (this lane's,
+// its previous bulk read complete) for bulk_add_block.  Without a branch.  Returns
+// whether it staged the block, with its address.
+template <int P>
 __device__ __forceinline__ bool frag_put_block(const Out &O, int el, int r0, int c0, bool act, double v0, double v1,
                                                double v2, double v3, double *slot, double *&blk) {
   constexpr int NN = Dims<P>::NN, CS = Dims<P>::CS;
   if (!act) r0 = c0 = 0;
-  uint32_t first = 0;
-  bool add = act;
-  if constexpr (PLAN) {
-    const uint32_t code = O.codes[el * CS + r0 * NN + c0];
-    blk = O.mat + 4 * ((int64_t)O.rbase[el * NN + r0] + (code & 0x7f));
-    first = code & 0x80;
-    add = act && !first;
-  } else {
-    blk = O.mat + O.map[(el * NN + r0) * NN + c0];
-    if ((reinterpret_cast<uintptr_t>(blk) & 15u) != 0) {
-      if (act) {
-        atomicAdd(blk + 0, v0);
-        atomicAdd(blk + 1, v1);
-        atomicAdd(blk + 2, v2);
-        atomicAdd(blk + 3, v3);
-      }
-      add = false;
-    }
-  }
+  const uint32_t code = O.codes[el * CS + r0 * NN + c0];
+  blk = O.mat + 4 * ((int64_t)O.rbase[el * NN + r0] + (code & 0x7f));
+  const uint32_t first = code & 0x80;
+  const bool add = act && !first;
   asm volatile("{\n\t.reg .pred f, s;\n\t"
                "setp.ne.u32 f, %6, 0;\n\t"
                "setp.ne.u32 s, %7, 0;\n\t"
@@ -805,7 +863,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
         constexpr int B0 = NN * NN / 16, NB = (NN * NN + NN - 1) / 16 - B0 + 1;
         const int e = lane / NB, i = B0 + lane - e * NB;
         if (e < c.ne) cp_async16(dst + e * CS + 16 * i, args(c).blockCode + (c.k0 + e) * CS + 16 * i);
-      } else if constexpr (JAC) {
+      } else if constexpr (JAC && STG > 0) {
         // element map rows: 16-byte copies when a row set is a multiple of 16 bytes
         const int *src = args(c).map + c.k0 * NN * NN;
         if ((NN * NN) % 4 == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
@@ -1129,7 +1187,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
         sx[x] = i ? r : v0;
         sy[x] = i ? v1 : r;
         const bool xl = EX && T + 1 == NTM && up;
-        const int a = xl ? XN : 8 * (T + up) + 4 * i + t;
+        const int a = xl ? XN : F::node(8 * (T + up) + 4 * i + t);
         act[x] = e < ne && (!xl || (i == 0 && t == 0));
         dst[x] = M.residual + 2 * (int64_t)nid[e * NN + a];
         first[x] = PLAN && O.codes[e * CS + NN * NN + a];
@@ -1147,6 +1205,15 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
       }
     } else {
       const int pa = 4 * (g & 1) + (g >> 1);  // pi(g)
+      // nodes of a lane's row (8T + pi(g)) and column (8T + 4h + t) positions (FragDims::node,
+      // drop-in)
+      constexpr bool PERM = P == 4 && !PLAN;
+      const int p0 = !PERM ? pa : 5 * (g & 1) + (g >> 1);
+      const int p2 = !PERM ? 16 + pa : ((g & 1) ? 5 * (g >> 1) + 4 : 20 + (g >> 1));
+      auto row_node = [&](int T) { return T == 2 ? p2 : (PERM ? 10 : 8) * T + p0; };
+      auto col_node = [&](int T, int h) {
+        return !PERM ? 8 * T + 4 * h + t : T == 2 ? (h ? 5 * t + 4 : 20 + t) : 5 * (2 * T + h) + t;
+      };
       int half = 0;  // orders 2 and 4: half of the lane's staging slots the next blocks use
       for (int el = 0; el < ne; el++) {
         // Strips: the blocks of an edge's nodes among themselves and their residual rows
@@ -1410,6 +1477,18 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
             }
           }
         };
+        // drop-in order 4: the lane's map entries of this pass, in flight during the products
+        int mp[L::DR ? L::DR / 32 : 1][4];
+        if constexpr (JAC && !PLAN && P == 4) {
+          const int *row = M.map + (cur.k0 + el) * (int64_t)(NN * NN);
+#pragma unroll
+          for (int x = 0; x < L::DR / 32; x++) {
+            const uint32_t e = tabR[PASS * L::DR + 32 * x + lane];
+            const int o = e == 0xffffffffu ? 0 : e & 0x3ff, n = e == 0xffffffffu ? 0 : (e >> 11) & 3;
+#pragma unroll
+            for (int j = 0; j < 4; j++) mp[x][j] = __ldg(row + o + (j <= n ? j : 0) * (e >> 10 & 1 ? 5 : 1));
+          }
+        }
         kstep_all(kstep, neg);
         // residual: sum over the four lanes t of a node (reduce-scatter over the two slots)
         [[maybe_unused]] const int Tm = t >> 1, To = Tm ^ 1;
@@ -1419,7 +1498,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
           sx += __shfl_xor_sync(0xffffffffu, sx, 1);
           sy += __shfl_xor_sync(0xffffffffu, sy, 1);
           if constexpr (STRIP) residual_carry(sx, sy, cin);
-          const int an = Tm == 0 ? 8 * RT0 + pa : (RT1 == NTM ? XN : 8 * RT1 + pa);
+          const int an = Tm == 0 ? row_node(RT0) : (RT1 == NTM ? XN : row_node(RT1));
           const bool act = (t & 1) == 0 && (Tm == 0 || RT1 < NTM || g == 0) && !halo && !(right && g >= 6);
           residual_put(M.residual + 2 * (int64_t)nid[el * NN + an], act, PLAN && O.codes[el * CS + NN * NN + an], sx, sy);
         }
@@ -1518,7 +1597,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
         // xs, lanes t/2 = x take slot x, t even (XN, a), t odd its transpose.  First stores
         // go out at once, the blocks to add are staged and leave FL at a time after one
         // proxy fence, as one bulk group, from two halves of the lane's slots in turn.
-        if constexpr (JAC && EX) {
+        if constexpr (JAC && EX && PLAN) {
           constexpr int FL = P == 2 && !NL ? 3 : 2, HALF = FL == 2 ? 2 : 0;
           double *reds = redsW + 4 * lane;
           double *dst[FL];
@@ -1529,9 +1608,9 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
 #pragma unroll
             for (int x = 0; x < FL; x++) any = any || (x < m && add[x]);
             if (!__any_sync(0xffffffffu, any)) return;
-            if (PLAN && el > 0) pair_first_landed();
+            if (el > 0) pair_first_landed();
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            if (PLAN && el > 0) {
+            if (el > 0) {
               __syncwarp();
               pair_first_visible();
             }
@@ -1547,7 +1626,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
               if constexpr (HALF) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
               else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
             }
-            add[n] = frag_put_block<P, PLAN>(O, el, r, c, act, v0, v1, v2, v3, reds + 128 * (HALF * half + n), dst[n]);
+            add[n] = frag_put_block<P>(O, el, r, c, act, v0, v1, v2, v3, reds + 128 * (HALF * half + n), dst[n]);
             if (++n == FL) {
               flush(FL);
               n = 0;
@@ -1559,7 +1638,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
 #pragma unroll
             for (int h = 0; h < 2; h++) {
               const int TA = F::ta(PASS, k), TB = F::tb(PASS, k);
-              const int a = 8 * TA + pa, b = 8 * TB + 4 * h + t;
+              const int a = row_node(TA), b = col_node(TB, h);
               const bool diag = NL && TA == TB;
               block(acc[k][0][h], acc[k][1][h], acc[k][2][h], acc[k][3][h], kxx, kxy, kyx, kyy);
               put(a, b, !diag || a <= b, kxx, kxy, kyx, kyy);
@@ -1572,10 +1651,69 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
             xv[c] += __shfl_xor_sync(0xffffffffu, xv[c], 1);
           }
           block(xv[0], xv[1], xv[2], xv[3], kxx, kxy, kyx, kyy);
-          const int xa = Tm == 0 ? 8 * RT0 + pa : (RT1 == NTM ? XN : 8 * RT1 + pa);
+          const int xa = Tm == 0 ? row_node(RT0) : (RT1 == NTM ? XN : row_node(RT1));
           const bool tr = t & 1;
           put(tr ? xa : XN, tr ? XN : xa, Tm == 0 || RT1 < NTM || (g == 0 && !tr), kxx, tr ? kyx : kxy, tr ? kxy : kyx, kyy);
           if (n) flush(n);
+        }
+        // drop-in, orders 2 and 4: every block is staged (drop_run), and each lane adds its
+        // entries' stretches of adjacent blocks.  A reduction of 32 bytes per block bounded
+        // these launches: 200 x 201 order 4, with the element kernel's FP64 atomics 987 us
+        // for the driver's two calls, with 32-byte reductions 1082, with stretches 648;
+        // 501 x 500 order 2 597 -> 496
+        if constexpr (JAC && EX && !PLAN) {
+          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          __syncwarp();
+          auto stage_at = [&](int block, double v0, double v1, double v2, double v3) {
+            double2 *x = reinterpret_cast<double2 *>(redsW + 4 * block);
+            x[0] = make_double2(v0, v1);
+            x[1] = make_double2(v2, v3);
+          };
+          double kxx, kxy, kyx, kyy;
+          int sl = 0;  // slots in the order of drop_run
+#pragma unroll
+          for (int k = 0; k < NPAIR; k++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+              const int TA = F::ta(PASS, k), TB = F::tb(PASS, k);
+              block(acc[k][0][h], acc[k][1][h], acc[k][2][h], acc[k][3][h], kxx, kxy, kyx, kyy);
+              if constexpr (NL) {  // order 2: (a, b) for a <= b and its exact transpose
+                const int b = 4 * h + t;
+                if (pa <= b) stage_at(32 * h + 4 * g + t, kxx, kxy, kyx, kyy);
+                if (pa < b) stage_at(32 * (pa >> 2) + 4 * (2 * (b & 3) + (b >> 2)) + (pa & 3), kxx, kyx, kxy, kyy);
+              } else {
+                stage_at(32 * sl++ + 4 * g + t, kxx, kxy, kyx, kyy);
+                if (TA < TB) stage_at(32 * sl++ + 8 * t + pa, kxx, kyx, kxy, kyy);
+              }
+            }
+          double xv[4];
+#pragma unroll
+          for (int c = 0; c < 4; c++) {
+            xv[c] = (Tm ? xs[1][c] : xs[0][c]) + __shfl_xor_sync(0xffffffffu, To ? xs[1][c] : xs[0][c], 2);
+            xv[c] += __shfl_xor_sync(0xffffffffu, xv[c], 1);
+          }
+          block(xv[0], xv[1], xv[2], xv[3], kxx, kxy, kyx, kyy);
+          constexpr int SX = 32 * (P == 2 ? 2 : PASS ? 10 : 8), NM = RT1 < NTM ? 16 : 8;
+          const bool tr = t & 1, xd = RT1 == NTM && Tm == 1;  // xd: the diagonal block's lanes
+          if (!xd || (g == 0 && !tr))
+            stage_at(SX + (xd ? 2 * NM : (tr ? NM : 0) + 8 * Tm + pa), kxx, tr ? kyx : kxy, tr ? kxy : kyx, kyy);
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+#pragma unroll
+          for (int x = 0; x < L::DR / 32; x++) {
+            const uint32_t e = tabR[PASS * L::DR + 32 * x + lane];
+            int m[4];
+            if constexpr (P == 4) {
+#pragma unroll
+              for (int j = 0; j < 4; j++) m[j] = mp[x][j];
+            } else {
+              const int *row = O.map + el * NN * NN + (e == 0xffffffffu ? 0 : e & 0x3ff);
+#pragma unroll
+              for (int j = 0; j < 4; j++) m[j] = row[j < (int)((e >> 11) & 3) + 1 ? j : 0];
+            }
+            drop_issue(O.mat, m, e == 0xffffffffu ? 0 : ((e >> 11) & 3) + 1, redsW + 4 * (e >> 13 & 0x1ff));
+          }
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
         };
         pass(IC<0>{});
@@ -1603,7 +1741,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
 template <int P, int MODE>
 __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB) frag_kernel(const __grid_constant__ AsmArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
-  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) == 0 && (MODE & kJac) != 0>(smem);
+  frag_prologue<P, MODE>(smem);
   const int warp = threadIdx.x >> 5;
   PairStride gen{A.begin, A.begin + A.count, (int64_t)blockIdx.x * FragDims<P>::WARPS + warp,
                  (int64_t)gridDim.x * FragDims<P>::WARPS};
@@ -1615,7 +1753,7 @@ template <int P, int MODE>
 __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB)
     frag_ranges_kernel(const __grid_constant__ AsmArgs A, const RangeList R) {
   extern __shared__ __align__(16) unsigned char smem[];
-  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) == 0 && (MODE & kJac) != 0>(smem);
+  frag_prologue<P, MODE>(smem);
   const int warp = threadIdx.x >> 5;
   PairRanges gen{R, (int64_t)blockIdx.x * FragDims<P>::WARPS + warp, (int64_t)gridDim.x * FragDims<P>::WARPS};
   frag_loop<P, MODE>(smem, gen, A, &A);
@@ -1631,7 +1769,7 @@ __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB)
     frag_strip_kernel(const __grid_constant__ AsmArgs A, const __grid_constant__ RangeList R,
                       const Strip *__restrict__ strips) {
   extern __shared__ __align__(16) unsigned char smem[];
-  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) == 0 && (MODE & kJac) != 0>(smem);
+  frag_prologue<P, MODE>(smem);
   const int warp = threadIdx.x >> 5;
   StripRanges gen{strips, R, (int64_t)blockIdx.x * FragDims<P>::WARPS + warp, (int64_t)gridDim.x * FragDims<P>::WARPS};
   gen.fetch();
@@ -1643,7 +1781,7 @@ template <int P, int MODE>
 __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB)
     frag_sched_kernel(const __grid_constant__ AsmArgs A, const __grid_constant__ SchedArgs S) {
   extern __shared__ __align__(16) unsigned char smem[];
-  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) == 0 && (MODE & kJac) != 0>(smem);
+  frag_prologue<P, MODE>(smem);
   PairSched gen{&S};
   frag_loop<P, MODE>(smem, gen, A, &A);
 }
@@ -1655,7 +1793,7 @@ template <int P, int MODE>
 __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB)
     frag_batched_sched_kernel(const AsmArgs *__restrict__ meshes, const __grid_constant__ SchedArgs S) {
   extern __shared__ __align__(16) unsigned char smem[];
-  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) == 0 && (MODE & kJac) != 0>(smem);
+  frag_prologue<P, MODE>(smem);
   PairSchedT<true> gen{&S};
   frag_loop<P, MODE>(smem, gen, meshes[0], meshes);
 }
@@ -1665,7 +1803,7 @@ template <int P, int MODE>
 __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB)
     frag_batched_kernel(const AsmArgs *__restrict__ meshes, const Tile *__restrict__ tiles, int ntiles, int *counter) {
   extern __shared__ __align__(16) unsigned char smem[];
-  frag_prologue<P, (MODE & kB16) != 0, (MODE & kNL) == 0 && (MODE & kJac) != 0>(smem);
+  frag_prologue<P, MODE>(smem);
   constexpr int W = FragDims<P>::WARPS;
   PairQueue gen{tiles, ntiles, counter, (int)gridDim.x * W, (int)blockIdx.x * W + (int)(threadIdx.x >> 5)};
   frag_loop<P, MODE>(smem, gen, meshes[0], meshes);
@@ -1859,23 +1997,21 @@ bool b16_stiffness(int order, int precision, int strain) {
   return precision == FEM_PRECISION_MIXED && strain == FEM_STRAIN_LINEAR && order == 3;
 }
 
-// FP64, LINEAR: orders 2 and 3 in every mode; order 4 in plan mode only (single
-// meshes, batches, the server): measured on B200, the order-4 fragment kernel runs
-// the 256-mesh batch in 170 against 217 ms and one 512^2 mesh in 3.03 against
-// 3.00 ms for the element kernel, and plans and batches must run the same kernel
-// (a mesh's batched result equals its single-mesh plan result bit for bit); the
-// order-4 drop-in keeps the element kernel (4.7 ms against 6.9 ms).
+// FP64, LINEAR: orders 2 to 4 in every mode (one 512^2 order-4 mesh took 3.00 ms with the
+// element kernel and 2.03 with this one; drop-in, 400 x 390 with its residual call 3.80
+// against 2.40 ms).  Plans and batches must run the same kernel (a mesh's batched result
+// equals its single-mesh plan result bit for bit).
 // MIXED at orders 2 and 3 also runs this kernel (faster than the FP32 element
 // products there: 3.1 against 3.8 ms at 1024^2 p = 3): at order 3 with the element
 // stiffness as BF16x6 tensor-core products (b16_stiffness), at order 2 in FP64 (the
-// FP64 result, as order-1 row assembly gives); at order 4 the FP32 element kernel is
-// the faster one (2.6 against 3.4 ms) and MIXED keeps it.
-bool frag_supported(int order, int precision, int strain, bool plan) {
+// FP64 result, as order-1 row assembly gives).  MIXED at order 4 keeps the FP32 element
+// kernel, whose results its callers have.
+bool frag_supported(int order, int precision, int strain) {
   if (strain == FEM_STRAIN_NONLINEAR) return precision == FEM_PRECISION_FP64 && (order == 2 || order == 3);
   if (strain != FEM_STRAIN_LINEAR) return false;
   if (precision == FEM_PRECISION_MIXED) return order == 2 || order == 3;
   if (precision != FEM_PRECISION_FP64) return false;
-  return order == 2 || order == 3 || (order == 4 && plan);
+  return order >= 2 && order <= 4;
 }
 
 int launch_frag(int order, int precision, int mode, const dev::AsmArgs &a, cudaStream_t s, int strain, bool chained) {

@@ -103,12 +103,12 @@ int launch(int order, int precision, int mode, const dev::AsmArgs &a, cudaStream
   if (strain == FEM_STRAIN_NONLINEAR) {
     if (precision != FEM_PRECISION_FP64)
       return fail(FEM_ERR_INVALID_ARGUMENT, "NONLINEAR strain is assembled in FP64 only (precision %d)", precision);
-    if (frag_supported(order, precision, strain, (mode & dev::kPlan) != 0))
+    if (frag_supported(order, precision, strain))
       return launch_frag(order, precision, mode, a, s, strain);
     return launch_nl(order, mode, a, s);
   }
   if (strain != FEM_STRAIN_LINEAR) return fail(FEM_ERR_INVALID_ARGUMENT, "strain type %d", strain);
-  if ((mode & dev::kPlan) == 0 && frag_supported(order, precision, strain, false))
+  if ((mode & dev::kPlan) == 0 && frag_supported(order, precision, strain))
     return launch_frag(order, precision, mode, a, s);
   if (precision == FEM_PRECISION_FP64) return launch_any<double>(order, mode, a, s);
   if (precision == FEM_PRECISION_MIXED && order == 4 && (mode & dev::kJac) && umma_order4()) {
@@ -372,7 +372,7 @@ bool plan_pairs(const fem_plan *p) { return p->usePairs && p->numPairColours > 0
 
 // Whether fem_plan_assemble runs `p` as one dependency-ordered launch.
 bool plan_sched(const fem_plan *p, int precision, int strain) {
-  return p->schedGroups > 0 && fem::frag_supported(p->order, precision, strain, true) &&
+  return p->schedGroups > 0 && fem::frag_supported(p->order, precision, strain) &&
          !(fem::plan_rows(p) && strain == FEM_STRAIN_LINEAR);
 }
 }  // namespace
@@ -681,7 +681,7 @@ int fem_plan_assemble_ex(const fem_plan *plan, const double *states, const doubl
     a.count = plan->numChunks;
     return fem::timed(s, elapsedSeconds, [&] { return fem::launch_rows(mode, a, s); });
   }
-  const bool frag = fem::frag_supported(plan->order, precision, strainType, true);
+  const bool frag = fem::frag_supported(plan->order, precision, strainType);
   if (plan_sched(plan, precision, strainType)) {
     // all colours in one dependency-ordered launch; the tile dispenser and the
     // per-group counters start at zero, the sticky timeout count (word 0) is kept
@@ -793,7 +793,7 @@ int fem_plan_assemble_host(const fem_plan *plan, const double *hostStates, doubl
       if (err != cudaSuccess) return fem::cuda_fail(err, "cudaStreamCreateWithFlags");
     }
   }
-  const bool frag = fem::frag_supported(plan->order, precision, strainType, true);
+  const bool frag = fem::frag_supported(plan->order, precision, strainType);
   const bool rows = fem::plan_rows(plan) && strainType == FEM_STRAIN_LINEAR;
   // the fragment kernel runs the pair layout when the plan uses it (each band's pairs
   // and unpaired elements are two ranges of a colour), else the colour layout

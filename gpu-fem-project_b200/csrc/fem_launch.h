@@ -117,7 +117,7 @@ constexpr int kRowTileChunks = 16, kRowWarpsResident = 148 * 12;
 // accumulate-into).
 // FEM_PRECISION_MIXED at order 3 runs its element stiffness as BF16x6 tensor-core
 // products (b16_stiffness); the rest stays FP64.
-bool frag_supported(int order, int precision, int strain, bool plan);
+bool frag_supported(int order, int precision, int strain);
 bool b16_stiffness(int order, int precision, int strain);
 // chained: the launch directly follows this assembly's previous fragment-kernel
 // launch on the stream and may overlap its tail (programmatic dependent launch).
