@@ -157,6 +157,21 @@ static void build_row_plan(HostPlan &hp) {
       ent[2 * (size_t)j + 1] = ranks;
     }
   }
+  // a row's first entry with a block: bit 7 of that block's rank
+#pragma omp parallel for schedule(static)
+  for (int r = 0; r < N; r++) {
+    uint64_t seen[2] = {0, 0};
+    for (int j = ptr[r]; j < ptr[r + 1]; j++) {
+      uint32_t ranks = (uint32_t)ent[2 * (size_t)j + 1];
+      for (int b = 0; b < 4; b++) {
+        const uint32_t k = (ranks >> (8 * b)) & 0x7f;
+        uint64_t &w = seen[k >> 6];
+        if (!(w >> (k & 63) & 1)) ranks |= 0x80u << (8 * b);
+        w |= 1ull << (k & 63);
+      }
+      ent[2 * (size_t)j + 1] = (int)ranks;
+    }
+  }
   std::vector<int> chunk(1, 0);
   int rows = 0;
   int64_t blocks = 0;
