@@ -82,6 +82,7 @@ struct HostPlan {
   std::vector<int> stripColourPtr, stripConn, stripLo, stripHi;  // Lo, Hi: node span per strip, halo included
   std::vector<uint8_t> stripCode;
 };
+constexpr int kPairMinElements = 4 * 148 * 12;  // four colours of one element per resident warp
 constexpr int kStripOrder = 3;
 constexpr int kStripWarps = 148 * 12;  // resident warps of the strip kernel
 constexpr int kRowChunkRows = 32, kRowChunkBlocks = 320;

@@ -545,13 +545,15 @@ struct PairCursor {
 };
 
 
-// Single mesh: pairs p, p + stride, ... of list positions [begin, end).
+// Single mesh: pairs p, p + stride, ... of list positions [begin, end); `unit` 1: single
+// elements (launches that do not fill the GPU).
 struct PairStride {
   static constexpr bool kBatched = false, kSched = false, kStrip = false;
   int64_t begin, end, p, stride;
+  int unit;
   __device__ PairCursor next(int) {
-    PairCursor c{0, 0, begin + 2 * p};
-    if (c.k0 < end) c.ne = (int)min((int64_t)2, end - c.k0);
+    PairCursor c{0, 0, begin + unit * p};
+    if (c.k0 < end) c.ne = (int)min((int64_t)unit, end - c.k0);
     p += stride;
     return c;
   }
@@ -1739,12 +1741,13 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
 // One mesh: plan mode, list positions [A.begin, A.begin + A.count) of one colour;
 // drop-in mode, elements [A.begin, A.begin + A.count) through the reference map.
 template <int P, int MODE>
-__global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB) frag_kernel(const __grid_constant__ AsmArgs A) {
+__global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB) frag_kernel(const __grid_constant__ AsmArgs A,
+                                                                                             int unit) {
   extern __shared__ __align__(16) unsigned char smem[];
   frag_prologue<P, MODE>(smem);
   const int warp = threadIdx.x >> 5;
   PairStride gen{A.begin, A.begin + A.count, (int64_t)blockIdx.x * FragDims<P>::WARPS + warp,
-                 (int64_t)gridDim.x * FragDims<P>::WARPS};
+                 (int64_t)gridDim.x * FragDims<P>::WARPS, unit};
   frag_loop<P, MODE>(smem, gen, A, &A);
 }
 
@@ -1832,8 +1835,10 @@ cudaError_t pdl_launch(K kernel, int grid, int nt, size_t smem, cudaStream_t s, 
 // stream (a later colour or band), whose outputs are the only ones it may read
 // early, so it may start as that one drains; a first launch follows the caller's
 // work, which may have produced its inputs, and launches in stream order.
+// single: the listed elements are independent (not the pair layout's), so that a small
+// launch may take them one by one.
 template <int P, int MODE>
-int launch_frag_p(const AsmArgs &a, cudaStream_t s, bool chained) {
+int launch_frag_p(const AsmArgs &a, cudaStream_t s, bool chained, bool single) {
   using F = FragDims<P>;
   constexpr int NT = 32 * F::WARPS;
   auto kernel = frag_kernel<P, MODE>;
@@ -1841,8 +1846,6 @@ int launch_frag_p(const AsmArgs &a, cudaStream_t s, bool chained) {
   LaunchInfo li;
   int st = launch_info(kernel, NT, smem, li);
   if (st) return st;
-  const int64_t pairs = (a.count + 1) / 2;
-  const int64_t need = (pairs + F::WARPS - 1) / F::WARPS;
   // Order-3 drop-in Jacobian (every block added through the element map, one launch
   // whose elements share blocks): two CTAs per SM.  At 1024^2 the kernel took 3.90 ms
   // with two resident CTAs per SM against 4.35 ms with three (the bulk reductions of
@@ -1851,13 +1854,20 @@ int launch_frag_p(const AsmArgs &a, cudaStream_t s, bool chained) {
   const int perSm =
       (P == 3 && (MODE & kPlan) == 0 && (MODE & kJac) != 0) ? std::min(li.grid_per_sm, 2) : li.grid_per_sm;
   const int64_t cap = (int64_t)perSm * li.num_sms;
+  // A launch whose elements all find a warp of their own takes one per warp instead of a
+  // pair: the warp's step is what the launch takes, and one element's stiffness and writes
+  // are most of half of it (33 x 31 order 4 63.5 -> 38.9 us, order 3 NONLINEAR
+  // 44.1 -> 22.6; order 2, bound by its four launches, 18.5 -> 18.4).
+  const int unit = single && a.count <= cap * F::WARPS ? 1 : 2;
+  const int64_t units = (a.count + unit - 1) / unit;
+  const int64_t need = (units + F::WARPS - 1) / F::WARPS;
   const int grid = (int)(need < cap ? need : cap);
   if (grid <= 0) return FEM_SUCCESS;
   cudaError_t err;
   if (chained) {
-    err = pdl_launch(kernel, grid, NT, smem, s, a);
+    err = pdl_launch(kernel, grid, NT, smem, s, a, unit);
   } else {
-    kernel<<<grid, NT, smem, s>>>(a);
+    kernel<<<grid, NT, smem, s>>>(a, unit);
     err = cudaGetLastError();
   }
   if (err != cudaSuccess) return cuda_fail(err, "frag_kernel launch");
@@ -1974,15 +1984,15 @@ int launch_frag_sched_p(const AsmArgs &a, const SchedArgs &sa, cudaStream_t s) {
 }
 
 template <int MODE>
-int launch_frag_mode(int order, const AsmArgs &a, cudaStream_t s, bool chained) {
+int launch_frag_mode(int order, const AsmArgs &a, cudaStream_t s, bool chained, bool single) {
   switch (order) {
     case 2:
       if constexpr ((MODE & kB16) != 0) return fail(FEM_ERR_INVALID_ORDER, "fragment kernel, BF16x6: order 2");
-      else return launch_frag_p<2, MODE>(a, s, chained);
-    case 3: return launch_frag_p<3, MODE>(a, s, chained);
+      else return launch_frag_p<2, MODE>(a, s, chained, single);
+    case 3: return launch_frag_p<3, MODE>(a, s, chained, single);
     case 4:
       if constexpr ((MODE & (kNL | kB16)) != 0) return fail(FEM_ERR_INVALID_ORDER, "fragment kernel, mode %d: order 4", MODE);
-      else return launch_frag_p<4, MODE>(a, s, chained);
+      else return launch_frag_p<4, MODE>(a, s, chained, single);
     default: return fail(FEM_ERR_INVALID_ORDER, "fragment kernel: order %d", order);
   }
 }
@@ -2014,27 +2024,28 @@ bool frag_supported(int order, int precision, int strain) {
   return order >= 2 && order <= 4;
 }
 
-int launch_frag(int order, int precision, int mode, const dev::AsmArgs &a, cudaStream_t s, int strain, bool chained) {
+int launch_frag(int order, int precision, int mode, const dev::AsmArgs &a, cudaStream_t s, int strain, bool chained,
+                bool single) {
   using namespace dev;
   if (strain == FEM_STRAIN_NONLINEAR) mode |= kNL;
   if (b16_stiffness(order, precision, strain) && (mode & kJac)) mode |= kB16;
   switch (mode) {
-    case kPlan | kJac | kB16: return launch_frag_mode<kPlan | kJac | kB16>(order, a, s, chained);
-    case kPlan | kRes | kJac | kB16: return launch_frag_mode<kPlan | kRes | kJac | kB16>(order, a, s, chained);
-    case kJac | kB16: return launch_frag_mode<kJac | kB16>(order, a, s, chained);
-    case kRes | kJac | kB16: return launch_frag_mode<kRes | kJac | kB16>(order, a, s, chained);
-    case kPlan | kRes: return launch_frag_mode<kPlan | kRes>(order, a, s, chained);
-    case kPlan | kJac: return launch_frag_mode<kPlan | kJac>(order, a, s, chained);
-    case kPlan | kRes | kJac: return launch_frag_mode<kPlan | kRes | kJac>(order, a, s, chained);
-    case kRes: return launch_frag_mode<kRes>(order, a, s, chained);
-    case kJac: return launch_frag_mode<kJac>(order, a, s, chained);
-    case kRes | kJac: return launch_frag_mode<kRes | kJac>(order, a, s, chained);
-    case kNL | kPlan | kRes: return launch_frag_mode<kNL | kPlan | kRes>(order, a, s, chained);
-    case kNL | kPlan | kJac: return launch_frag_mode<kNL | kPlan | kJac>(order, a, s, chained);
-    case kNL | kPlan | kRes | kJac: return launch_frag_mode<kNL | kPlan | kRes | kJac>(order, a, s, chained);
-    case kNL | kRes: return launch_frag_mode<kNL | kRes>(order, a, s, chained);
-    case kNL | kJac: return launch_frag_mode<kNL | kJac>(order, a, s, chained);
-    case kNL | kRes | kJac: return launch_frag_mode<kNL | kRes | kJac>(order, a, s, chained);
+    case kPlan | kJac | kB16: return launch_frag_mode<kPlan | kJac | kB16>(order, a, s, chained, single);
+    case kPlan | kRes | kJac | kB16: return launch_frag_mode<kPlan | kRes | kJac | kB16>(order, a, s, chained, single);
+    case kJac | kB16: return launch_frag_mode<kJac | kB16>(order, a, s, chained, single);
+    case kRes | kJac | kB16: return launch_frag_mode<kRes | kJac | kB16>(order, a, s, chained, single);
+    case kPlan | kRes: return launch_frag_mode<kPlan | kRes>(order, a, s, chained, single);
+    case kPlan | kJac: return launch_frag_mode<kPlan | kJac>(order, a, s, chained, single);
+    case kPlan | kRes | kJac: return launch_frag_mode<kPlan | kRes | kJac>(order, a, s, chained, single);
+    case kRes: return launch_frag_mode<kRes>(order, a, s, chained, single);
+    case kJac: return launch_frag_mode<kJac>(order, a, s, chained, single);
+    case kRes | kJac: return launch_frag_mode<kRes | kJac>(order, a, s, chained, single);
+    case kNL | kPlan | kRes: return launch_frag_mode<kNL | kPlan | kRes>(order, a, s, chained, single);
+    case kNL | kPlan | kJac: return launch_frag_mode<kNL | kPlan | kJac>(order, a, s, chained, single);
+    case kNL | kPlan | kRes | kJac: return launch_frag_mode<kNL | kPlan | kRes | kJac>(order, a, s, chained, single);
+    case kNL | kRes: return launch_frag_mode<kNL | kRes>(order, a, s, chained, single);
+    case kNL | kJac: return launch_frag_mode<kNL | kJac>(order, a, s, chained, single);
+    case kNL | kRes | kJac: return launch_frag_mode<kNL | kRes | kJac>(order, a, s, chained, single);
     default: return fail(FEM_ERR_INVALID_ARGUMENT, "fragment kernel: mode %d", mode);
   }
 }

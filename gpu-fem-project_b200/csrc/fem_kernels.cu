@@ -365,10 +365,14 @@ int build_schedule(fem_plan *p, int band, int tile) {
 // NONLINEAR strain and the residual alone are bound by their arithmetic, which a strip's
 // halo adds to (400 x 397 NONLINEAR: 707 colours, 710 pairs, 789 strips; 600 x 590
 // residual: 249, 248, 281).  The other plans run their pairs.
+//
 bool plan_strips(const fem_plan *p, int strain, const double *matEntries) {
   return p->usePairs && p->numStripColours > 0 && strain == FEM_STRAIN_LINEAR && matEntries;
 }
-bool plan_pairs(const fem_plan *p) { return p->usePairs && p->numPairColours > 0 && p->numStripColours == 0; }
+// Small plans run the colours too: each element of a launch then has a warp of its own.
+bool plan_pairs(const fem_plan *p) {
+  return p->usePairs && p->numPairColours > 0 && p->numStripColours == 0 && p->numElements > fem::kPairMinElements;
+}
 
 // Whether fem_plan_assemble runs `p` as one dependency-ordered launch.
 bool plan_sched(const fem_plan *p, int precision, int strain) {
@@ -724,7 +728,7 @@ int fem_plan_assemble_ex(const fem_plan *plan, const double *states, const doubl
     for (int c = 0; c < ncol; c++) {
       a.begin = cptr[c];
       a.count = cptr[c + 1] - cptr[c];
-      int st = frag ? fem::launch_frag(plan->order, precision, mode, a, s, strainType, /*chained=*/c > 0)
+      int st = frag ? fem::launch_frag(plan->order, precision, mode, a, s, strainType, /*chained=*/c > 0, /*single=*/!pairs)
                     : fem::launch(plan->order, precision, mode, a, s, strainType);
       if (st) return st;
     }

@@ -121,8 +121,10 @@ bool frag_supported(int order, int precision, int strain);
 bool b16_stiffness(int order, int precision, int strain);
 // chained: the launch directly follows this assembly's previous fragment-kernel
 // launch on the stream and may overlap its tail (programmatic dependent launch).
+// single: the listed elements share no output in plan mode (every list but the pair
+// layout's), so a small launch may give each a warp of its own.
 int launch_frag(int order, int precision, int mode, const dev::AsmArgs &a, cudaStream_t s,
-                int strain = FEM_STRAIN_LINEAR, bool chained = false);
+                int strain = FEM_STRAIN_LINEAR, bool chained = false, bool single = true);
 // Its multi-range form (plan mode, residual always, Jacobian optional): up to
 // kMaxRanges list-position ranges of one mesh in one launch.
 int launch_frag_ranges(int order, int precision, int mode, const dev::AsmArgs &a, const dev::RangeList &r,
