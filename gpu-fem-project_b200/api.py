@@ -53,6 +53,11 @@ def _dptr(x, dtype=None, name="array"):
 def _stream(stream):
     if stream is None:
         import torch
+        # the handle itself, without building a Stream object around it (3.4 -> 0.3 us of
+        # a small call's host time: a 64 x 64 order-1 assembly 11.4 -> 7.7 us)
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        if raw is not None and torch.cuda.is_initialized():
+            return raw(torch._C._cuda_getDevice())
         return torch.cuda.current_stream().cuda_stream
     if isinstance(stream, int):
         return stream

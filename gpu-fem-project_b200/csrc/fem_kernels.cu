@@ -365,7 +365,6 @@ int build_schedule(fem_plan *p, int band, int tile) {
 // NONLINEAR strain and the residual alone are bound by their arithmetic, which a strip's
 // halo adds to (400 x 397 NONLINEAR: 707 colours, 710 pairs, 789 strips; 600 x 590
 // residual: 249, 248, 281).  The other plans run their pairs.
-//
 bool plan_strips(const fem_plan *p, int strain, const double *matEntries) {
   return p->usePairs && p->numStripColours > 0 && strain == FEM_STRAIN_LINEAR && matEntries;
 }
