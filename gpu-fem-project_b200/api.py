@@ -191,19 +191,11 @@ class Plan:
         self.row_chunks = rc.value
 
     def launches(self, strain="linear", precision="fp64") -> int:
-        """Kernel launches of one assemble(): 1 for order-1 row assembly and for a
-        dependency-ordered plan, else one per colour."""
-        if self.row_chunks > 0 and _strain(strain) == FEM_STRAIN_LINEAR:
-            return 1
-        if self.scheduled(strain, precision):
-            return 1
-        lay, _, pair_colours = self.layout()
-        if lay != "pairs" or not self.fragment(strain, precision):
-            return self.num_colours
-        _, strip_colours = self.strips()
-        if strip_colours:
-            return strip_colours if _strain(strain) == FEM_STRAIN_LINEAR else self.num_colours
-        return pair_colours
+        """Kernel launches of one residual + Jacobian assemble(): 1 for order-1 row assembly
+        and for a dependency-ordered plan, else one per colour of the layout it runs."""
+        n = C.c_int()
+        check(lib.fem_plan_launches(self._h, _prec(precision), _strain(strain), C.byref(n)), "fem_plan_launches")
+        return n.value
 
     def strips(self):
         """(strips, strip colours) of an order-3 plan's LINEAR Jacobian; (0, 0): none."""

@@ -1378,6 +1378,57 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
         // whether a point of this element has s (mu) < 0 (inverted element or negative
         // thickness or modulus): only then do the A fragments take the points' signs
         const bool neg = SCALED && (negm & (el ? 0xccccccccu : 0x33333333u)) != 0;
+        // a strip's halo: the blocks and residual rows of its right edge alone, as one 8 x 8
+        // tile (rows and columns (edge node, component)) instead of twelve; short strips of
+        // small meshes are half halos (43 x 37 18.4 -> 14.5 us, 128^2 53.3 -> 50.0, 512^2
+        // 547 -> 537)
+        if constexpr (STRIP && !B16) {
+          if (halo) {
+            const int ay = g >> 1, i = g & 1;
+            double c0, c1, px = 0.0, py = 0.0;
+#pragma unroll
+            for (int ks = 0; ks < K4; ks++) {
+              const int o = el * PS + L::slot(4 * ks) + t;
+              const double2 w = i ? WI1[o] : WI0[o];
+              const double2 d = tabF[(ks * NTM + (ay >> 1)) * 32 + 4 * (6 + (ay & 1)) + t];
+              const double fr = fma(w.x, d.x, w.y * d.y);
+              if constexpr (RES) {
+                const double2 sj = i ? WS1[o] : WS0[o];  // (S-hat_xi, S-hat_yi)
+                px = fma(fr, sj.x, px);
+                py = fma(fr, sj.y, py);
+              }
+              const double af = neg ? SGs[el * NQP + 4 * ks + t] * fr : fr;
+              if (ks == 0) dmma_first(c0, c1, af, fr);
+              else dmma(c0, c1, af, fr);
+            }
+            // lane (g, t): (M_i0, M_i1) of edge nodes (ay, by = t); the other row from lane^4
+            const double o0 = __shfl_xor_sync(0xffffffffu, c0, 4), o1 = __shfl_xor_sync(0xffffffffu, c1, 4);
+            const double mxx = i ? o0 : c0, mxy = i ? o1 : c1, myx = i ? c0 : o0, myy = i ? c1 : o1;
+            double kxx, kxy, kyx, kyy;
+            block(mxx, mxy, myx, myy, kxx, kxy, kyx, kyy);
+            // to the give lanes' staging positions, where the next element takes them
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            __syncwarp();
+            if ((ay >> 1) <= (t >> 1)) {
+              const int k = (ay >> 1) + (t >> 1);  // pairs (0, 0), (0, 1), (1, 1)
+              const int sl = k == 0 ? (t & 1) : k == 1 ? 2 + 2 * (t & 1) : 6 + (t & 1);
+              double2 *x = reinterpret_cast<double2 *>(redsW + 128 * sl + 4 * (27 + 4 * (ay & 1)));
+              x[i] = i ? make_double2(kyx, kyy) : make_double2(kxx, kxy);
+            }
+            if constexpr (RES) {
+#pragma unroll
+              for (int x = 1; x <= 4; x <<= 1) {
+                px += __shfl_xor_sync(0xffffffffu, px, x);
+                py += __shfl_xor_sync(0xffffffffu, py, x);
+              }
+              const int src = 8 * (2 * (t >> 1) + (g & 1));
+              crx = __shfl_sync(0xffffffffu, px, src);
+              cry = __shfl_sync(0xffffffffu, py, src);
+            }
+            __syncwarp();
+            continue;
+          }
+        }
         auto pass = [&](auto passc) {
         constexpr int PASS = decltype(passc)::value;
         // fragments of tiles [0, NF); residual slots: tiles RT0 and RT1, NTM = node XN;

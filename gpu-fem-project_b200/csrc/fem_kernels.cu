@@ -365,8 +365,8 @@ int build_schedule(fem_plan *p, int band, int tile) {
 // NONLINEAR strain and the residual alone are bound by their arithmetic, which a strip's
 // halo adds to (400 x 397 NONLINEAR: 707 colours, 710 pairs, 789 strips; 600 x 590
 // residual: 249, 248, 281).  The other plans run their pairs.
-bool plan_strips(const fem_plan *p, int strain, const double *matEntries) {
-  return p->usePairs && p->numStripColours > 0 && strain == FEM_STRAIN_LINEAR && matEntries;
+bool plan_strips(const fem_plan *p, int strain, bool jacobian) {
+  return p->usePairs && p->numStripColours > 0 && strain == FEM_STRAIN_LINEAR && jacobian;
 }
 // Small plans run the colours too: each element of a launch then has a warp of its own.
 bool plan_pairs(const fem_plan *p) {
@@ -703,7 +703,7 @@ int fem_plan_assemble_ex(const fem_plan *plan, const double *states, const doubl
   }
   // the fragment kernel runs the pair layout (a step's two elements share an edge,
   // so the lines of the rows they share are written while they are still in L2)
-  if (frag && plan_strips(plan, strainType, matEntries)) {
+  if (frag && plan_strips(plan, strainType, matEntries != nullptr)) {
     a.connList = plan->d_stripConn;
     a.blockCode = plan->d_stripCode;
     return fem::timed(s, elapsedSeconds, [&] {
@@ -743,6 +743,17 @@ int fem_plan_set_layout(fem_plan *plan, int layout) {
   if (layout == FEM_LAYOUT_PAIRS && plan->numPairColours == 0)
     return fem::fail(FEM_ERR_UNSUPPORTED, "this plan has no pair layout (order 1, or its pairs need > 64 colours)");
   plan->usePairs = layout == FEM_LAYOUT_PAIRS;
+  return FEM_SUCCESS;
+}
+
+int fem_plan_launches(const fem_plan *plan, int precision, int strainType, int *launches) {
+  fem::clear_error();
+  if (!plan || !launches) return fem::fail(FEM_ERR_INVALID_ARGUMENT, "NULL argument");
+  const bool frag = fem::frag_supported(plan->order, precision, strainType);
+  if ((fem::plan_rows(plan) && strainType == FEM_STRAIN_LINEAR) || plan_sched(plan, precision, strainType)) *launches = 1;
+  else if (frag && plan_strips(plan, strainType, /*jacobian=*/true)) *launches = plan->numStripColours;
+  else if (frag && plan_pairs(plan)) *launches = plan->numPairColours;
+  else *launches = plan->numColours;
   return FEM_SUCCESS;
 }
 
@@ -800,7 +811,7 @@ int fem_plan_assemble_host(const fem_plan *plan, const double *hostStates, doubl
   const bool rows = fem::plan_rows(plan) && strainType == FEM_STRAIN_LINEAR;
   // the fragment kernel runs the pair layout when the plan uses it (each band's pairs
   // and unpaired elements are two ranges of a colour), else the colour layout
-  const bool strips = frag && !rows && plan_strips(plan, strainType, matEntries);
+  const bool strips = frag && !rows && plan_strips(plan, strainType, matEntries != nullptr);
   const bool pairs = frag && !rows && !strips && plan_pairs(plan);
   const int N = plan->numNodes, nE = plan->numElements;
   const int nc = strips ? plan->numStripColours : pairs ? plan->numPairColours : plan->numColours;

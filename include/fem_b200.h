@@ -179,7 +179,9 @@ int fem_plan_row_chunks(const fem_plan *plan, int *numChunks);
  *                       plans whose elements form chains of such neighbours run the
  *                       LINEAR Jacobian (with or without the residual) by strips of
  *                       these chains instead, one launch per colour of the chains
- *                       (fem_plan_get_strips), and everything else by FEM_LAYOUT_COLOURS;
+ *                       (fem_plan_get_strips), and everything else by
+ *                       FEM_LAYOUT_COLOURS, as do plans of orders 2 and 4 with few
+ *                       elements (up to 7104: a warp then takes a single element);
  *   FEM_LAYOUT_COLOURS  the element colouring above (what every other path runs).
  * The results agree to rounding: a block's contributions are added in another
  * order where more than two elements share it.  fem_plan_get_layout also reports
@@ -189,6 +191,8 @@ int fem_plan_row_chunks(const fem_plan *plan, int *numChunks);
 #define FEM_LAYOUT_PAIRS 1
 int fem_plan_set_layout(fem_plan *plan, int layout);
 int fem_plan_get_layout(const fem_plan *plan, int *layout, int64_t *numPairs, int *numPairColours);
+/* Kernel launches of one residual + Jacobian fem_plan_assemble_ex of this plan. */
+int fem_plan_launches(const fem_plan *plan, int precision, int strainType, int *launches);
 /* Strips of an order-3 plan and their colours (launches); 0, 0 when it has none. */
 int fem_plan_get_strips(const fem_plan *plan, int *numStrips, int *numStripColours);
 /* Device pointers of the plan's rowp/cols (owned by the plan). */
