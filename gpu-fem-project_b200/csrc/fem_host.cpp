@@ -113,6 +113,44 @@ int build_pattern(int numNodes, const int *connPtr, const int *conn, int numElem
   return FEM_SUCCESS;
 }
 
+// Row pointers and columns together, each row's neighbours collected and sorted once
+// (build_pattern is called for the size first, then for the columns): blocks of rows per
+// thread, joined afterwards.  The mesh is valid.
+static int build_pattern_once(HostPlan &hp, const int *connPtr, const int *conn) {
+  const int N = hp.numNodes;
+  std::vector<int64_t> nptr;
+  std::vector<int> nelem;
+  node_elements(N, connPtr, conn, hp.numElements, nptr, nelem);
+  constexpr int kBlock = 256;
+  const int nb = (int)(((int64_t)N + kBlock - 1) / kBlock);
+  std::vector<std::vector<int>> part((size_t)nb);
+  std::vector<int64_t> len((size_t)N + 1, 0);
+#pragma omp parallel
+  {
+    std::vector<int> buf;
+#pragma omp for schedule(dynamic, 1)
+    for (int b = 0; b < nb; b++) {
+      for (int r = b * kBlock, end = std::min(N - r, kBlock) + r; r < end; r++) {
+        row_neighbours(r, nptr, nelem, connPtr, conn, buf);
+        len[(size_t)r + 1] = (int64_t)buf.size();
+        part[b].insert(part[b].end(), buf.begin(), buf.end());
+      }
+    }
+  }
+  for (int r = 0; r < N; r++) len[r + 1] += len[r];
+  hp.nnzb = len[N];
+  if (hp.nnzb > INT_MAX)
+    return fail(FEM_ERR_OVERFLOW, "nnzb = %lld does not fit int32 row pointers", (long long)hp.nnzb);
+  hp.rowp.assign(len.begin(), len.end());
+  hp.cols.resize((size_t)hp.nnzb);
+#pragma omp parallel for schedule(dynamic, 1)
+  for (int b = 0; b < nb; b++) {
+    std::copy(part[b].begin(), part[b].end(), hp.cols.begin() + len[(size_t)b * kBlock]);
+    std::vector<int>().swap(part[b]);
+  }
+  return FEM_SUCCESS;
+}
+
 int colour_greedy(int numNodes, const int *connPtr, const int *conn, int numElements, int *colour,
                   int *numColours) {
   if (!colour || !numColours) return fail(FEM_ERR_INVALID_ARGUMENT, "colour/numColours is NULL");
@@ -248,7 +286,9 @@ static int strip_length(const std::vector<int> &chainPtr, const std::vector<int>
 
 // Strip layout (HostPlan::strips ...), left empty when the mesh's chains are short, meet
 // themselves, or need more than 64 colours.
-static void build_strip_plan(const int *connPtr, const int *conn, const std::vector<int> &right, HostPlan &hp) {
+// at: the elements' positions in the colour layout, whose codes hold the blocks' ranks.
+static void build_strip_plan(const int *connPtr, const int *conn, const std::vector<int> &right,
+                             const std::vector<int> &at, HostPlan &hp) {
   const int P = hp.order, P1 = P + 1, nn = hp.nn, nE = hp.numElements;
   if (P != kStripOrder || nE == 0) return;
   // chains of right neighbours (an element is the right neighbour of one at most)
@@ -315,7 +355,7 @@ static void build_strip_plan(const int *connPtr, const int *conn, const std::vec
   for (int c = 0; c < nc; c++) {
     const std::vector<int> &chains = byColour[c];
     // the chains of one colour share no node, hence no block
-#pragma omp parallel for schedule(dynamic, 1)
+#pragma omp parallel for schedule(static)
     for (int64_t y = 0; y < (int64_t)chains.size(); y++) {
       for (int x = stripPtr[chains[y]]; x < stripPtr[chains[y] + 1]; x++) {
         const dev::Strip &st = strips[x];
@@ -325,17 +365,18 @@ static void build_strip_plan(const int *connPtr, const int *conn, const std::vec
           if ((st.flags & dev::kHalo) && k == st.begin) continue;
           const bool give = k + 1 < st.begin + st.count || (st.flags & dev::kRight);
           uint8_t *rec = &hp.stripCode[(size_t)k * hp.codeStride];
+          const uint8_t *ranks = &hp.blockCode[(size_t)at[listed[k]] * hp.codeStride];
           for (int a = 0; a < nn; a++) {
             const int r = en[a];
             const bool ra = give && a % P1 == P;
             rec[nn * nn + a] = nodeWritten[r] ? 0 : 1;
             if (!ra) nodeWritten[r] = 1;
-            const int *c0 = hp.cols.data() + hp.rowp[r], *c1 = hp.cols.data() + hp.rowp[r + 1];
+            uint8_t *row = &blockWritten[(size_t)hp.rowp[r]];
             for (int b = 0; b < nn; b++) {
-              const int *pos = std::lower_bound(c0, c1, en[b]);  // present: the colour layout found it
-              uint8_t &bf = blockWritten[(size_t)(pos - hp.cols.data())];
+              const int rank = ranks[a * nn + b] & 0x7f;
+              uint8_t &bf = row[rank];
               const bool rb = ra && b % P1 == P;
-              rec[a * nn + b] = (uint8_t)((pos - c0) | (rb || !bf ? 0x80 : 0));
+              rec[a * nn + b] = (uint8_t)(rank | (rb || !bf ? 0x80 : 0));
               if (!rb) bf = 1;
             }
           }
@@ -369,7 +410,8 @@ static void build_strip_plan(const int *connPtr, const int *conn, const std::vec
 // layout; codes are computed per colour with the units in parallel (they share no
 // node) and the two elements of a pair in order.  Leaves the layout empty when
 // the units need more than 64 colours.
-static void build_pair_plan(const int *connPtr, const int *conn, const std::vector<int> &right, HostPlan &hp) {
+static void build_pair_plan(const int *connPtr, const int *conn, const std::vector<int> &right,
+                            const std::vector<int> &at, HostPlan &hp) {
   const bool tables = hp.numStripColours == 0;  // else the counts alone
   const int nn = hp.nn, nE = hp.numElements;
   std::vector<int> partner((size_t)nE, -1);
@@ -408,6 +450,9 @@ static void build_pair_plan(const int *connPtr, const int *conn, const std::vect
     (partner[unitLead[u]] >= 0 ? pairsOf : singlesOf)[unitColour[u]]++;
   hp.pairColourPtr.assign((size_t)nc + 1, 0);
   for (int c = 0; c < nc; c++) hp.pairColourPtr[c + 1] = hp.pairColourPtr[c] + (int)(2 * pairsOf[c] + singlesOf[c]);
+  hp.numPairColours = nc;
+  for (int c = 0; c < nc; c++) hp.numPairs += pairsOf[c];
+  if (!tables) return;
   hp.pairList.assign((size_t)nE, -1);
   std::vector<int64_t> fillP((size_t)nc), fillS((size_t)nc);
   for (int c = 0; c < nc; c++) {
@@ -427,9 +472,6 @@ static void build_pair_plan(const int *connPtr, const int *conn, const std::vect
       hp.pairList[fillS[c]++] = e;
     }
   }
-  hp.numPairColours = nc;
-  for (int c = 0; c < nc; c++) hp.numPairs += pairsOf[c];
-  if (!tables) return;
   hp.pairConnList.resize((size_t)nE * nn);
   hp.pairCode.assign((size_t)nE * hp.codeStride, 0);
   std::vector<uint8_t> blockWritten((size_t)hp.nnzb, 0), nodeWritten((size_t)hp.numNodes, 0);
@@ -449,16 +491,17 @@ static void build_pair_plan(const int *connPtr, const int *conn, const std::vect
         const int *en = conn + connPtr[e];
         int *cl = &hp.pairConnList[(size_t)k * nn];
         uint8_t *rec = &hp.pairCode[(size_t)k * hp.codeStride];
+        const uint8_t *ranks = &hp.blockCode[(size_t)at[e] * hp.codeStride];
         for (int a = 0; a < nn; a++) cl[a] = en[a];
         for (int a = 0; a < nn; a++) {
           const int r = en[a];
           rec[nn * nn + a] = nodeWritten[r] ? 0 : 1;
           nodeWritten[r] = 1;
-          const int *c0 = hp.cols.data() + hp.rowp[r], *c1 = hp.cols.data() + hp.rowp[r + 1];
+          uint8_t *row = &blockWritten[(size_t)hp.rowp[r]];
           for (int b = 0; b < nn; b++) {
-            const int *pos = std::lower_bound(c0, c1, en[b]);  // present: the colour layout found it
-            uint8_t &bf = blockWritten[(size_t)(pos - hp.cols.data())];
-            rec[a * nn + b] = (uint8_t)((pos - c0) | (bf ? 0 : 0x80));
+            const int rank = ranks[a * nn + b] & 0x7f;
+            uint8_t &bf = row[rank];
+            rec[a * nn + b] = (uint8_t)(rank | (bf ? 0 : 0x80));
             bf = 1;
           }
         }
@@ -482,11 +525,7 @@ int build_host_plan(int order, int numNodes, const int *connPtr, const int *conn
   hp.nn = nn;
   hp.numNodes = numNodes;
   hp.numElements = numElements;
-  hp.rowp.resize((size_t)numNodes + 1);
-  st = build_pattern(numNodes, connPtr, conn, numElements, hp.rowp.data(), nullptr, &hp.nnzb);
-  if (st) return st;
-  hp.cols.resize((size_t)hp.nnzb);
-  st = build_pattern(numNodes, connPtr, conn, numElements, hp.rowp.data(), hp.cols.data(), &hp.nnzb);
+  st = build_pattern_once(hp, connPtr, conn);
   if (st) return st;
 
   std::vector<int> colour((size_t)numElements);
@@ -540,8 +579,10 @@ int build_host_plan(int order, int numNodes, const int *connPtr, const int *conn
   if (order >= 2) {
     std::vector<int> right;
     right_neighbours(connPtr, conn, hp, right);
-    if (strips) build_strip_plan(connPtr, conn, right, hp);
-    build_pair_plan(connPtr, conn, right, hp);
+    std::vector<int> at((size_t)numElements);
+    for (int k = 0; k < numElements; k++) at[hp.elemList[k]] = k;
+    if (strips) build_strip_plan(connPtr, conn, right, at, hp);
+    build_pair_plan(connPtr, conn, right, at, hp);
   }
   return FEM_SUCCESS;
 }
