@@ -62,12 +62,12 @@ def make_mesh(mesh_mod, name):
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per assembly from ncu
 # captures, keyed by workload, kernel label prefix and element layout.  The 1024^2
-# order-3 figures are the sums over the four colour launches of the 512^2 case
-# (colour layout 2.835 GB, the FP64 and BF16x6 kernels moving the same bytes; pair
-# layout 2.592 GB) times 4: traffic grows with the element count.
+# order-3 figures are the sums over the colour launches of the 512^2 case (colour
+# layout 2.835 GB in four, strips 2.360 GB in two; the FP64 and BF16x6 kernels move the
+# same bytes) times 4: traffic grows with the element count.
 MEASURED_TRAFFIC = {
     ("square1024_p3", "frag_kernel<3", "colours"): 4 * 2.835e9,
-    ("square1024_p3", "frag_kernel<3>", "pairs"): 4 * 2.5917e9,
+    ("square1024_p3", "frag_kernel<3", "strips"): 4 * 2.3603e9,
 }
 
 
@@ -410,8 +410,8 @@ def run_ours(args):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                      "traffic": traffic, "peak_kind": peak_kind, "algorithmic_bytes_per_step": abytes, "kernel": label,
                      "traffic_note": ("DRAM bytes per step (all colour launches of one assembly) from an ncu capture "
-                                      "of the 512^2 order-3 mesh scaled x4; above the algorithmic bytes: later "
-                                      "colours' bulk reductions read the blocks an earlier colour stored"
+                                      "of the 512^2 order-3 mesh scaled x4; above the algorithmic bytes: the "
+                                      "later colour's bulk reductions read the blocks the earlier one stored"
                                       if traffic else "no ncu capture for this workload")},
         "gpu_launches": launches,
         "clocks": clk.summary(),
@@ -524,6 +524,8 @@ def kernel_label(plan, order, prec):
     # order 4 in FP64; FP32 order 4 runs the element kernel
     n = plan.launches(precision=prec)
     lay = plan.layout()[0]
+    if order == 3 and lay == "pairs" and plan.strips()[0]:
+        lay = "strips"
     if order == 3 and prec == "mixed":
         return f"frag_kernel<{order}, BF16x6 stiffness> x {n} colour launches per step ({lay} layout)"
     if order in (2, 3) or (order == 4 and prec == "fp64"):
