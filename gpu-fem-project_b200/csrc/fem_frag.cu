@@ -1649,9 +1649,13 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
         // and the exact transpose); then the row and column of node XN: of the two slots of
         // xs, lanes t/2 = x take slot x, t even (XN, a), t odd its transpose.  First stores
         // go out at once, the blocks to add are staged and leave FL at a time after one
-        // proxy fence, as one bulk group, from two halves of the lane's slots in turn.
+        // proxy fence, as one bulk group.  Fewer fences and groups, against waiting for the
+        // group before: order 4 takes all four slots at a time (256^2 486 us; two from each
+        // half of the slots in turn 503), order 2 an element's three (512 x 2048 annulus 1178
+        // us, from two sets of slots in turn 1184), its NONLINEAR blocks two (500 x 512 770 us,
+        // four 808).
         if constexpr (JAC && EX && PLAN) {
-          constexpr int FL = P == 2 && !NL ? 3 : 2, HALF = FL == 2 ? 2 : 0;
+          constexpr int FL = P == 4 ? 4 : (NL ? 2 : 3), HALF = FL == 2 ? 2 : 0;
           double *reds = redsW + 4 * lane;
           double *dst[FL];
           bool add[FL];
