@@ -53,8 +53,9 @@ struct HostPlan {
   // Order 1, row assembly (each block row written once by the warp that owns it):
   // rowElemPtr[numNodes+1] indexes rowElem, two ints per (node r, element k listing
   // r): {k << 2 | a (local index of r), ranks of the element's four nodes in row r,
-  // one byte each, | 0x80 in the row's first entry with that block}; rowChunk[numChunks+1] cuts the rows into chunks of at most
-  // kRowChunkRows rows and kRowChunkBlocks blocks.  Empty when not applicable.
+  // one byte each, | 0x80 in the row's first entry with that block}; rowChunk[numChunks+1]
+  // cuts the rows into chunks of at most kRowChunkRows rows and kRowChunkBlocks blocks.
+  // Empty when not applicable.
   std::vector<int> rowElemPtr, rowElem, rowChunk;
   // Orders 2-4, pair layout of the fragment kernel's single-mesh assembly: elements
   // paired with the neighbour across their right edge (its left edge, node for

@@ -41,8 +41,8 @@
 //                two passes of twelve accumulator tiles (an earlier form, 28 tiles of
 //                interleaved rows r = 2a + i in five groups, formed 19 instead of 5
 //                fragment pairs per k-step and exchanged the two rows of every block
-//                between lanes: 256^2 703 -> 507 us; the same at two CTAs per SM and 255
-//                registers: 537 us).  Blocks above the diagonal are also written
+//                between lanes: 256^2 703 -> 507 us, now 486; the same at two CTAs per SM
+//                and 255 registers: 537 against 507 us).  Blocks above the diagonal are also written
 //                transposed.
 //
 // Writes.  Plan mode: a launch is one colour; the first contributor of a block
@@ -1821,7 +1821,7 @@ __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB)
 // order-3 assembly is bound by its writes: a probe that stores every block once at its
 // real address took 568 us for 512^2 in the pair layout's order (four colours, x-neighbours
 // written in different launches: lines leave L2 half written), 466 us with each element row
-// in one launch (linear fill: 378-400).  512^2: 668 -> 576 us, 1024^2 2.63 -> 2.21 ms.
+// in one launch (linear fill: 378-400).  512^2: 668 -> 537 us, 1024^2 2.63 -> 2.18 ms.
 template <int P, int MODE>
 __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB)
     frag_strip_kernel(const __grid_constant__ AsmArgs A, const __grid_constant__ RangeList R,

@@ -361,7 +361,7 @@ int build_schedule(fem_plan *p, int band, int tile) {
 
 // How the fragment kernel's single-mesh launches run a plan in its pair layout.  A plan
 // with a strip layout runs the LINEAR Jacobian by strips (order 3, us, before / strips:
-// 1024^2 2630 / 2210, 515 x 509 MIXED 698 / 640) and the rest by the element colours:
+// 1024^2 2630 / 2180, 515 x 509 MIXED 698 / 636) and the rest by the element colours:
 // NONLINEAR strain and the residual alone are bound by their arithmetic, which a strip's
 // halo adds to (400 x 397 NONLINEAR: 707 colours, 710 pairs, 789 strips; 600 x 590
 // residual: 249, 248, 281).  The other plans run their pairs.
