@@ -811,6 +811,10 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
   double *redsW = reinterpret_cast<double *>(ws + L::REDS);  // staging slot s at redsW + 128 s
   double *ATs = reinterpret_cast<double *>(ws + L::AT);      // NONLINEAR tangent
   double crx = 0.0, cry = 0.0;                               // strips: carried residual rows
+  // order 2, NONLINEAR: half of the lane's staging slots that the next blocks use.  It
+  // turns with every bulk group and is kept from step to step, so the one group that a
+  // put's wait leaves unfinished always reads the other half.
+  [[maybe_unused]] int half = 0;
 
   // Mesh arguments are read through `mtab` (for one mesh, a pointer to the kernel
   // parameter).  At p = 4 it is laundered once per step: the compiler then reloads
@@ -1216,7 +1220,6 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
       auto col_node = [&](int T, int h) {
         return !PERM ? 8 * T + 4 * h + t : T == 2 ? (h ? 5 * t + 4 : 20 + t) : 5 * (2 * T + h) + t;
       };
-      int half = 0;  // orders 2 and 4: half of the lane's staging slots the next blocks use
       for (int el = 0; el < ne; el++) {
         // Strips: the blocks of an edge's nodes among themselves and their residual rows
         // belong to the element right of it; lanes (g = 6, 7; t = 3) hold exactly those
