@@ -245,9 +245,10 @@ __host__ __device__ __forceinline__ uint32_t drop_run(int pass, int i) {
 
 // Drop-in: the blocks staged from `src` on are added at map offsets m[0..3] (n = 1 or 4
 // of them), each maximal stretch of blocks adjacent in the matrix with one reduction;
-// FP64 atomics where the matrix is not 16-byte aligned.  n = 0: none.
+// FP64 atomics where a block is not 16-byte aligned (the matrix is not, or the caller's map
+// has an odd offset).  n = 0: none.
 __device__ __forceinline__ void drop_issue(double *mat, const int (&m)[4], int n, const double *src) {
-  if ((reinterpret_cast<uintptr_t>(mat) & 15u) != 0) {
+  if (((reinterpret_cast<uintptr_t>(mat) | 8u * (unsigned)(m[0] | m[1] | m[2] | m[3])) & 15u) != 0) {
     for (int j = 0; j < n; j++)
       for (int c = 0; c < 4; c++) atomicAdd(mat + m[j] + c, src[4 * j + c]);
     return;
