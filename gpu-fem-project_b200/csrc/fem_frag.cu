@@ -523,7 +523,8 @@ __device__ __forceinline__ bool frag_put_block(const Out &O, int el, int r0, int
                "@s st.shared.v2.f64 [%1], {%2, %3};\n\t"
                "@s st.shared.v2.f64 [%1 + 16], {%4, %5};\n\t}" ::"l"(blk),
                "r"((unsigned)__cvta_generic_to_shared(slot)), "d"(v0), "d"(v1), "d"(v2), "d"(v3),
-               "r"(act ? first : 0u), "r"((uint32_t)add));
+               "r"(act ? first : 0u), "r"((uint32_t)add)
+               : "memory");
   return add;
 }
 
