@@ -99,6 +99,21 @@ bool umma_order4() {
   return on;
 }
 
+// Drop-in order-4 Jacobians (FP64, LINEAR) of few elements: the element kernel.  Its time
+// grows with the elements (12 us, then about 16 us per W = 1184, the fragment kernel's
+// resident warps); the fragment kernel's grows by steps, one element per warp up to W, then
+// two at a time, each about 16 us (23 us for any mesh up to W: two passes of twelve
+// accumulator tiles and 1250 staged blocks per warp).  So the fragment kernel is taken where its last step is full
+// enough; both kernels, us (element / fragment): 64 elements 12.1 / 22.6, 900 22.6 / 25.0,
+// 1156 26.7 / 25.7, 1600 32.8 / 39.0, 2304 42.8 / 39.0, 3136 53.9 / 63.6, 4096 67.9 / 67.6,
+// 5184 84.4 / 90.3, 5776 97.8 / 94.6, 8100 145 / 122.
+static bool dropin_element_kernel(int order, int mode, int64_t elements) {
+  constexpr int64_t W = 148 * 8;
+  if (order != 4 || !(mode & dev::kJac)) return false;
+  const int64_t steps = elements <= W ? 1 : 2 * ((elements + 2 * W - 1) / (2 * W));
+  return 32 * (steps * W - elements) > steps * steps * W;
+}
+
 int launch(int order, int precision, int mode, const dev::AsmArgs &a, cudaStream_t s, int strain) {
   if (strain == FEM_STRAIN_NONLINEAR) {
     if (precision != FEM_PRECISION_FP64)
@@ -108,7 +123,7 @@ int launch(int order, int precision, int mode, const dev::AsmArgs &a, cudaStream
     return launch_nl(order, mode, a, s);
   }
   if (strain != FEM_STRAIN_LINEAR) return fail(FEM_ERR_INVALID_ARGUMENT, "strain type %d", strain);
-  if ((mode & dev::kPlan) == 0 && frag_supported(order, precision, strain))
+  if ((mode & dev::kPlan) == 0 && frag_supported(order, precision, strain) && !dropin_element_kernel(order, mode, a.count))
     return launch_frag(order, precision, mode, a, s);
   if (precision == FEM_PRECISION_FP64) return launch_any<double>(order, mode, a, s);
   if (precision == FEM_PRECISION_MIXED && order == 4 && (mode & dev::kJac) && umma_order4()) {
