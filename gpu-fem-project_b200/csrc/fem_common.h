@@ -69,8 +69,8 @@ struct HostPlan {
   std::vector<int> pairColourPtr, pairList, pairConnList;
   std::vector<int> pairRegionEnd;  // per colour: the end of its pairs (its unpaired elements follow)
   std::vector<uint8_t> pairCode;
-  // Order kStripOrder: strip layout (LINEAR Jacobians, in the pair layout's place; the
-  // pair tables are then left out).  Chains of right neighbours are coloured so that the
+  // Order kStripOrder: strip layout (LINEAR Jacobians, in the pair layout's place; up to
+  // kStripColours colours the pair tables are then left out).  Chains of right neighbours are coloured so that the
   // chains of one colour share no node and cut into strips.  The blocks of an edge's nodes among
   // themselves and their residual rows belong to the element right of the edge; a strip
   // that does not begin its chain lists the element before it first, as a halo whose
@@ -86,6 +86,17 @@ struct HostPlan {
 constexpr int kPairMinElements = 4 * 148 * 12;  // four colours of one element per resident warp
 constexpr int kStripOrder = 3;
 constexpr int kStripWarps = 148 * 12;  // resident warps of the strip kernel
+// Strips against pairs, by the colours of the chains (order 3, us, strips / pairs).  Up to
+// three (the rows of a grid, in any numbering, or of a ring) strips win at every size: 64^2
+// 27 / 29, 128^2 49 / 67, 256^2 160 / 183, 512^2 537 / 704, eight wide 59 / 67, MIXED 512^2
+// 633 / 669.  Chains that cross (blocks with turned axes, turned elements) need four to
+// seven, and their launches are smaller: strips lose up to about 440^2 (four blocks with
+// crossed axes 128^2 95 / 76, 400^2 456 / 422; blocks of 8 256^2 255 / 194, 430^2 511 / 480) and win
+// beyond in FP64 (470^2: crossed 577 / 627, blocks of 8, 20, 64 575 / 604, 598 / 603, 581 / 604, with 2
+// and 10 % of the elements turned 569 / 593, 600 / 620; 700^2: 1172 / 1318, 1196 / 1314, 1193 / 1312,
+// 1174 / 1311, 1129 / 1276, 1232 / 1330), not in MIXED (512^2 833 / 760, 758 / 735), which runs the pairs.
+// Strips longer than kStripCrossedLength lose there (blocks of 20: 470^2 707 us with 19).
+constexpr int kStripColours = 3, kStripColoursLarge = 7, kStripLargeElements = 210000, kStripCrossedLength = 7;
 constexpr int kRowChunkRows = 32, kRowChunkBlocks = 320;
 int build_host_plan(int order, int numNodes, const int *connPtr, const int *conn, int numElements, HostPlan &hp,
                     bool strips = true);

@@ -267,7 +267,7 @@ static int strip_length(const std::vector<int> &chainPtr, const std::vector<int>
   int best = 1;
   double cost = 1e300;
   std::vector<int64_t> strips((size_t)nc);
-  for (int n = 1; n <= 31; n += 2) {
+  for (int n = 1; n <= (nc > kStripColours ? kStripCrossedLength : 31); n += 2) {
     std::fill(strips.begin(), strips.end(), 0);
     for (size_t i = 0; i < colour.size(); i++)  // a chain's first strip takes n + 1
       strips[colour[i]] += std::max(1, (chainPtr[i + 1] - chainPtr[i] - 1 + n - 1) / n);
@@ -285,7 +285,7 @@ static int strip_length(const std::vector<int> &chainPtr, const std::vector<int>
 }
 
 // Strip layout (HostPlan::strips ...), left empty when the mesh's chains are short, meet
-// themselves, or need more than 64 colours.
+// themselves, or need more colours than strips pay for (kStripColours).
 // at: the elements' positions in the colour layout, whose codes hold the blocks' ranks.
 static void build_strip_plan(const int *connPtr, const int *conn, const std::vector<int> &right,
                              const std::vector<int> &at, HostPlan &hp) {
@@ -330,6 +330,7 @@ static void build_strip_plan(const int *connPtr, const int *conn, const std::vec
     for (int k = chainPtr[i]; k < chainPtr[i + 1]; k++)
       for (int a = 0; a < nn; a++) used[conn[connPtr[chain[k]] + a]] |= 1ull << colour[i];
   }
+  if (nc > kStripColours && (nc > kStripColoursLarge || nE < kStripLargeElements)) return;
   // strips, chain by chain: the first of a chain has no halo and takes one element more
   const int len = strip_length(chainPtr, colour, nc);
   std::vector<int> stripPtr(1, 0), chainOf;
@@ -412,7 +413,7 @@ static void build_strip_plan(const int *connPtr, const int *conn, const std::vec
 // the units need more than 64 colours.
 static void build_pair_plan(const int *connPtr, const int *conn, const std::vector<int> &right,
                             const std::vector<int> &at, HostPlan &hp) {
-  const bool tables = hp.numStripColours == 0;  // else the counts alone
+  const bool tables = hp.numStripColours == 0 || hp.numStripColours > kStripColours;  // else the counts alone
   const int nn = hp.nn, nE = hp.numElements;
   std::vector<int> partner((size_t)nE, -1);
   std::vector<char> lead((size_t)nE, 0);

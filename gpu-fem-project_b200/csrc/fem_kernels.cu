@@ -376,16 +376,20 @@ int build_schedule(fem_plan *p, int band, int tile) {
 
 // How the fragment kernel's single-mesh launches run a plan in its pair layout.  A plan
 // with a strip layout runs the LINEAR Jacobian by strips (order 3, us, before / strips:
-// 1024^2 2630 / 2180, 515 x 509 MIXED 698 / 636) and the rest by the element colours:
+// 1024^2 2630 / 2180, 515 x 509 MIXED 698 / 636; the rule at kStripColours) and the rest by
+// its pairs where it has their tables, else by the element colours:
 // NONLINEAR strain and the residual alone are bound by their arithmetic, which a strip's
-// halo adds to (400 x 397 NONLINEAR: 707 colours, 710 pairs, 789 strips; 600 x 590
-// residual: 249, 248, 281).  The other plans run their pairs.
-bool plan_strips(const fem_plan *p, int strain, bool jacobian) {
-  return p->usePairs && p->numStripColours > 0 && strain == FEM_STRAIN_LINEAR && jacobian;
+// halo adds to (400 x 397 NONLINEAR: 707 colours, 710 pairs, 789 strips when a halo took a
+// whole element's products; 600 x 590 residual: 249, 248, 281).  The other plans run their
+// pairs.
+bool plan_strips(const fem_plan *p, int precision, int strain, bool jacobian) {
+  return p->usePairs && p->numStripColours > 0 && strain == FEM_STRAIN_LINEAR && jacobian &&
+         (precision == FEM_PRECISION_FP64 || p->numStripColours <= fem::kStripColours);
 }
-// Small plans run the colours too: each element of a launch then has a warp of its own.
+// Asked after plan_strips.  Small plans run the colours: each element of a launch then has
+// a warp of its own.
 bool plan_pairs(const fem_plan *p) {
-  return p->usePairs && p->numPairColours > 0 && p->numStripColours == 0 && p->numElements > fem::kPairMinElements;
+  return p->usePairs && p->d_pairCode && p->numElements > fem::kPairMinElements;
 }
 
 // Whether fem_plan_assemble runs `p` as one dependency-ordered launch.
@@ -512,10 +516,8 @@ int fem_plan_create(int elementOrder, int numNodes, const int *connPtr, const in
     p->stripLead.resize(hp.strips.size());
     for (size_t x = 0; x < hp.strips.size(); x++) p->stripLead[x] = hp.strips[x].lead;
     p->numStripColours = hp.numStripColours;
-    p->numPairColours = hp.numPairColours;
-    p->numPairs = hp.numPairs;
-    p->usePairs = hp.numPairColours > 0;
-  } else if (hp.numPairColours > 0) {
+  }
+  if (!hp.pairCode.empty()) {
     if ((st = upload(hp.pairConnList, &p->d_pairConnList, p->deviceBytes)) ||
         (st = upload(hp.pairCode, &p->d_pairCode, p->deviceBytes))) {
       plan_free(p);
@@ -531,10 +533,10 @@ int fem_plan_create(int elementOrder, int numNodes, const int *connPtr, const in
       p->pairNodeLo[k] = *std::min_element(c, c + hp.nn);
       p->pairNodeHi[k] = *std::max_element(c, c + hp.nn);
     }
-    p->numPairColours = hp.numPairColours;
-    p->numPairs = hp.numPairs;
-    p->usePairs = true;
   }
+  p->numPairColours = hp.numPairColours;
+  p->numPairs = hp.numPairs;
+  p->usePairs = hp.numPairColours > 0 || hp.numStripColours > 0;
   if ((st = fem::uploads_visible("fem_plan_create: table upload"))) {
     plan_free(p);
     return st;
@@ -718,7 +720,7 @@ int fem_plan_assemble_ex(const fem_plan *plan, const double *states, const doubl
   }
   // the fragment kernel runs the pair layout (a step's two elements share an edge,
   // so the lines of the rows they share are written while they are still in L2)
-  if (frag && plan_strips(plan, strainType, matEntries != nullptr)) {
+  if (frag && plan_strips(plan, precision, strainType, matEntries != nullptr)) {
     a.connList = plan->d_stripConn;
     a.blockCode = plan->d_stripCode;
     return fem::timed(s, elapsedSeconds, [&] {
@@ -755,7 +757,7 @@ int fem_plan_set_layout(fem_plan *plan, int layout) {
   if (!plan) return fem::fail(FEM_ERR_INVALID_ARGUMENT, "plan is NULL");
   if (layout != FEM_LAYOUT_COLOURS && layout != FEM_LAYOUT_PAIRS)
     return fem::fail(FEM_ERR_INVALID_ARGUMENT, "layout %d", layout);
-  if (layout == FEM_LAYOUT_PAIRS && plan->numPairColours == 0)
+  if (layout == FEM_LAYOUT_PAIRS && plan->numPairColours == 0 && plan->numStripColours == 0)
     return fem::fail(FEM_ERR_UNSUPPORTED, "this plan has no pair layout (order 1, or its pairs need > 64 colours)");
   plan->usePairs = layout == FEM_LAYOUT_PAIRS;
   return FEM_SUCCESS;
@@ -766,7 +768,7 @@ int fem_plan_launches(const fem_plan *plan, int precision, int strainType, int *
   if (!plan || !launches) return fem::fail(FEM_ERR_INVALID_ARGUMENT, "NULL argument");
   const bool frag = fem::frag_supported(plan->order, precision, strainType);
   if ((fem::plan_rows(plan) && strainType == FEM_STRAIN_LINEAR) || plan_sched(plan, precision, strainType)) *launches = 1;
-  else if (frag && plan_strips(plan, strainType, /*jacobian=*/true)) *launches = plan->numStripColours;
+  else if (frag && plan_strips(plan, precision, strainType, /*jacobian=*/true)) *launches = plan->numStripColours;
   else if (frag && plan_pairs(plan)) *launches = plan->numPairColours;
   else *launches = plan->numColours;
   return FEM_SUCCESS;
@@ -826,7 +828,7 @@ int fem_plan_assemble_host(const fem_plan *plan, const double *hostStates, doubl
   const bool rows = fem::plan_rows(plan) && strainType == FEM_STRAIN_LINEAR;
   // the fragment kernel runs the pair layout when the plan uses it (each band's pairs
   // and unpaired elements are two ranges of a colour), else the colour layout
-  const bool strips = frag && !rows && plan_strips(plan, strainType, matEntries != nullptr);
+  const bool strips = frag && !rows && plan_strips(plan, precision, strainType, matEntries != nullptr);
   const bool pairs = frag && !rows && !strips && plan_pairs(plan);
   const int N = plan->numNodes, nE = plan->numElements;
   const int nc = strips ? plan->numStripColours : pairs ? plan->numPairColours : plan->numColours;
