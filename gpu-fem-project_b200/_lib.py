@@ -71,6 +71,7 @@ SIGNATURES = {
     "fem_plan_set_layout": (_i, [_p, _i]),
     "fem_plan_get_layout": (_i, [_p, _pi, _pi64, _pi]),
     "fem_plan_launches": (_i, [_p, _i, _i, _pi]),
+    "fem_plan_get_path": (_i, [_p, _i, _i, _i, _pi]),
     "fem_plan_get_strips": (_i, [_p, _pi, _pi]),
     "fem_plan_assemble_ex": (_i, [_p, _p, _p, _d, _d, _d, _p, _p, _i, _i, _p, _pd]),
     "fem_plan_assemble_host": (_i, [_p, _p, _p, _p, _d, _d, _d, _p, _p, _p, _i, _i, _i, _p, _pd]),

@@ -197,6 +197,13 @@ class Plan:
         check(lib.fem_plan_launches(self._h, _prec(precision), _strain(strain), C.byref(n)), "fem_plan_launches")
         return n.value
 
+    def path(self, strain="linear", precision="fp64", jacobian=True) -> str:
+        """What assemble() runs: 'rows', 'ordered', 'strips', 'pairs' or 'colours'."""
+        n = C.c_int()
+        check(lib.fem_plan_get_path(self._h, _prec(precision), _strain(strain), int(jacobian), C.byref(n)),
+              "fem_plan_get_path")
+        return ("colours", "pairs", "strips", "ordered", "rows")[n.value]
+
     def strips(self):
         """(strips, strip colours) of an order-3 plan's LINEAR Jacobian; (0, 0): none."""
         n, c = C.c_int(), C.c_int()
@@ -243,12 +250,12 @@ class Plan:
 
     def set_layout(self, layout):
         """'pairs' (default where built) or 'colours': the element order of the
-        fragment kernel's single-mesh colour launches."""
+        fragment kernel's single-mesh colour launches (what 'pairs' runs: path())."""
         code = {"colours": _lib.FEM_LAYOUT_COLOURS, "pairs": _lib.FEM_LAYOUT_PAIRS}[layout]
         check(lib.fem_plan_set_layout(self._h, code), "fem_plan_set_layout")
 
     def layout(self):
-        """(layout name, pairs formed, pair colours)."""
+        """(layout name as set, pairs formed, pair colours); path() says what runs."""
         lay, npairs, ncol = C.c_int(), C.c_int64(), C.c_int()
         check(lib.fem_plan_get_layout(self._h, C.byref(lay), C.byref(npairs), C.byref(ncol)), "fem_plan_get_layout")
         return ("pairs" if lay.value == _lib.FEM_LAYOUT_PAIRS else "colours"), npairs.value, ncol.value

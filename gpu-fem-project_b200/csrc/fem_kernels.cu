@@ -397,6 +397,14 @@ bool plan_sched(const fem_plan *p, int precision, int strain) {
   return p->schedGroups > 0 && fem::frag_supported(p->order, precision, strain) &&
          !(fem::plan_rows(p) && strain == FEM_STRAIN_LINEAR);
 }
+
+// What fem_plan_assemble runs.
+int plan_path(const fem_plan *p, int precision, int strain, bool jacobian) {
+  if (fem::plan_rows(p) && strain == FEM_STRAIN_LINEAR) return FEM_PATH_ROWS;
+  if (plan_sched(p, precision, strain)) return FEM_PATH_ORDERED;
+  if (!fem::frag_supported(p->order, precision, strain)) return FEM_PATH_COLOURS;
+  return plan_strips(p, precision, strain, jacobian) ? FEM_PATH_STRIPS : plan_pairs(p) ? FEM_PATH_PAIRS : FEM_PATH_COLOURS;
+}
 }  // namespace
 
 extern "C" {
@@ -693,7 +701,8 @@ int fem_plan_assemble_ex(const fem_plan *plan, const double *states, const doubl
   fem::set_material(a, E, nu, t);
   const int mode = fem::dev::kPlan | (residual ? fem::dev::kRes : 0) | (matEntries ? fem::dev::kJac : 0);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (fem::plan_rows(plan) && strainType == FEM_STRAIN_LINEAR) {
+  const int path = plan_path(plan, precision, strainType, matEntries != nullptr);
+  if (path == FEM_PATH_ROWS) {
     // order 1: row assembly (FP64 arithmetic for both precisions)
     if (precision != FEM_PRECISION_FP64 && precision != FEM_PRECISION_MIXED)
       return fem::fail(FEM_ERR_INVALID_ARGUMENT, "precision %d", precision);
@@ -701,8 +710,7 @@ int fem_plan_assemble_ex(const fem_plan *plan, const double *states, const doubl
     a.count = plan->numChunks;
     return fem::timed(s, elapsedSeconds, [&] { return fem::launch_rows(mode, a, s); });
   }
-  const bool frag = fem::frag_supported(plan->order, precision, strainType);
-  if (plan_sched(plan, precision, strainType)) {
+  if (path == FEM_PATH_ORDERED) {
     // all colours in one dependency-ordered launch; the tile dispenser and the
     // per-group counters start at zero, the sticky timeout count (word 0) is kept
     const int st = fem::timed(s, elapsedSeconds, [&]() -> int {
@@ -720,7 +728,7 @@ int fem_plan_assemble_ex(const fem_plan *plan, const double *states, const doubl
   }
   // the fragment kernel runs the pair layout (a step's two elements share an edge,
   // so the lines of the rows they share are written while they are still in L2)
-  if (frag && plan_strips(plan, precision, strainType, matEntries != nullptr)) {
+  if (path == FEM_PATH_STRIPS) {
     a.connList = plan->d_stripConn;
     a.blockCode = plan->d_stripCode;
     return fem::timed(s, elapsedSeconds, [&] {
@@ -733,7 +741,7 @@ int fem_plan_assemble_ex(const fem_plan *plan, const double *states, const doubl
       return (int)FEM_SUCCESS;
     });
   }
-  const bool pairs = frag && plan_pairs(plan);
+  const bool frag = fem::frag_supported(plan->order, precision, strainType), pairs = path == FEM_PATH_PAIRS;
   if (pairs) {
     a.connList = plan->d_pairConnList;
     a.blockCode = plan->d_pairCode;
@@ -766,11 +774,20 @@ int fem_plan_set_layout(fem_plan *plan, int layout) {
 int fem_plan_launches(const fem_plan *plan, int precision, int strainType, int *launches) {
   fem::clear_error();
   if (!plan || !launches) return fem::fail(FEM_ERR_INVALID_ARGUMENT, "NULL argument");
-  const bool frag = fem::frag_supported(plan->order, precision, strainType);
-  if ((fem::plan_rows(plan) && strainType == FEM_STRAIN_LINEAR) || plan_sched(plan, precision, strainType)) *launches = 1;
-  else if (frag && plan_strips(plan, precision, strainType, /*jacobian=*/true)) *launches = plan->numStripColours;
-  else if (frag && plan_pairs(plan)) *launches = plan->numPairColours;
-  else *launches = plan->numColours;
+  switch (plan_path(plan, precision, strainType, /*jacobian=*/true)) {
+    case FEM_PATH_ROWS:
+    case FEM_PATH_ORDERED: *launches = 1; break;
+    case FEM_PATH_STRIPS: *launches = plan->numStripColours; break;
+    case FEM_PATH_PAIRS: *launches = plan->numPairColours; break;
+    default: *launches = plan->numColours;
+  }
+  return FEM_SUCCESS;
+}
+
+int fem_plan_get_path(const fem_plan *plan, int precision, int strainType, int jacobian, int *path) {
+  fem::clear_error();
+  if (!plan || !path) return fem::fail(FEM_ERR_INVALID_ARGUMENT, "NULL argument");
+  *path = plan_path(plan, precision, strainType, jacobian != 0);
   return FEM_SUCCESS;
 }
 

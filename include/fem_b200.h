@@ -175,12 +175,14 @@ int fem_plan_row_chunks(const fem_plan *plan, int *numChunks);
  *                       step, the second element adding to the shared edge's
  *                       blocks the first one stored, so that the rows the two
  *                       share are written while their lines are in L2.  Order-3
- *                       plans whose elements form chains of such neighbours run the
- *                       LINEAR Jacobian (with or without the residual) by strips of
- *                       these chains instead, one launch per colour of the chains
- *                       (fem_plan_get_strips), and everything else by
- *                       FEM_LAYOUT_COLOURS, as do plans of orders 2 and 4 with few
- *                       elements (up to 7104: a warp then takes a single element);
+ *                       plans whose elements form chains of such neighbours in up to
+ *                       three colours (grids, rings; seven in FP64 from 210,000
+ *                       elements on) run the LINEAR Jacobian (with or without the
+ *                       residual) by strips of these chains instead, one launch per
+ *                       colour of the chains (fem_plan_get_strips), and where up to
+ *                       three colours do, everything else by FEM_LAYOUT_COLOURS, as
+ *                       do plans with few elements (up to 7104: a warp then takes a
+ *                       single element); fem_plan_get_path says which;
  *   FEM_LAYOUT_COLOURS  the element colouring above (what every other path runs).
  * The results agree to rounding: a block's contributions are added in another
  * order where more than two elements share it.  fem_plan_get_layout also reports
@@ -190,6 +192,16 @@ int fem_plan_row_chunks(const fem_plan *plan, int *numChunks);
 #define FEM_LAYOUT_PAIRS 1
 int fem_plan_set_layout(fem_plan *plan, int layout);
 int fem_plan_get_layout(const fem_plan *plan, int *layout, int64_t *numPairs, int *numPairColours);
+/* What fem_plan_assemble_ex runs for these arguments (jacobian: whether matEntries is
+ * given): FEM_PATH_ROWS order-1 row assembly; FEM_PATH_ORDERED all colours in one
+ * dependency-ordered launch; FEM_PATH_STRIPS, FEM_PATH_PAIRS, FEM_PATH_COLOURS one launch
+ * per colour of the strips, the pairs, the elements. */
+#define FEM_PATH_COLOURS 0
+#define FEM_PATH_PAIRS 1
+#define FEM_PATH_STRIPS 2
+#define FEM_PATH_ORDERED 3
+#define FEM_PATH_ROWS 4
+int fem_plan_get_path(const fem_plan *plan, int precision, int strainType, int jacobian, int *path);
 /* Kernel launches of one residual + Jacobian fem_plan_assemble_ex of this plan. */
 int fem_plan_launches(const fem_plan *plan, int precision, int strainType, int *launches);
 /* Strips of an order-3 plan and their colours (launches); 0, 0 when it has none. */
