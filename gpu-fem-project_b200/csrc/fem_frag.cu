@@ -1913,18 +1913,7 @@ int launch_frag_p(const AsmArgs &a, cudaStream_t s, bool chained, bool single) {
   // ms on the 512x2048 annulus, so it keeps its occupancy.
   const int perSm =
       (P == 3 && (MODE & kPlan) == 0 && (MODE & kJac) != 0) ? std::min(li.grid_per_sm, 2) : li.grid_per_sm;
-  int64_t cap = (int64_t)perSm * li.num_sms;
-  // Order-3 plan Jacobians (FP64, LINEAR) in the element and pair layouts, launches of
-  // many steps: somewhat fewer than three CTAs per SM, since the stores and reductions of
-  // more warps contend here too (the elements' colours from 8 steps on, 21 CTAs per 8 SMs:
-  // 512^2 790 -> 777 us, 1024^2 3144 -> 3052, 700 x 500 1043 -> 1027; the pairs from 14, 11 per 4:
-  // 512^2 with 5, 10, 15 % of the elements turned 714 -> 698, 740 -> 718, 756 -> 740).  In shorter
-  // launches the longer last wave costs more (colours 256^2 200 -> 212, pairs 362^2 358 ->
-  // 363).  The other forms are bound by their arithmetic (NONLINEAR 1153 us, 2.5 CTAs per SM
-  // 1363; MIXED 776, 835).
-  constexpr bool kContended = P == 3 && (MODE & (kPlan | kJac | kNL | kB16)) == (kPlan | kJac);
-  if (kContended && a.count >= (single ? 8 : 14) * 2 * F::WARPS * cap)
-    cap = (int64_t)li.num_sms * (single ? 21 : 22) / 8;
+  const int64_t cap = (int64_t)perSm * li.num_sms;
   // A launch whose elements all find a warp of their own takes one per warp instead of a
   // pair: the warp's step is what the launch takes, and one element's stiffness and writes
   // are most of half of it (33 x 31 order 4 63.5 -> 38.9 us, order 3 NONLINEAR
