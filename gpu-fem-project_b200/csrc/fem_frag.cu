@@ -1917,8 +1917,10 @@ int launch_frag_p(const AsmArgs &a, cudaStream_t s, bool chained, bool single) {
   // A launch whose elements all find a warp of their own takes one per warp instead of a
   // pair: the warp's step is what the launch takes, and one element's stiffness and writes
   // are most of half of it (33 x 31 order 4 63.5 -> 38.9 us, order 3 NONLINEAR
-  // 44.1 -> 22.6; order 2, bound by its four launches, 18.5 -> 18.4).
-  const int unit = single && a.count <= cap * F::WARPS ? 1 : 2;
+  // 44.1 -> 22.6; order 2, bound by its four launches, 18.5 -> 18.4).  Not the residual
+  // alone, where both elements of a step are rows of the same products (90 x 89 in the
+  // colour layout, order 2 one / two per warp 20.5 / 14.4, order 3 22.0 / 16.4).
+  const int unit = single && (MODE & kJac) != 0 && a.count <= cap * F::WARPS ? 1 : 2;
   const int64_t units = (a.count + unit - 1) / unit;
   const int64_t need = (units + F::WARPS - 1) / F::WARPS;
   const int grid = (int)(need < cap ? need : cap);
