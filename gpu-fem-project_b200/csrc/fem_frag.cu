@@ -243,20 +243,24 @@ __host__ __device__ __forceinline__ uint32_t drop_run(int pass, int i) {
   return 0xffffffffu;
 }
 
-// Drop-in: the blocks staged from `src` on are added at map offsets m[0..3] (n = 1 or 4
-// of them), each maximal stretch of blocks adjacent in the matrix with one reduction;
-// FP64 atomics where a block is not 16-byte aligned (the matrix is not, or the caller's map
-// has an odd offset).  n = 0: none.
-__device__ __forceinline__ void drop_issue(double *mat, const int (&m)[4], int n, const double *src) {
-  if (((reinterpret_cast<uintptr_t>(mat) | 8u * (unsigned)(m[0] | m[1] | m[2] | m[3])) & 15u) != 0) {
-    for (int j = 0; j < n; j++)
-      for (int c = 0; c < 4; c++) atomicAdd(mat + m[j] + c, src[4 * j + c]);
-    return;
-  }
+// Drop-in: the blocks staged from double `src` of redsW on are added at map offsets m[0..3]
+// (n = 0, 1 or 4 of them), each maximal stretch of blocks adjacent in the matrix with one
+// reduction.  The warp adds with FP64 atomics, four lanes to a block, where a block is not
+// 16-byte aligned (the matrix is not, or the caller's map has an odd offset), and where an
+// entry's four blocks are all apart, if that holds for more than half of the warp's
+// entries, as on a mesh numbered at random: four reductions of 32 bytes are slower than
+// that there (order 4 100 x 99 246 / 214 us, 200 x 199 960 / 837; order 2 250 x 249 123 /
+// 107).  A grid's last columns are apart too (8 of 32 entries, order 4): reductions are
+// faster for those (200 x 199 477 / 513 us).
+__device__ __forceinline__ void drop_issue(double *mat, const int (&m)[4], int n, const double *redsW, int src, int lane) {
+  const bool odd = ((reinterpret_cast<uintptr_t>(mat) | 8u * (unsigned)(m[0] | m[1] | m[2] | m[3])) & 15u) != 0;
   const int c1 = n == 4 && m[1] == m[0] + 4, c2 = n == 4 && m[2] == m[1] + 4, c3 = n == 4 && m[3] == m[2] + 4;
-  const int b[4] = {n ? 32 * (1 + c1 * (1 + c2 * (1 + c3))) : 0, n == 4 && !c1 ? 32 * (1 + c2 * (1 + c3)) : 0,
-                    n == 4 && !c2 ? 32 * (1 + c3) : 0, n == 4 && !c3 ? 32 : 0};
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(src);
+  const int joined = __popc(__ballot_sync(0xffffffffu, c1 | c2 | c3)), fours = __popc(__ballot_sync(0xffffffffu, n == 4));
+  const bool single = n > 0 && (odd || (n == 4 && !(c1 | c2 | c3) && 2 * joined < fours));
+  const int k = single ? 0 : n;
+  const int b[4] = {k ? 32 * (1 + c1 * (1 + c2 * (1 + c3))) : 0, k == 4 && !c1 ? 32 * (1 + c2 * (1 + c3)) : 0,
+                    k == 4 && !c2 ? 32 * (1 + c3) : 0, k == 4 && !c3 ? 32 : 0};
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(redsW + src);
 #pragma unroll
   for (int j = 0; j < 4; j++)
     asm volatile("{\n\t.reg .pred p;\n\t"
@@ -264,6 +268,17 @@ __device__ __forceinline__ void drop_issue(double *mat, const int (&m)[4], int n
                  "@p cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f64 [%0], [%1], %2;\n\t}" ::"l"(mat + m[j]),
                  "r"(sa + 32 * j), "r"(b[j])
                  : "memory");
+  if (!__any_sync(0xffffffffu, single)) return;
+#pragma unroll
+  for (int g = 0; g < 4; g++) {  // the entries of lanes 8g .. 8g + 7
+    const int from = 8 * g + (lane >> 2), c = lane & 3;
+    const int count = __shfl_sync(0xffffffffu, single ? n : 0, from), s0 = __shfl_sync(0xffffffffu, src, from);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int off = __shfl_sync(0xffffffffu, m[j], from);
+      if (j < count) atomicAdd(mat + off + c, redsW[s0 + 4 * j + c]);
+    }
+  }
 }
 
 template <int P, int MODE>
@@ -1773,7 +1788,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
 #pragma unroll
               for (int j = 0; j < 4; j++) m[j] = row[j < (int)((e >> 11) & 3) + 1 ? j : 0];
             }
-            drop_issue(O.mat, m, e == 0xffffffffu ? 0 : ((e >> 11) & 3) + 1, redsW + 4 * (e >> 13 & 0x1ff));
+            drop_issue(O.mat, m, e == 0xffffffffu ? 0 : ((e >> 11) & 3) + 1, redsW, 4 * (e >> 13 & 0x1ff), lane);
           }
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
