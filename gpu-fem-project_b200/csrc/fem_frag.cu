@@ -562,15 +562,14 @@ struct PairCursor {
 };
 
 
-// Single mesh: pairs p, p + stride, ... of list positions [begin, end); `unit` 1: single
-// elements (launches that do not fill the GPU).
+// Single mesh: units p, p + stride, ... of list positions [begin, end), `pairs` pairs and
+// then single elements.
 struct PairStride {
   static constexpr bool kBatched = false, kSched = false, kStrip = false;
-  int64_t begin, end, p, stride;
-  int unit;
+  int64_t begin, end, p, stride, pairs;
   __device__ PairCursor next(int) {
-    PairCursor c{0, 0, begin + unit * p};
-    if (c.k0 < end) c.ne = (int)min((int64_t)unit, end - c.k0);
+    PairCursor c{0, 0, begin + p + min(p, pairs)};
+    if (c.k0 < end) c.ne = (int)min((int64_t)(p < pairs ? 2 : 1), end - c.k0);
     p += stride;
     return c;
   }
@@ -1817,12 +1816,12 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
 // drop-in mode, elements [A.begin, A.begin + A.count) through the reference map.
 template <int P, int MODE>
 __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB) frag_kernel(const __grid_constant__ AsmArgs A,
-                                                                                             int unit) {
+                                                                                             int64_t pairs) {
   extern __shared__ __align__(16) unsigned char smem[];
   frag_prologue<P, MODE>(smem);
   const int warp = threadIdx.x >> 5;
   PairStride gen{A.begin, A.begin + A.count, (int64_t)blockIdx.x * FragDims<P>::WARPS + warp,
-                 (int64_t)gridDim.x * FragDims<P>::WARPS, unit};
+                 (int64_t)gridDim.x * FragDims<P>::WARPS, pairs};
   frag_loop<P, MODE>(smem, gen, A, &A);
 }
 
@@ -1932,19 +1931,23 @@ int launch_frag_p(const AsmArgs &a, cudaStream_t s, bool chained, bool single) {
   // A launch whose elements all find a warp of their own takes one per warp instead of a
   // pair: the warp's step is what the launch takes, and one element's stiffness and writes
   // are most of half of it (33 x 31 order 4 63.5 -> 38.9 us, order 3 NONLINEAR
-  // 44.1 -> 22.6; order 2, bound by its four launches, 18.5 -> 18.4).  Not the residual
-  // alone, where both elements of a step are rows of the same products (90 x 89 in the
-  // colour layout, order 2 one / two per warp 20.5 / 14.4, order 3 22.0 / 16.4).
-  const int unit = single && (MODE & kJac) != 0 && a.count <= cap * F::WARPS ? 1 : 2;
-  const int64_t units = (a.count + unit - 1) / unit;
+  // 44.1 -> 22.6; order 2, bound by its four launches, 18.5 -> 18.4), and so does the last
+  // round of the warps as far as its elements go around (order-4 drop-in 90 x 89 128 -> 113
+  // us, order-3 drop-in 80 x 79 34.8 -> 32.8, order-3 NONLINEAR plan 90 x 89 63.5 -> 58.4).
+  // Not the residual alone, where both elements of a step are rows of the same products
+  // (90 x 89 in the colour layout, order 2 one / two per warp 20.5 / 14.4, order 3 22.0 / 16.4).
+  const int64_t per = cap * F::WARPS, left = a.count % (2 * per);
+  const int64_t pairs =
+      single && (MODE & kJac) != 0 ? (a.count - left) / 2 + std::max<int64_t>(left - per, 0) : (a.count + 1) / 2;
+  const int64_t units = std::max(a.count - pairs, pairs);
   const int64_t need = (units + F::WARPS - 1) / F::WARPS;
   const int grid = (int)(need < cap ? need : cap);
   if (grid <= 0) return FEM_SUCCESS;
   cudaError_t err;
   if (chained) {
-    err = pdl_launch(kernel, grid, NT, smem, s, a, unit);
+    err = pdl_launch(kernel, grid, NT, smem, s, a, pairs);
   } else {
-    kernel<<<grid, NT, smem, s>>>(a, unit);
+    kernel<<<grid, NT, smem, s>>>(a, pairs);
     err = cudaGetLastError();
   }
   if (err != cudaSuccess) return cuda_fail(err, "frag_kernel launch");

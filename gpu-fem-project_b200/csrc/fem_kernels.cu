@@ -101,17 +101,21 @@ bool umma_order4() {
 
 // Drop-in order-4 Jacobians (FP64, LINEAR) of few elements: the element kernel.  Its time
 // grows with the elements (12 us, then about 16 us per W = 1184, the fragment kernel's
-// resident warps); the fragment kernel's grows by steps, one element per warp up to W, then
-// two at a time, each about 16 us (23 us for any mesh up to W: two passes of twelve
-// accumulator tiles and 1250 staged blocks per warp).  So the fragment kernel is taken where its last step is full
-// enough; both kernels, us (element / fragment): 64 elements 12.1 / 22.6, 900 22.6 / 25.0,
-// 1156 26.7 / 25.7, 1600 32.8 / 39.0, 2304 42.8 / 39.0, 3136 53.9 / 63.6, 4096 67.9 / 67.6,
-// 5184 84.4 / 90.3, 5776 97.8 / 94.6, 8100 145 / 122.
+// resident warps); the fragment kernel's grows by steps, one element per warp each (23 us
+// for any mesh up to W: two passes of twelve accumulator tiles and 1250 staged blocks per
+// warp).  So the fragment kernel is taken where its last two steps are full enough; both
+// kernels, us (element / fragment), grid numbering: 64 elements 12.4 / 22.6, 900 22.6 /
+// 26.4, 1184 26.7 / 26.7, 1600 32.8 / 36.9, 2304 42.9 / 40.8, 3025 51.6 / 55.3, 3540 59.6 /
+// 55.4, 4096 68.2 / 67.5, 4692 76.1 / 69.5, 5184 82.3 / 82.2, 5550 90 / 84, 5776 96.1 / 85.0,
+// 8100 145 / 113.  Nodes numbered vertices first or at random, which the host cannot see,
+// cost the fragment kernel more (3540: 61.2 / 65.6 and 62.5 / 67.4, 5550 91.5 / 100.7 and
+// 101 / 111, 5776 99.8 / 102 and 112 / 115, 8100 154 / 137 and 178 / 171): the sizes where it gains a little
+// on a grid alone stay with the element kernel.
 static bool dropin_element_kernel(int order, int mode, int64_t elements) {
   constexpr int64_t W = 148 * 8;
   if (order != 4 || !(mode & dev::kJac)) return false;
-  const int64_t steps = elements <= W ? 1 : 2 * ((elements + 2 * W - 1) / (2 * W));
-  return 32 * (steps * W - elements) > steps * steps * W;
+  const int64_t steps = 2 * ((elements + 2 * W - 1) / (2 * W));
+  return elements <= W || 32 * (steps * W - elements) > steps * steps * W;
 }
 
 int launch(int order, int precision, int mode, const dev::AsmArgs &a, cudaStream_t s, int strain) {
