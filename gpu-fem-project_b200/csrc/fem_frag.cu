@@ -243,24 +243,20 @@ __host__ __device__ __forceinline__ uint32_t drop_run(int pass, int i) {
   return 0xffffffffu;
 }
 
-// Drop-in: the blocks staged from double `src` of redsW on are added at map offsets m[0..3]
-// (n = 0, 1 or 4 of them), each maximal stretch of blocks adjacent in the matrix with one
-// reduction.  The warp adds with FP64 atomics, four lanes to a block, where a block is not
-// 16-byte aligned (the matrix is not, or the caller's map has an odd offset), and where an
-// entry's four blocks are all apart, if that holds for more than half of the warp's
-// entries, as on a mesh numbered at random: four reductions of 32 bytes are slower than
-// that there (order 4 100 x 99 246 / 214 us, 200 x 199 960 / 837; order 2 250 x 249 123 /
-// 107).  A grid's last columns are apart too (8 of 32 entries, order 4): reductions are
-// faster for those (200 x 199 477 / 513 us).
-__device__ __forceinline__ void drop_issue(double *mat, const int (&m)[4], int n, const double *redsW, int src, int lane) {
-  const bool odd = ((reinterpret_cast<uintptr_t>(mat) | 8u * (unsigned)(m[0] | m[1] | m[2] | m[3])) & 15u) != 0;
+// Drop-in: the blocks staged from `src` on are added at map offsets m[0..3] (n = 1 or 4
+// of them), each maximal stretch of blocks adjacent in the matrix with one reduction;
+// FP64 atomics where a block is not 16-byte aligned (the matrix is not, or the caller's map
+// has an odd offset).  n = 0: none.
+__device__ __forceinline__ void drop_issue(double *mat, const int (&m)[4], int n, const double *src) {
+  if (((reinterpret_cast<uintptr_t>(mat) | 8u * (unsigned)(m[0] | m[1] | m[2] | m[3])) & 15u) != 0) {
+    for (int j = 0; j < n; j++)
+      for (int c = 0; c < 4; c++) atomicAdd(mat + m[j] + c, src[4 * j + c]);
+    return;
+  }
   const int c1 = n == 4 && m[1] == m[0] + 4, c2 = n == 4 && m[2] == m[1] + 4, c3 = n == 4 && m[3] == m[2] + 4;
-  const int joined = __popc(__ballot_sync(0xffffffffu, c1 | c2 | c3)), fours = __popc(__ballot_sync(0xffffffffu, n == 4));
-  const bool single = n > 0 && (odd || (n == 4 && !(c1 | c2 | c3) && 2 * joined < fours));
-  const int k = single ? 0 : n;
-  const int b[4] = {k ? 32 * (1 + c1 * (1 + c2 * (1 + c3))) : 0, k == 4 && !c1 ? 32 * (1 + c2 * (1 + c3)) : 0,
-                    k == 4 && !c2 ? 32 * (1 + c3) : 0, k == 4 && !c3 ? 32 : 0};
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(redsW + src);
+  const int b[4] = {n ? 32 * (1 + c1 * (1 + c2 * (1 + c3))) : 0, n == 4 && !c1 ? 32 * (1 + c2 * (1 + c3)) : 0,
+                    n == 4 && !c2 ? 32 * (1 + c3) : 0, n == 4 && !c3 ? 32 : 0};
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(src);
 #pragma unroll
   for (int j = 0; j < 4; j++)
     asm volatile("{\n\t.reg .pred p;\n\t"
@@ -268,15 +264,32 @@ __device__ __forceinline__ void drop_issue(double *mat, const int (&m)[4], int n
                  "@p cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f64 [%0], [%1], %2;\n\t}" ::"l"(mat + m[j]),
                  "r"(sa + 32 * j), "r"(b[j])
                  : "memory");
-  if (!__any_sync(0xffffffffu, single)) return;
-#pragma unroll
+}
+
+// Whether the four blocks of an entry are all apart.
+__device__ __forceinline__ bool drop_apart(const int (&m)[4], int n) {
+  return n == 4 && m[1] != m[0] + 4 && m[2] != m[1] + 4 && m[3] != m[2] + 4;
+}
+
+// drop_issue at order 4 for an element whose entries' blocks are mostly apart (a mesh
+// numbered at random): those by FP64 atomics, four lanes to a block, which is faster there
+// than four reductions of 32 bytes (90 x 89 184 / 165 us, 200 x 199 866 / 800; the element
+// kernel's atomics 175 and 917).  A grid's last columns are apart too (8 of 32 entries):
+// reductions are faster for those (200 x 199 485 / 513 us).
+__device__ __forceinline__ void drop_issue_scattered(double *mat, const int (&m)[4], int n, const double *redsW, int src,
+                                                     int lane) {
+  const bool apart = drop_apart(m, n);
+  drop_issue(mat, m, apart ? 0 : n, redsW + src);
+  __syncwarp();
+#pragma unroll 1
   for (int g = 0; g < 4; g++) {  // the entries of lanes 8g .. 8g + 7
     const int from = 8 * g + (lane >> 2), c = lane & 3;
-    const int count = __shfl_sync(0xffffffffu, single ? n : 0, from), s0 = __shfl_sync(0xffffffffu, src, from);
+    const bool add = __shfl_sync(0xffffffffu, (int)apart, from) != 0;
+    const int s0 = __shfl_sync(0xffffffffu, src, from);
 #pragma unroll
     for (int j = 0; j < 4; j++) {
       const int off = __shfl_sync(0xffffffffu, m[j], from);
-      if (j < count) atomicAdd(mat + off + c, redsW[s0 + 4 * j + c]);
+      if (add) atomicAdd(mat + off + c, redsW[s0 + 4 * j + c]);
     }
   }
 }
@@ -562,14 +575,29 @@ struct PairCursor {
 };
 
 
-// Single mesh: units p, p + stride, ... of list positions [begin, end), `pairs` pairs and
-// then single elements.
+// Single mesh, order-4 plans: units p, p + stride, ... of list positions [begin, end), all of
+// `unit` elements (their kernel, short of registers, is slower with the next form: 381 x 379
+// 999 -> 1054 us).
+struct UnitStride {
+  static constexpr bool kBatched = false, kSched = false, kStrip = false;
+  int64_t begin, end, p, stride;
+  int unit;
+  __device__ PairCursor next(int) {
+    PairCursor c{0, 0, begin + unit * p};
+    if (c.k0 < end) c.ne = (int)min((int64_t)unit, end - c.k0);
+    p += stride;
+    return c;
+  }
+};
+
+// Single mesh: units p, p + stride, ... of `units`, the first `pairs` of them pairs of list
+// positions from `begin` on, the others single elements.
 struct PairStride {
   static constexpr bool kBatched = false, kSched = false, kStrip = false;
-  int64_t begin, end, p, stride, pairs;
+  int64_t begin;
+  unsigned p, stride, pairs, units;
   __device__ PairCursor next(int) {
-    PairCursor c{0, 0, begin + p + min(p, pairs)};
-    if (c.k0 < end) c.ne = (int)min((int64_t)(p < pairs ? 2 : 1), end - c.k0);
+    PairCursor c{0, (p < pairs) + (p < units), begin + (p + min(p, pairs))};
     p += stride;
     return c;
   }
@@ -831,6 +859,7 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
   // turns with every bulk group and is kept from step to step, so the one group that a
   // put's wait leaves unfinished always reads the other half.
   [[maybe_unused]] int half = 0;
+  [[maybe_unused]] bool scattered = false;  // drop-in, order 4: drop_issue_scattered adds the blocks
 
   // Mesh arguments are read through `mtab` (for one mesh, a pointer to the kernel
   // parameter).  At p = 4 it is laundered once per step: the compiler then reloads
@@ -1775,10 +1804,9 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
             stage_at(SX + (xd ? 2 * NM : (tr ? NM : 0) + 8 * Tm + pa), kxx, tr ? kyx : kxy, tr ? kxy : kyx, kyy);
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncwarp();
-#pragma unroll
-          for (int x = 0; x < L::DR / 32; x++) {
+          auto entry = [&](int x, int (&m)[4], int &src) {
             const uint32_t e = tabR[PASS * L::DR + 32 * x + lane];
-            int m[4];
+            src = 4 * (e >> 13 & 0x1ff);
             if constexpr (P == 4) {
 #pragma unroll
               for (int j = 0; j < 4; j++) m[j] = mp[x][j];
@@ -1787,7 +1815,25 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
 #pragma unroll
               for (int j = 0; j < 4; j++) m[j] = row[j < (int)((e >> 11) & 3) + 1 ? j : 0];
             }
-            drop_issue(O.mat, m, e == 0xffffffffu ? 0 : ((e >> 11) & 3) + 1, redsW, 4 * (e >> 13 & 0x1ff), lane);
+            return e == 0xffffffffu ? 0 : (int)((e >> 11) & 3) + 1;
+          };
+          int m[4], src;
+          if (P == 4 && PASS == 0) {
+            const int n = entry(0, m, src);
+            scattered = 2 * __popc(__ballot_sync(0xffffffffu, drop_apart(m, n))) > __popc(__ballot_sync(0xffffffffu, n == 4));
+          }
+          if (P == 4 && scattered) {
+#pragma unroll
+            for (int x = 0; x < L::DR / 32; x++) {
+              const int n = entry(x, m, src);
+              drop_issue_scattered(O.mat, m, n, redsW, src, lane);
+            }
+          } else {
+#pragma unroll
+            for (int x = 0; x < L::DR / 32; x++) {
+              const int n = entry(x, m, src);
+              drop_issue(O.mat, m, n, redsW + src);
+            }
           }
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         }
@@ -1813,16 +1859,23 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
 }
 
 // One mesh: plan mode, list positions [A.begin, A.begin + A.count) of one colour;
-// drop-in mode, elements [A.begin, A.begin + A.count) through the reference map.
+// drop-in mode, elements [A.begin, A.begin + A.count) through the reference map.  split: the
+// pairs (PairStride), for order-4 plans the elements of a unit (UnitStride).
 template <int P, int MODE>
 __global__ void __launch_bounds__(32 * FragDims<P>::WARPS, FEM_FRAG_MINB) frag_kernel(const __grid_constant__ AsmArgs A,
-                                                                                             int64_t pairs) {
+                                                                                             int split) {
   extern __shared__ __align__(16) unsigned char smem[];
   frag_prologue<P, MODE>(smem);
   const int warp = threadIdx.x >> 5;
-  PairStride gen{A.begin, A.begin + A.count, (int64_t)blockIdx.x * FragDims<P>::WARPS + warp,
-                 (int64_t)gridDim.x * FragDims<P>::WARPS, pairs};
-  frag_loop<P, MODE>(smem, gen, A, &A);
+  if constexpr (P == 4 && (MODE & kPlan) != 0) {
+    UnitStride gen{A.begin, A.begin + A.count, (int64_t)blockIdx.x * FragDims<P>::WARPS + warp,
+                   (int64_t)gridDim.x * FragDims<P>::WARPS, split};
+    frag_loop<P, MODE>(smem, gen, A, &A);
+  } else {
+    PairStride gen{A.begin, blockIdx.x * FragDims<P>::WARPS + warp, gridDim.x * FragDims<P>::WARPS, (unsigned)split,
+                   (unsigned)A.count - (unsigned)split};
+    frag_loop<P, MODE>(smem, gen, A, &A);
+  }
 }
 
 // One mesh, several list-position ranges (plan mode).
@@ -1932,22 +1985,31 @@ int launch_frag_p(const AsmArgs &a, cudaStream_t s, bool chained, bool single) {
   // pair: the warp's step is what the launch takes, and one element's stiffness and writes
   // are most of half of it (33 x 31 order 4 63.5 -> 38.9 us, order 3 NONLINEAR
   // 44.1 -> 22.6; order 2, bound by its four launches, 18.5 -> 18.4), and so does the last
-  // round of the warps as far as its elements go around (order-4 drop-in 90 x 89 128 -> 113
-  // us, order-3 drop-in 80 x 79 34.8 -> 32.8, order-3 NONLINEAR plan 90 x 89 63.5 -> 58.4).
+  // round of the warps as far as its elements go around (order-4 drop-in 90 x 89 122 -> 112
+  // us, order-3 drop-in 80 x 79 34.8 -> 32.8, order-3 NONLINEAR plan 90 x 89 63.5 -> 58.4;
+  // not in order-4 plans, see UnitStride).
   // Not the residual alone, where both elements of a step are rows of the same products
   // (90 x 89 in the colour layout, order 2 one / two per warp 20.5 / 14.4, order 3 22.0 / 16.4).
-  const int64_t per = cap * F::WARPS, left = a.count % (2 * per);
-  const int64_t pairs =
-      single && (MODE & kJac) != 0 ? (a.count - left) / 2 + std::max<int64_t>(left - per, 0) : (a.count + 1) / 2;
-  const int64_t units = std::max(a.count - pairs, pairs);
+  [[maybe_unused]] const int64_t per = cap * F::WARPS, left = a.count % (2 * per);
+  int split;
+  int64_t units;
+  if constexpr (P == 4 && (MODE & kPlan) != 0) {
+    split = single && (MODE & kJac) != 0 && a.count <= per ? 1 : 2;
+    units = (a.count + split - 1) / split;
+  } else {
+    const int64_t pairs =
+        single && (MODE & kJac) != 0 ? (a.count - left) / 2 + std::max<int64_t>(left - per, 0) : a.count / 2;
+    split = (int)pairs;
+    units = a.count - pairs;
+  }
   const int64_t need = (units + F::WARPS - 1) / F::WARPS;
   const int grid = (int)(need < cap ? need : cap);
   if (grid <= 0) return FEM_SUCCESS;
   cudaError_t err;
   if (chained) {
-    err = pdl_launch(kernel, grid, NT, smem, s, a, pairs);
+    err = pdl_launch(kernel, grid, NT, smem, s, a, split);
   } else {
-    kernel<<<grid, NT, smem, s>>>(a, pairs);
+    kernel<<<grid, NT, smem, s>>>(a, split);
     err = cudaGetLastError();
   }
   if (err != cudaSuccess) return cuda_fail(err, "frag_kernel launch");
