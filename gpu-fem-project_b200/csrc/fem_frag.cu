@@ -66,8 +66,11 @@
 #include "fem_launch.h"
 
 // Resident CTAs per SM the register budget is sized for: 3 (168 registers) at
-// p = 3, where the 12 live stiffness accumulators need them, and at p = 4; 4 (128)
-// at p = 2.  The residual alone, without stiffness accumulators: 6 (85 registers) at
+// p = 3, where the 12 live stiffness accumulators need them, and in p = 4 plans; 4 (128)
+// at p = 2; 2 (255) in the p = 4 drop-in Jacobian, whose map entries are in flight beside
+// the accumulators and whose reductions, not its warps, set the time (200 x 199 485 us, with
+// 3 CTAs 511; the plan, whose blocks leave one by one, loses: 256^2 507, with 2 CTAs 537).
+// The residual alone, without stiffness accumulators: 6 (85 registers) at
 // p = 2, 3 (800 x 512 p = 2: 175 / 159 / 152 us with 4 / 5 / 6; 600 x 590 p = 3: 172 / 162 /
 // 160 us), 4 at p = 4 (256^2: 102 / 107 / 115 us).
 #ifndef FEM_FRAG_MINB

@@ -258,10 +258,11 @@ static void right_neighbours(const int *connPtr, const int *conn, const HostPlan
 // Elements per strip (odd: with the halo, whole steps of two).  A launch of a colour
 // (about half of the elements) runs its strips in waves over the resident warps, so a
 // strip's steps times the waves are what it takes, and half a step is lost to a strip's
-// halo.  Measured (order 3, us, when a halo still took a whole element's products; 5 / 7 /
-// 11 / 15 / 23 elements): 128^2 55 / 65 / 77 / 74 / 104, 200^2 123 / 120 / 137 / 121 / 154, 256^2 177 / 175 / 176 / 189 / 175, 512^2 622 /
-// 593 / 582 / 576 / 596, 1024^2 2454 / 2338 / 2252 / 2218 / 2209; the last wave is partly
-// overlapped, hence the mean of whole and exact waves.
+// halo.  Measured (order 3, us; 3 / 5 / 7 / 11 / 15 / 23 elements, then the length taken): 128^2 58 /
+// 50 / 61 / 71 / 69 / 99, 50; 200^2 106 / 111 / 111 / 127 / 115 / 147, 103; 256^2 159 / 160 / 162 / 166 / 178 /
+// 168, 156; 512^2 580 / 559 / 536 / 545 / 551 / 574, 535; 1024^2 2261 / 2149 / 2098 / 2056 / 2057 / 2053,
+// 2056; 43^2 17 with 1, which it takes, 21 with 3.  The last wave is partly overlapped, hence
+// the mean of whole and exact waves.
 // chainPtr, colour: the chains and their colours (nc).
 static int strip_length(const std::vector<int> &chainPtr, const std::vector<int> &colour, int nc) {
   int best = 1;

@@ -155,7 +155,8 @@ __device__ __forceinline__ void row_stream(const AsmArgs &M, int64_t c, int64_t 
       // xi-derivative of a column node depends on the point's eta only (times the node's
       // side), so M_ij[b] = sum_q s mu G_ai G_bj comes from A0_ij(eta) = sum_xi hv_i adj_0j,
       // A1_ij(xi) = sum_eta hv_i adj_1j: about 290 FP64 operations per entry instead of 380
-      // with the four nodes' gradients formed at every point (2048^2: 636 -> 558 us).
+      // with the four nodes' gradients formed at every point (2048^2: 636 -> 558 us; 538 on
+      // another GPU).
       double A0[2][4], A1[2][4];  // [eta | xi][xx, xy, yx, yy]
 #pragma unroll
       for (int q = 0; q < 4; q++) {

@@ -347,11 +347,13 @@ int fem_batch_wait_status(fem_batch *batch, void *stream, int64_t *timedOutWaits
 int fem_batch_set_schedule_waits(fem_batch *batch, int64_t waitLimitNs, int order, int stallGroup);
 /* One assembly of every mesh, stream-ordered on `stream`. */
 int fem_batch_assemble(fem_batch *batch, int precision, void *stream, double *elapsedSeconds);
-/* Autotuner: per order, times the order's launches for every kernel variant the
- * precision allows, every candidate tile length (1, 4, 16, 64, 256 element
- * batches; reps repetitions after a warm-up) and, for the fragment kernels, both
- * launch forms (per colour, dependency-ordered), and keeps the fastest
- * (fem_batch_get_kernels / fem_batch_get_tiles / fem_batch_get_ordered report it).  Replaces the
+/* Autotuner: per order, times the order's launches as the batch has them, then for every
+ * kernel variant the precision allows, every candidate tile length (1, 4, 16, 64, 256
+ * element batches; reps repetitions after a warm-up) and, for the fragment kernels, both
+ * launch forms (per colour, dependency-ordered).  The orders' fastest choices are kept
+ * where the whole batch's captured replay is faster with them than with what it had
+ * (fem_batch_get_kernels / fem_batch_get_tiles / fem_batch_get_ordered report it); a graph
+ * captured before is dropped.  Replaces the
  * (order, precision) reference tables of hand-tuned elements per block
  * (element/FEKernels.h:1009-1028, 1104-1123). */
 int fem_batch_tune(fem_batch *batch, int precision, void *stream, int reps, double *bestSeconds);
