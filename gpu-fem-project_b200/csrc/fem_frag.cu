@@ -1481,365 +1481,364 @@ __device__ __forceinline__ void frag_loop(unsigned char *smem, Gen &gen, const A
           }
         }
         auto pass = [&](auto passc) {
-        constexpr int PASS = decltype(passc)::value;
-        // fragments of tiles [0, NF); residual slots: tiles RT0 and RT1, NTM = node XN;
-        // xs[0], xs[1]: M[XN][tile] (orders 2: tile 0; 4: tiles 0, 1 | 2) and M[XN][XN]
-        constexpr int NF = PASS ? 3 : (NTM == 1 ? 1 : 2);
-        [[maybe_unused]] constexpr int RT0 = PASS ? 2 : 0, RT1 = PASS || NTM == 1 ? NTM : 1;
-        constexpr bool XD = EX && RT1 == NTM;  // this pass has XN's own row
-        double acc[NPAIR][4][2];
-        [[maybe_unused]] double rp[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-        [[maybe_unused]] double xs[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
-        auto kstep = [&](int ks, auto firstc, auto negc) {
-          constexpr bool FIRST = decltype(firstc)::value, NEG = decltype(negc)::value;
-          const int o = el * PS + L::slot(4 * ks) + t;
-          const double2 w0 = WI0[o], w1 = WI1[o];
-          double fr[NTM][2];
-  #pragma unroll
-          for (int T = 0; T < NF; T++) {
-            const double2 d = tabF[(ks * NTM + T) * 32 + lane];
-            fr[T][0] = fma(w0.x, d.x, w0.y * d.y);
-            fr[T][1] = fma(w1.x, d.x, w1.y * d.y);
-          }
-          [[maybe_unused]] double h0 = 0.0, h1 = 0.0;  // G-hat(q, XN)
-          if constexpr (EX && (JAC || XD)) {
-            const double2 d = tabX[4 * ks + t];
-            h0 = fma(w0.x, d.x, w0.y * d.y);
-            h1 = fma(w1.x, d.x, w1.y * d.y);
-          }
-          if constexpr (RES) {
-            // LINEAR: the stress is symmetric, S-hat_yx = S-hat_xy
-            const double2 s0 = WS0[o];
-            const double s1y = WS1[o].y, s1x = NL ? WS1[o].x : s0.y;
-  #pragma unroll
-            for (int x = 0; x < 2; x++) {
-              const int T = x ? RT1 : RT0;
-              const double f0 = T == NTM ? h0 : fr[T < NTM ? T : 0][0], f1 = T == NTM ? h1 : fr[T < NTM ? T : 0][1];
-              rp[x][0] = fma(f0, s0.x, fma(f1, s1x, rp[x][0]));
-              rp[x][1] = fma(f0, s0.y, fma(f1, s1y, rp[x][1]));
+          constexpr int PASS = decltype(passc)::value;
+          // fragments of tiles [0, NF); residual slots: tiles RT0 and RT1, NTM = node XN;
+          // xs[0], xs[1]: M[XN][tile] (orders 2: tile 0; 4: tiles 0, 1 | 2) and M[XN][XN]
+          constexpr int NF = PASS ? 3 : (NTM == 1 ? 1 : 2);
+          [[maybe_unused]] constexpr int RT0 = PASS ? 2 : 0, RT1 = PASS || NTM == 1 ? NTM : 1;
+          double acc[NPAIR][4][2];
+          [[maybe_unused]] double rp[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+          [[maybe_unused]] double xs[2][4] = {{0.0, 0.0, 0.0, 0.0}, {0.0, 0.0, 0.0, 0.0}};
+          auto kstep = [&](int ks, auto firstc, auto negc) {
+            constexpr bool FIRST = decltype(firstc)::value, NEG = decltype(negc)::value;
+            const int o = el * PS + L::slot(4 * ks) + t;
+            const double2 w0 = WI0[o], w1 = WI1[o];
+            double fr[NTM][2];
+#pragma unroll
+            for (int T = 0; T < NF; T++) {
+              const double2 d = tabF[(ks * NTM + T) * 32 + lane];
+              fr[T][0] = fma(w0.x, d.x, w0.y * d.y);
+              fr[T][1] = fma(w1.x, d.x, w1.y * d.y);
             }
-          }
-          if constexpr (JAC && NL) {
-            // K_ik[a][b] = sum over (q, l) of G-hat_l(q, a) B_ikl(q, b),
-            // B_ikl = sign(s) sum_n A_{il,kn} G-hat_n(q, b): 4 (i, k) x 2 (l) MMAs per pair
-            const double *at = ATs + (el * NQP + 4 * ks + t) * 16;
-#pragma unroll
-            for (int ll = 0; ll < 2; ll++) {
-              double C[2][2][2];  // [i][k][n]
-#pragma unroll
-              for (int j = 0; j < 4; j++) {
-                const double2 v = *reinterpret_cast<const double2 *>(at + ll * 8 + 2 * j);
-                C[j >> 1][j & 1][0] = v.x;
-                C[j >> 1][j & 1][1] = v.y;
-              }
-#pragma unroll
-              for (int k = 0; k < NPAIR; k++) {
-                const int TA = F::ta(PASS, k), TB = F::tb(PASS, k);
-#pragma unroll
-                for (int ik = 0; ik < 4; ik++) {
-                  const double bv = fma(C[ik >> 1][ik & 1][0], fr[TB][0], C[ik >> 1][ik & 1][1] * fr[TB][1]);
-                  if (FIRST && ll == 0) dmma_first(acc[k][ik][0], acc[k][ik][1], fr[TA][ll], bv);
-                  else dmma(acc[k][ik][0], acc[k][ik][1], fr[TA][ll], bv);
-                }
-              }
-              if constexpr (EX) {
-                const double hl = ll ? h1 : h0;
-#pragma unroll
-                for (int ik = 0; ik < 4; ik++) {
-                  xs[0][ik] = fma(hl, fma(C[ik >> 1][ik & 1][0], fr[0][0], C[ik >> 1][ik & 1][1] * fr[0][1]), xs[0][ik]);
-                  xs[1][ik] = fma(hl, fma(C[ik >> 1][ik & 1][0], h0, C[ik >> 1][ik & 1][1] * h1), xs[1][ik]);
-                }
-              }
-            }
-          }
-          if constexpr (JAC && !NL) {
-            double sg = 1.0;
-            if constexpr (NEG) sg = SGs[el * NQP + 4 * ks + t];
-            double af[NTM][2];  // A fragments: times the point's sign
-  #pragma unroll
-            for (int T = 0; T < NF; T++) af[T][0] = NEG ? sg * fr[T][0] : fr[T][0], af[T][1] = NEG ? sg * fr[T][1] : fr[T][1];
-  #pragma unroll
-            for (int k = 0; k < NPAIR; k++) {
-              const int TA = F::ta(PASS, k), TB = F::tb(PASS, k);
-  #pragma unroll
-              for (int ij = 0; ij < 4; ij++) {
-                if constexpr (FIRST) dmma_first(acc[k][ij][0], acc[k][ij][1], af[TA][ij >> 1], fr[TB][ij & 1]);
-                else dmma(acc[k][ij][0], acc[k][ij][1], af[TA][ij >> 1], fr[TB][ij & 1]);
-              }
-            }
+            [[maybe_unused]] double h0 = 0.0, h1 = 0.0;  // G-hat(q, XN)
             if constexpr (EX) {
-              const double s0 = NEG ? sg * h0 : h0, s1 = NEG ? sg * h1 : h1;
-  #pragma unroll
+              const double2 d = tabX[4 * ks + t];
+              h0 = fma(w0.x, d.x, w0.y * d.y);
+              h1 = fma(w1.x, d.x, w1.y * d.y);
+            }
+            if constexpr (RES) {
+              // LINEAR: the stress is symmetric, S-hat_yx = S-hat_xy
+              const double2 s0 = WS0[o];
+              const double s1y = WS1[o].y, s1x = NL ? WS1[o].x : s0.y;
+#pragma unroll
               for (int x = 0; x < 2; x++) {
                 const int T = x ? RT1 : RT0;
                 const double f0 = T == NTM ? h0 : fr[T < NTM ? T : 0][0], f1 = T == NTM ? h1 : fr[T < NTM ? T : 0][1];
-                xs[x][0] = fma(s0, f0, xs[x][0]);
-                xs[x][1] = fma(s0, f1, xs[x][1]);
-                xs[x][2] = fma(s1, f0, xs[x][2]);
-                xs[x][3] = fma(s1, f1, xs[x][3]);
+                rp[x][0] = fma(f0, s0.x, fma(f1, s1x, rp[x][0]));
+                rp[x][1] = fma(f0, s0.y, fma(f1, s1y, rp[x][1]));
               }
             }
-          }
-        };
-        // drop-in order 4: the lane's map entries of this pass, in flight during the products
-        int mp[L::DR ? L::DR / 32 : 1][4];
-        if constexpr (JAC && !PLAN && P == 4) {
-          const int *row = M.map + (cur.k0 + el) * (int64_t)(NN * NN);
+            if constexpr (NL) {
+              // K_ik[a][b] = sum over (q, l) of G-hat_l(q, a) B_ikl(q, b),
+              // B_ikl = sign(s) sum_n A_{il,kn} G-hat_n(q, b): 4 (i, k) x 2 (l) MMAs per pair
+              const double *at = ATs + (el * NQP + 4 * ks + t) * 16;
 #pragma unroll
-          for (int x = 0; x < L::DR / 32; x++) {
-            const uint32_t e = tabR[PASS * L::DR + 32 * x + lane];
-            const int o = e == 0xffffffffu ? 0 : e & 0x3ff, n = e == 0xffffffffu ? 0 : (e >> 11) & 3;
+              for (int ll = 0; ll < 2; ll++) {
+                double C[2][2][2];  // [i][k][n]
 #pragma unroll
-            for (int j = 0; j < 4; j++) mp[x][j] = __ldg(row + o + (j <= n ? j : 0) * (e >> 10 & 1 ? 5 : 1));
-          }
-        }
-        kstep_all(kstep, neg);
-        // residual: sum over the four lanes t of a node (reduce-scatter over the two slots)
-        [[maybe_unused]] const int Tm = t >> 1, To = Tm ^ 1;
-        if constexpr (RES) {
-          double sx = (Tm ? rp[1][0] : rp[0][0]) + __shfl_xor_sync(0xffffffffu, To ? rp[1][0] : rp[0][0], 2);
-          double sy = (Tm ? rp[1][1] : rp[0][1]) + __shfl_xor_sync(0xffffffffu, To ? rp[1][1] : rp[0][1], 2);
-          sx += __shfl_xor_sync(0xffffffffu, sx, 1);
-          sy += __shfl_xor_sync(0xffffffffu, sy, 1);
-          if constexpr (STRIP) residual_carry(sx, sy, cin);
-          const int an = Tm == 0 ? row_node(RT0) : (RT1 == NTM ? XN : row_node(RT1));
-          const bool act = (t & 1) == 0 && (Tm == 0 || RT1 < NTM || g == 0) && !halo && !(right && g >= 6);
-          residual_put(M.residual + 2 * (int64_t)nid[el * NN + an], act, PLAN && O.codes[el * CS + NN * NN + an], sx, sy);
-        }
-        if constexpr (JAC && RUNS) {
-          // acc becomes the blocks (xx, xy, yx, yy)
-  #pragma unroll
-          for (int k = 0; k < NPAIR; k++)
-  #pragma unroll
-            for (int h = 0; h < 2; h++) {
-              double kxx, kxy, kyx, kyy;
-              block(acc[k][0][h], acc[k][1][h], acc[k][2][h], acc[k][3][h], kxx, kxy, kyx, kyy);
-              acc[k][0][h] = kxx, acc[k][1][h] = kxy, acc[k][2][h] = kyx, acc[k][3][h] = kyy;
-            }
-          // every lane's previous bulk reads of the staging slots are complete
-          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-          __syncwarp();
-          double *stg = redsW + 4 * lane;  // direct blocks: position 4g + t of their slot
-          if constexpr (STRIP) {
-            if (take) {
-  #pragma unroll
-              for (int k = 0; k < NPAIR; k++)
-  #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                  const double2 *cs = reinterpret_cast<const double2 *>(stg + 128 * frag_slot(k, h, 0) + 4 * 27);
-                  acc[k][0][h] += cs[0].x, acc[k][1][h] += cs[0].y;
-                  acc[k][2][h] += cs[1].x, acc[k][3][h] += cs[1].y;
+                for (int j = 0; j < 4; j++) {
+                  const double2 v = *reinterpret_cast<const double2 *>(at + ll * 8 + 2 * j);
+                  C[j >> 1][j & 1][0] = v.x;
+                  C[j >> 1][j & 1][1] = v.y;
                 }
-            }
-            __syncwarp();
-          }
-          uint32_t allfirst = 0x80u;
-          if constexpr (PLAN && !NL) {
-            // the lane's code bytes and row addresses first: rows pi(g) and 8 + pi(g) hold
-            // its direct blocks, rows 8 + 4h + t the transposed ones of pair (0, 1)
-            const uint8_t *rec = O.codes + el * CS;
-            const int *rbe = O.rbase + el * NN;
-            uint32_t cd[NPAIR][2], ct[2];
-  #pragma unroll
-            for (int k = 0; k < NPAIR; k++)
-  #pragma unroll
-              for (int h = 0; h < 2; h++) cd[k][h] = rec[pa * NN + t + (k == 2 ? 8 * NN : 0) + (k == 0 ? 0 : 8) + 4 * h];
-  #pragma unroll
-            for (int h = 0; h < 2; h++) ct[h] = rec[t * NN + pa + (8 + 4 * h) * NN];
-            const double *r0 = O.mat + 4 * (int64_t)rbe[pa], *r1 = O.mat + 4 * (int64_t)rbe[8 + pa];
-            const double *rt0 = O.mat + 4 * (int64_t)rbe[8 + t], *rt1 = O.mat + 4 * (int64_t)rbe[12 + t];
-            const unsigned sd = (unsigned)__cvta_generic_to_shared(stg);
-            const unsigned st = (unsigned)__cvta_generic_to_shared(redsW + 4 * (8 * t + pa));
-            auto direct = [&](auto kc, auto hc) {
-              constexpr int k = decltype(kc)::value, h = decltype(hc)::value;
-              frag_put_row<1024 * frag_slot(k, h, 0)>(k == 2 ? r1 : r0, cd[k][h], m80, sd, acc[k][0][h], acc[k][1][h],
-                                                      acc[k][2][h], acc[k][3][h]);
-              allfirst &= cd[k][h];
-            };
-            direct(IC<0>{}, IC<0>{});
-            direct(IC<0>{}, IC<1>{});
-            direct(IC<1>{}, IC<0>{});
-            direct(IC<1>{}, IC<1>{});
-            frag_put_row<1024 * frag_slot(1, 0, 1)>(rt0, ct[0], m80, st, acc[1][0][0], acc[1][2][0], acc[1][1][0], acc[1][3][0]);
-            frag_put_row<1024 * frag_slot(1, 1, 1)>(rt1, ct[1], m80, st, acc[1][0][1], acc[1][2][1], acc[1][1][1], acc[1][3][1]);
-            direct(IC<2>{}, IC<0>{});
-            direct(IC<2>{}, IC<1>{});
-            allfirst &= ct[0] & ct[1];
-          } else {
-  #pragma unroll
-            for (int k = 0; k < NPAIR; k++) {
-              {
-                const int TA = F::ta(0, k), TB = F::tb(0, k);
-                const int a = 8 * TA + pa;
-  #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                  const int b = 8 * TB + 4 * h + t;
-                  const double kxx = acc[k][0][h], kxy = acc[k][1][h], kyx = acc[k][2][h], kyy = acc[k][3][h];
-                  // NONLINEAR diagonal tiles: (a, b) for a <= b and, for a < b, its exact
-                  // transpose (b, a) at the staging position the (b, a) lane would use
-                  const bool diag = NL && TA == TB;
-                  allfirst &= frag_put<P, PLAN>(O, el, a, b, 0, !diag || a <= b, m80, kxx, kxy, kyx, kyy,
-                                                stg + 128 * frag_slot(k, h, 0));
-                  if (TA < TB) {
-                    allfirst &= frag_put<P, PLAN>(O, el, a, b, 1, true, m80, kxx, kxy, kyx, kyy,
-                                                  redsW + 128 * frag_slot(k, h, 1) + 4 * (8 * t + pa));
-                  } else if (diag) {
-                    const int xb = b - 8 * TA, xa = a - 8 * TA;  // pi(g') = xb; a = 8T + 4h' + t'
-                    const int gb = 2 * (xb & 3) + (xb >> 2);
-                    allfirst &= frag_put<P, PLAN>(O, el, a, b, 1, a < b, m80, kxx, kxy, kyx, kyy,
-                                                  redsW + 128 * frag_slot(k, xa >> 2, 0) + 4 * (4 * gb + (xa & 3)));
+#pragma unroll
+                for (int k = 0; k < NPAIR; k++) {
+                  const int TA = F::ta(PASS, k), TB = F::tb(PASS, k);
+#pragma unroll
+                  for (int ik = 0; ik < 4; ik++) {
+                    const double bv = fma(C[ik >> 1][ik & 1][0], fr[TB][0], C[ik >> 1][ik & 1][1] * fr[TB][1]);
+                    if (FIRST && ll == 0) dmma_first(acc[k][ik][0], acc[k][ik][1], fr[TA][ll], bv);
+                    else dmma(acc[k][ik][0], acc[k][ik][1], fr[TA][ll], bv);
+                  }
+                }
+                if constexpr (EX) {
+                  const double hl = ll ? h1 : h0;
+#pragma unroll
+                  for (int ik = 0; ik < 4; ik++) {
+                    xs[0][ik] = fma(hl, fma(C[ik >> 1][ik & 1][0], fr[0][0], C[ik >> 1][ik & 1][1] * fr[0][1]), xs[0][ik]);
+                    xs[1][ik] = fma(hl, fma(C[ik >> 1][ik & 1][0], h0, C[ik >> 1][ik & 1][1] * h1), xs[1][ik]);
                   }
                 }
               }
             }
-          }
-          issue_runs(O, el, !halo && (allfirst & 0x80u) == 0);
-        }
-        // stiffness blocks, orders 2 and 4: lane (g, t) writes (8TA + pi(g), 8TB + 4h + t) of
-        // each pair and, for TA < TB, its transpose (NONLINEAR diagonal pairs: for a <= b,
-        // and the exact transpose); then the row and column of node XN: of the two slots of
-        // xs, lanes t/2 = x take slot x, t even (XN, a), t odd its transpose.  First stores
-        // go out at once, the blocks to add are staged and leave FL at a time after one
-        // proxy fence, as one bulk group.  Fewer fences and groups, against waiting for the
-        // group before: order 4 takes all four slots at a time (256^2 486 us; two from each
-        // half of the slots in turn 503), order 2 an element's three (512 x 2048 annulus 1178
-        // us, from two sets of slots in turn 1184), its NONLINEAR blocks two (500 x 512 770 us,
-        // four 808).
-        if constexpr (JAC && EX && PLAN) {
-          constexpr int FL = P == 4 ? 4 : (NL ? 2 : 3), HALF = FL == 2 ? 2 : 0;
-          double *reds = redsW + 4 * lane;
-          double *dst[FL];
-          bool add[FL];
-          int n = 0;
-          auto flush = [&](int m) {
-            bool any = false;
+            if constexpr (!NL) {
+              double sg = 1.0;
+              if constexpr (NEG) sg = SGs[el * NQP + 4 * ks + t];
+              double af[NTM][2];  // A fragments: times the point's sign
 #pragma unroll
-            for (int x = 0; x < FL; x++) any = any || (x < m && add[x]);
-            if (!__any_sync(0xffffffffu, any)) return;
-            if (el > 0) pair_first_landed();
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            if (el > 0) {
-              __syncwarp();
-              pair_first_visible();
-            }
+              for (int T = 0; T < NF; T++) af[T][0] = NEG ? sg * fr[T][0] : fr[T][0], af[T][1] = NEG ? sg * fr[T][1] : fr[T][1];
 #pragma unroll
-            for (int x = 0; x < FL; x++)
-              if (x < m) bulk_add_block(dst[x], reds + 128 * (HALF * half + x), add[x]);
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-            half ^= 1;
-          };
-          auto put = [&](int r, int c, bool act, double v0, double v1, double v2, double v3) {
-            // the bulk reads of the slots used next are complete
-            if (n == 0) {
-              if constexpr (HALF) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-              else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-            }
-            add[n] = frag_put_block<P>(O, el, r, c, act, v0, v1, v2, v3, reds + 128 * (HALF * half + n), dst[n]);
-            if (++n == FL) {
-              flush(FL);
-              n = 0;
-            }
-          };
-          double kxx, kxy, kyx, kyy;
+              for (int k = 0; k < NPAIR; k++) {
+                const int TA = F::ta(PASS, k), TB = F::tb(PASS, k);
 #pragma unroll
-          for (int k = 0; k < NPAIR; k++)
+                for (int ij = 0; ij < 4; ij++) {
+                  if constexpr (FIRST) dmma_first(acc[k][ij][0], acc[k][ij][1], af[TA][ij >> 1], fr[TB][ij & 1]);
+                  else dmma(acc[k][ij][0], acc[k][ij][1], af[TA][ij >> 1], fr[TB][ij & 1]);
+                }
+              }
+              if constexpr (EX) {
+                const double s0 = NEG ? sg * h0 : h0, s1 = NEG ? sg * h1 : h1;
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-              const int TA = F::ta(PASS, k), TB = F::tb(PASS, k);
-              const int a = row_node(TA), b = col_node(TB, h);
-              const bool diag = NL && TA == TB;
-              block(acc[k][0][h], acc[k][1][h], acc[k][2][h], acc[k][3][h], kxx, kxy, kyx, kyy);
-              put(a, b, !diag || a <= b, kxx, kxy, kyx, kyy);
-              if (TA < TB || diag) put(b, a, !diag || a < b, kxx, kyx, kxy, kyy);
-            }
-          double xv[4];
-#pragma unroll
-          for (int c = 0; c < 4; c++) {
-            xv[c] = (Tm ? xs[1][c] : xs[0][c]) + __shfl_xor_sync(0xffffffffu, To ? xs[1][c] : xs[0][c], 2);
-            xv[c] += __shfl_xor_sync(0xffffffffu, xv[c], 1);
-          }
-          block(xv[0], xv[1], xv[2], xv[3], kxx, kxy, kyx, kyy);
-          const int xa = Tm == 0 ? row_node(RT0) : (RT1 == NTM ? XN : row_node(RT1));
-          const bool tr = t & 1;
-          put(tr ? xa : XN, tr ? XN : xa, Tm == 0 || RT1 < NTM || (g == 0 && !tr), kxx, tr ? kyx : kxy, tr ? kxy : kyx, kyy);
-          if (n) flush(n);
-        }
-        // drop-in, orders 2 and 4: every block is staged (drop_run), and each lane adds its
-        // entries' stretches of adjacent blocks.  A reduction of 32 bytes per block bounded
-        // these launches: 200 x 201 order 4, with the element kernel's FP64 atomics 987 us
-        // for the driver's two calls, with 32-byte reductions 1082, with stretches 648;
-        // 501 x 500 order 2 597 -> 496
-        if constexpr (JAC && EX && !PLAN) {
-          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-          __syncwarp();
-          auto stage_at = [&](int block, double v0, double v1, double v2, double v3) {
-            double2 *x = reinterpret_cast<double2 *>(redsW + 4 * block);
-            x[0] = make_double2(v0, v1);
-            x[1] = make_double2(v2, v3);
-          };
-          double kxx, kxy, kyx, kyy;
-          int sl = 0;  // slots in the order of drop_run
-#pragma unroll
-          for (int k = 0; k < NPAIR; k++)
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-              const int TA = F::ta(PASS, k), TB = F::tb(PASS, k);
-              block(acc[k][0][h], acc[k][1][h], acc[k][2][h], acc[k][3][h], kxx, kxy, kyx, kyy);
-              if constexpr (NL) {  // order 2: (a, b) for a <= b and its exact transpose
-                const int b = 4 * h + t;
-                if (pa <= b) stage_at(32 * h + 4 * g + t, kxx, kxy, kyx, kyy);
-                if (pa < b) stage_at(32 * (pa >> 2) + 4 * (2 * (b & 3) + (b >> 2)) + (pa & 3), kxx, kyx, kxy, kyy);
-              } else {
-                stage_at(32 * sl++ + 4 * g + t, kxx, kxy, kyx, kyy);
-                if (TA < TB) stage_at(32 * sl++ + 8 * t + pa, kxx, kyx, kxy, kyy);
+                for (int x = 0; x < 2; x++) {
+                  const int T = x ? RT1 : RT0;
+                  const double f0 = T == NTM ? h0 : fr[T < NTM ? T : 0][0], f1 = T == NTM ? h1 : fr[T < NTM ? T : 0][1];
+                  xs[x][0] = fma(s0, f0, xs[x][0]);
+                  xs[x][1] = fma(s0, f1, xs[x][1]);
+                  xs[x][2] = fma(s1, f0, xs[x][2]);
+                  xs[x][3] = fma(s1, f1, xs[x][3]);
+                }
               }
             }
-          double xv[4];
-#pragma unroll
-          for (int c = 0; c < 4; c++) {
-            xv[c] = (Tm ? xs[1][c] : xs[0][c]) + __shfl_xor_sync(0xffffffffu, To ? xs[1][c] : xs[0][c], 2);
-            xv[c] += __shfl_xor_sync(0xffffffffu, xv[c], 1);
-          }
-          block(xv[0], xv[1], xv[2], xv[3], kxx, kxy, kyx, kyy);
-          constexpr int SX = 32 * (P == 2 ? 2 : PASS ? 10 : 8), NM = RT1 < NTM ? 16 : 8;
-          const bool tr = t & 1, xd = RT1 == NTM && Tm == 1;  // xd: the diagonal block's lanes
-          if (!xd || (g == 0 && !tr))
-            stage_at(SX + (xd ? 2 * NM : (tr ? NM : 0) + 8 * Tm + pa), kxx, tr ? kyx : kxy, tr ? kxy : kyx, kyy);
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          __syncwarp();
-          auto entry = [&](int x, int (&m)[4], int &src) {
-            const uint32_t e = tabR[PASS * L::DR + 32 * x + lane];
-            src = 4 * (e >> 13 & 0x1ff);
-            if constexpr (P == 4) {
-#pragma unroll
-              for (int j = 0; j < 4; j++) m[j] = mp[x][j];
-            } else {
-              const int *row = O.map + el * NN * NN + (e == 0xffffffffu ? 0 : e & 0x3ff);
-#pragma unroll
-              for (int j = 0; j < 4; j++) m[j] = row[j < (int)((e >> 11) & 3) + 1 ? j : 0];
-            }
-            return e == 0xffffffffu ? 0 : (int)((e >> 11) & 3) + 1;
           };
-          int m[4], src;
-          if (P == 4 && PASS == 0) {
-            const int n = entry(0, m, src);
-            scattered = 2 * __popc(__ballot_sync(0xffffffffu, drop_apart(m, n))) > __popc(__ballot_sync(0xffffffffu, n == 4));
-          }
-          if (P == 4 && scattered) {
+          // drop-in order 4: the lane's map entries of this pass, in flight during the products
+          int mp[L::DR ? L::DR / 32 : 1][4];
+          if constexpr (!PLAN && P == 4) {
+            const int *row = M.map + (cur.k0 + el) * (int64_t)(NN * NN);
 #pragma unroll
             for (int x = 0; x < L::DR / 32; x++) {
-              const int n = entry(x, m, src);
-              drop_issue_scattered(O.mat, m, n, redsW, src, lane);
-            }
-          } else {
+              const uint32_t e = tabR[PASS * L::DR + 32 * x + lane];
+              const int o = e == 0xffffffffu ? 0 : e & 0x3ff, n = e == 0xffffffffu ? 0 : (e >> 11) & 3;
 #pragma unroll
-            for (int x = 0; x < L::DR / 32; x++) {
-              const int n = entry(x, m, src);
-              drop_issue(O.mat, m, n, redsW + src);
+              for (int j = 0; j < 4; j++) mp[x][j] = __ldg(row + o + (j <= n ? j : 0) * (e >> 10 & 1 ? 5 : 1));
             }
           }
-          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        }
+          kstep_all(kstep, neg);
+          // residual: sum over the four lanes t of a node (reduce-scatter over the two slots)
+          [[maybe_unused]] const int Tm = t >> 1, To = Tm ^ 1;
+          if constexpr (RES) {
+            double sx = (Tm ? rp[1][0] : rp[0][0]) + __shfl_xor_sync(0xffffffffu, To ? rp[1][0] : rp[0][0], 2);
+            double sy = (Tm ? rp[1][1] : rp[0][1]) + __shfl_xor_sync(0xffffffffu, To ? rp[1][1] : rp[0][1], 2);
+            sx += __shfl_xor_sync(0xffffffffu, sx, 1);
+            sy += __shfl_xor_sync(0xffffffffu, sy, 1);
+            if constexpr (STRIP) residual_carry(sx, sy, cin);
+            const int an = Tm == 0 ? row_node(RT0) : (RT1 == NTM ? XN : row_node(RT1));
+            const bool act = (t & 1) == 0 && (Tm == 0 || RT1 < NTM || g == 0) && !halo && !(right && g >= 6);
+            residual_put(M.residual + 2 * (int64_t)nid[el * NN + an], act, PLAN && O.codes[el * CS + NN * NN + an], sx, sy);
+          }
+          if constexpr (RUNS) {
+            // acc becomes the blocks (xx, xy, yx, yy)
+#pragma unroll
+            for (int k = 0; k < NPAIR; k++)
+#pragma unroll
+              for (int h = 0; h < 2; h++) {
+                double kxx, kxy, kyx, kyy;
+                block(acc[k][0][h], acc[k][1][h], acc[k][2][h], acc[k][3][h], kxx, kxy, kyx, kyy);
+                acc[k][0][h] = kxx, acc[k][1][h] = kxy, acc[k][2][h] = kyx, acc[k][3][h] = kyy;
+              }
+            // every lane's previous bulk reads of the staging slots are complete
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            __syncwarp();
+            double *stg = redsW + 4 * lane;  // direct blocks: position 4g + t of their slot
+            if constexpr (STRIP) {
+              if (take) {
+#pragma unroll
+                for (int k = 0; k < NPAIR; k++)
+#pragma unroll
+                  for (int h = 0; h < 2; h++) {
+                    const double2 *cs = reinterpret_cast<const double2 *>(stg + 128 * frag_slot(k, h, 0) + 4 * 27);
+                    acc[k][0][h] += cs[0].x, acc[k][1][h] += cs[0].y;
+                    acc[k][2][h] += cs[1].x, acc[k][3][h] += cs[1].y;
+                  }
+              }
+              __syncwarp();
+            }
+            uint32_t allfirst = 0x80u;
+            if constexpr (PLAN && !NL) {
+              // the lane's code bytes and row addresses first: rows pi(g) and 8 + pi(g) hold
+              // its direct blocks, rows 8 + 4h + t the transposed ones of pair (0, 1)
+              const uint8_t *rec = O.codes + el * CS;
+              const int *rbe = O.rbase + el * NN;
+              uint32_t cd[NPAIR][2], ct[2];
+#pragma unroll
+              for (int k = 0; k < NPAIR; k++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) cd[k][h] = rec[pa * NN + t + (k == 2 ? 8 * NN : 0) + (k == 0 ? 0 : 8) + 4 * h];
+#pragma unroll
+              for (int h = 0; h < 2; h++) ct[h] = rec[t * NN + pa + (8 + 4 * h) * NN];
+              const double *r0 = O.mat + 4 * (int64_t)rbe[pa], *r1 = O.mat + 4 * (int64_t)rbe[8 + pa];
+              const double *rt0 = O.mat + 4 * (int64_t)rbe[8 + t], *rt1 = O.mat + 4 * (int64_t)rbe[12 + t];
+              const unsigned sd = (unsigned)__cvta_generic_to_shared(stg);
+              const unsigned st = (unsigned)__cvta_generic_to_shared(redsW + 4 * (8 * t + pa));
+              auto direct = [&](auto kc, auto hc) {
+                constexpr int k = decltype(kc)::value, h = decltype(hc)::value;
+                frag_put_row<1024 * frag_slot(k, h, 0)>(k == 2 ? r1 : r0, cd[k][h], m80, sd, acc[k][0][h], acc[k][1][h],
+                                                        acc[k][2][h], acc[k][3][h]);
+                allfirst &= cd[k][h];
+              };
+              direct(IC<0>{}, IC<0>{});
+              direct(IC<0>{}, IC<1>{});
+              direct(IC<1>{}, IC<0>{});
+              direct(IC<1>{}, IC<1>{});
+              frag_put_row<1024 * frag_slot(1, 0, 1)>(rt0, ct[0], m80, st, acc[1][0][0], acc[1][2][0], acc[1][1][0], acc[1][3][0]);
+              frag_put_row<1024 * frag_slot(1, 1, 1)>(rt1, ct[1], m80, st, acc[1][0][1], acc[1][2][1], acc[1][1][1], acc[1][3][1]);
+              direct(IC<2>{}, IC<0>{});
+              direct(IC<2>{}, IC<1>{});
+              allfirst &= ct[0] & ct[1];
+            } else {
+#pragma unroll
+              for (int k = 0; k < NPAIR; k++) {
+                {
+                  const int TA = F::ta(0, k), TB = F::tb(0, k);
+                  const int a = 8 * TA + pa;
+#pragma unroll
+                  for (int h = 0; h < 2; h++) {
+                    const int b = 8 * TB + 4 * h + t;
+                    const double kxx = acc[k][0][h], kxy = acc[k][1][h], kyx = acc[k][2][h], kyy = acc[k][3][h];
+                    // NONLINEAR diagonal tiles: (a, b) for a <= b and, for a < b, its exact
+                    // transpose (b, a) at the staging position the (b, a) lane would use
+                    const bool diag = NL && TA == TB;
+                    allfirst &= frag_put<P, PLAN>(O, el, a, b, 0, !diag || a <= b, m80, kxx, kxy, kyx, kyy,
+                                                  stg + 128 * frag_slot(k, h, 0));
+                    if (TA < TB) {
+                      allfirst &= frag_put<P, PLAN>(O, el, a, b, 1, true, m80, kxx, kxy, kyx, kyy,
+                                                    redsW + 128 * frag_slot(k, h, 1) + 4 * (8 * t + pa));
+                    } else if (diag) {
+                      const int xb = b - 8 * TA, xa = a - 8 * TA;  // pi(g') = xb; a = 8T + 4h' + t'
+                      const int gb = 2 * (xb & 3) + (xb >> 2);
+                      allfirst &= frag_put<P, PLAN>(O, el, a, b, 1, a < b, m80, kxx, kxy, kyx, kyy,
+                                                    redsW + 128 * frag_slot(k, xa >> 2, 0) + 4 * (4 * gb + (xa & 3)));
+                    }
+                  }
+                }
+              }
+            }
+            issue_runs(O, el, !halo && (allfirst & 0x80u) == 0);
+          }
+          // stiffness blocks, orders 2 and 4: lane (g, t) writes (8TA + pi(g), 8TB + 4h + t) of
+          // each pair and, for TA < TB, its transpose (NONLINEAR diagonal pairs: for a <= b,
+          // and the exact transpose); then the row and column of node XN: of the two slots of
+          // xs, lanes t/2 = x take slot x, t even (XN, a), t odd its transpose.  First stores
+          // go out at once, the blocks to add are staged and leave FL at a time after one
+          // proxy fence, as one bulk group.  Fewer fences and groups, against waiting for the
+          // group before: order 4 takes all four slots at a time (256^2 486 us; two from each
+          // half of the slots in turn 503), order 2 an element's three (512 x 2048 annulus 1178
+          // us, from two sets of slots in turn 1184), its NONLINEAR blocks two (500 x 512 770 us,
+          // four 808).
+          if constexpr (EX && PLAN) {
+            constexpr int FL = P == 4 ? 4 : (NL ? 2 : 3), HALF = FL == 2 ? 2 : 0;
+            double *reds = redsW + 4 * lane;
+            double *dst[FL];
+            bool add[FL];
+            int n = 0;
+            auto flush = [&](int m) {
+              bool any = false;
+#pragma unroll
+              for (int x = 0; x < FL; x++) any = any || (x < m && add[x]);
+              if (!__any_sync(0xffffffffu, any)) return;
+              if (el > 0) pair_first_landed();
+              asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+              if (el > 0) {
+                __syncwarp();
+                pair_first_visible();
+              }
+#pragma unroll
+              for (int x = 0; x < FL; x++)
+                if (x < m) bulk_add_block(dst[x], reds + 128 * (HALF * half + x), add[x]);
+              asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+              half ^= 1;
+            };
+            auto put = [&](int r, int c, bool act, double v0, double v1, double v2, double v3) {
+              // the bulk reads of the slots used next are complete
+              if (n == 0) {
+                if constexpr (HALF) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+              }
+              add[n] = frag_put_block<P>(O, el, r, c, act, v0, v1, v2, v3, reds + 128 * (HALF * half + n), dst[n]);
+              if (++n == FL) {
+                flush(FL);
+                n = 0;
+              }
+            };
+            double kxx, kxy, kyx, kyy;
+#pragma unroll
+            for (int k = 0; k < NPAIR; k++)
+#pragma unroll
+              for (int h = 0; h < 2; h++) {
+                const int TA = F::ta(PASS, k), TB = F::tb(PASS, k);
+                const int a = row_node(TA), b = col_node(TB, h);
+                const bool diag = NL && TA == TB;
+                block(acc[k][0][h], acc[k][1][h], acc[k][2][h], acc[k][3][h], kxx, kxy, kyx, kyy);
+                put(a, b, !diag || a <= b, kxx, kxy, kyx, kyy);
+                if (TA < TB || diag) put(b, a, !diag || a < b, kxx, kyx, kxy, kyy);
+              }
+            double xv[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+              xv[c] = (Tm ? xs[1][c] : xs[0][c]) + __shfl_xor_sync(0xffffffffu, To ? xs[1][c] : xs[0][c], 2);
+              xv[c] += __shfl_xor_sync(0xffffffffu, xv[c], 1);
+            }
+            block(xv[0], xv[1], xv[2], xv[3], kxx, kxy, kyx, kyy);
+            const int xa = Tm == 0 ? row_node(RT0) : (RT1 == NTM ? XN : row_node(RT1));
+            const bool tr = t & 1;
+            put(tr ? xa : XN, tr ? XN : xa, Tm == 0 || RT1 < NTM || (g == 0 && !tr), kxx, tr ? kyx : kxy, tr ? kxy : kyx, kyy);
+            if (n) flush(n);
+          }
+          // drop-in, orders 2 and 4: every block is staged (drop_run), and each lane adds its
+          // entries' stretches of adjacent blocks.  A reduction of 32 bytes per block bounded
+          // these launches: 200 x 201 order 4, with the element kernel's FP64 atomics 987 us
+          // for the driver's two calls, with 32-byte reductions 1082, with stretches 648;
+          // 501 x 500 order 2 597 -> 496
+          if constexpr (EX && !PLAN) {
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            __syncwarp();
+            auto stage_at = [&](int block, double v0, double v1, double v2, double v3) {
+              double2 *x = reinterpret_cast<double2 *>(redsW + 4 * block);
+              x[0] = make_double2(v0, v1);
+              x[1] = make_double2(v2, v3);
+            };
+            double kxx, kxy, kyx, kyy;
+            int sl = 0;  // slots in the order of drop_run
+#pragma unroll
+            for (int k = 0; k < NPAIR; k++)
+#pragma unroll
+              for (int h = 0; h < 2; h++) {
+                const int TA = F::ta(PASS, k), TB = F::tb(PASS, k);
+                block(acc[k][0][h], acc[k][1][h], acc[k][2][h], acc[k][3][h], kxx, kxy, kyx, kyy);
+                if constexpr (NL) {  // order 2: (a, b) for a <= b and its exact transpose
+                  const int b = 4 * h + t;
+                  if (pa <= b) stage_at(32 * h + 4 * g + t, kxx, kxy, kyx, kyy);
+                  if (pa < b) stage_at(32 * (pa >> 2) + 4 * (2 * (b & 3) + (b >> 2)) + (pa & 3), kxx, kyx, kxy, kyy);
+                } else {
+                  stage_at(32 * sl++ + 4 * g + t, kxx, kxy, kyx, kyy);
+                  if (TA < TB) stage_at(32 * sl++ + 8 * t + pa, kxx, kyx, kxy, kyy);
+                }
+              }
+            double xv[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+              xv[c] = (Tm ? xs[1][c] : xs[0][c]) + __shfl_xor_sync(0xffffffffu, To ? xs[1][c] : xs[0][c], 2);
+              xv[c] += __shfl_xor_sync(0xffffffffu, xv[c], 1);
+            }
+            block(xv[0], xv[1], xv[2], xv[3], kxx, kxy, kyx, kyy);
+            constexpr int SX = 32 * (P == 2 ? 2 : PASS ? 10 : 8), NM = RT1 < NTM ? 16 : 8;
+            const bool tr = t & 1, xd = RT1 == NTM && Tm == 1;  // xd: the diagonal block's lanes
+            if (!xd || (g == 0 && !tr))
+              stage_at(SX + (xd ? 2 * NM : (tr ? NM : 0) + 8 * Tm + pa), kxx, tr ? kyx : kxy, tr ? kxy : kyx, kyy);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            auto entry = [&](int x, int (&m)[4], int &src) {
+              const uint32_t e = tabR[PASS * L::DR + 32 * x + lane];
+              src = 4 * (e >> 13 & 0x1ff);
+              if constexpr (P == 4) {
+#pragma unroll
+                for (int j = 0; j < 4; j++) m[j] = mp[x][j];
+              } else {
+                const int *row = O.map + el * NN * NN + (e == 0xffffffffu ? 0 : e & 0x3ff);
+#pragma unroll
+                for (int j = 0; j < 4; j++) m[j] = row[j < (int)((e >> 11) & 3) + 1 ? j : 0];
+              }
+              return e == 0xffffffffu ? 0 : (int)((e >> 11) & 3) + 1;
+            };
+            int m[4], src;
+            if (P == 4 && PASS == 0) {
+              const int n = entry(0, m, src);
+              scattered = 2 * __popc(__ballot_sync(0xffffffffu, drop_apart(m, n))) > __popc(__ballot_sync(0xffffffffu, n == 4));
+            }
+            if (P == 4 && scattered) {
+#pragma unroll
+              for (int x = 0; x < L::DR / 32; x++) {
+                const int n = entry(x, m, src);
+                drop_issue_scattered(O.mat, m, n, redsW, src, lane);
+              }
+            } else {
+#pragma unroll
+              for (int x = 0; x < L::DR / 32; x++) {
+                const int n = entry(x, m, src);
+                drop_issue(O.mat, m, n, redsW + src);
+              }
+            }
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          }
         };
         pass(IC<0>{});
         if constexpr (F::NPASS == 2) {
