@@ -1987,7 +1987,7 @@ int launch_frag_p(const AsmArgs &a, cudaStream_t s, bool chained, bool single) {
   // pair: the warp's step is what the launch takes, and one element's stiffness and writes
   // are most of half of it (33 x 31 order 4 63.5 -> 38.9 us, order 3 NONLINEAR
   // 44.1 -> 22.6; order 2, bound by its four launches, 18.5 -> 18.4), and so does the last
-  // round of the warps as far as its elements go around (order-4 drop-in 90 x 89 122 -> 112
+  // wave of the warps as far as its elements go around (order-4 drop-in 90 x 89 122 -> 112
   // us, order-3 drop-in 80 x 79 34.8 -> 32.8, order-3 NONLINEAR plan 90 x 89 63.5 -> 58.4;
   // not in order-4 plans, see UnitStride).
   // Not the residual alone, where both elements of a step are rows of the same products

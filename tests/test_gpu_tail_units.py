@@ -1,7 +1,7 @@
-"""GPU: fragment-kernel launches whose last round of the resident warps holds fewer than two
+"""GPU: fragment-kernel launches whose last wave of the resident warps holds fewer than two
 elements per warp, so that some or all warps take one: element counts either side of whole
-and half rounds, drop-in and plans in the colour layout (two colours of a one-element-high
-strip), against the FP64 oracle at 1e-12; and a half round costs less than a whole one."""
+and half waves, drop-in and plans in the colour layout (two colours of a one-element-high
+strip), against the FP64 oracle at 1e-12; and a half wave costs less than a whole one."""
 import numpy as np
 import pytest
 
@@ -60,7 +60,7 @@ def test_plan(fem, orc, cuda, order, strain, n):
     plan.close()
 
 
-def test_half_a_round_costs_less(fem, cuda):
+def test_half_a_wave_costs_less(fem, cuda):
     import torch
 
     def best(nx, ny):
